@@ -169,11 +169,12 @@ struct Links {
   template <typename R>
   __device__ __forceinline__ m3<R> load(int mu, int par, uint32_t i) const {
     m3<R> u;
+    const V* q = p + idx(mu, par, 0, i);
     if constexpr (sizeof(V) == 4 * sizeof(S)) {
       // FP32 12-real: three float4 chunks (e00,e01), (e02,e10), (e11,e12).
-      const V a = ldv<LM>(&p[idx(mu, par, 0, i)]);
-      const V b = ldv<LM>(&p[idx(mu, par, 1, i)]);
-      const V c = ldv<LM>(&p[idx(mu, par, 2, i)]);
+      const V a = ldv<LM>(q);
+      const V b = ldv<LM>(q + stride);
+      const V c = ldv<LM>(q + 2 * (size_t)stride);
       u.e[0][0] = mk<R>(R(a.x), R(a.y));
       u.e[0][1] = mk<R>(R(a.z), R(a.w));
       u.e[0][2] = mk<R>(R(b.x), R(b.y));
@@ -184,7 +185,7 @@ struct Links {
       // 2-component chunks: chunk c = element c of the row-major 3x3.
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const V v = ldv<LM>(&p[idx(mu, par, c, i)]);
+        const V v = ldv<LM>(q + c * (size_t)stride);
         u.e[c / 3][c % 3] = mk<R>(R(v.x), R(v.y));
       }
     }
@@ -197,10 +198,11 @@ struct Links {
   template <typename R>
   __device__ __forceinline__ m3<R> load_rows01(int mu, int par, uint32_t i) const {
     m3<R> u;
+    const V* q = p + idx(mu, par, 0, i);
     if constexpr (sizeof(V) == 4 * sizeof(S)) {
-      const V a = ldv<LM>(&p[idx(mu, par, 0, i)]);
-      const V b = ldv<LM>(&p[idx(mu, par, 1, i)]);
-      const V c = ldv<LM>(&p[idx(mu, par, 2, i)]);
+      const V a = ldv<LM>(q);
+      const V b = ldv<LM>(q + stride);
+      const V c = ldv<LM>(q + 2 * (size_t)stride);
       u.e[0][0] = mk<R>(R(a.x), R(a.y));
       u.e[0][1] = mk<R>(R(a.z), R(a.w));
       u.e[0][2] = mk<R>(R(b.x), R(b.y));
@@ -210,7 +212,7 @@ struct Links {
     } else {
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
-        const V v = ldv<LM>(&p[idx(mu, par, c, i)]);
+        const V v = ldv<LM>(q + c * (size_t)stride);
         u.e[c / 3][c % 3] = mk<R>(R(v.x), R(v.y));
       }
     }
@@ -219,21 +221,22 @@ struct Links {
 
   template <typename R>
   __device__ __forceinline__ void store(int mu, int par, uint32_t i, const m3<R>& u) const {
+    V* q = p + idx(mu, par, 0, i);
     if constexpr (sizeof(V) == 4 * sizeof(S)) {
       V a, b, c;
       a.x = S(u.e[0][0].re), a.y = S(u.e[0][0].im), a.z = S(u.e[0][1].re), a.w = S(u.e[0][1].im);
       b.x = S(u.e[0][2].re), b.y = S(u.e[0][2].im), b.z = S(u.e[1][0].re), b.w = S(u.e[1][0].im);
       c.x = S(u.e[1][1].re), c.y = S(u.e[1][1].im), c.z = S(u.e[1][2].re), c.w = S(u.e[1][2].im);
-      p[idx(mu, par, 0, i)] = a;
-      p[idx(mu, par, 1, i)] = b;
-      p[idx(mu, par, 2, i)] = c;
+      q[0] = a;
+      q[stride] = b;
+      q[2 * (size_t)stride] = c;
     } else {
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         V v;
         v.x = S(u.e[c / 3][c % 3].re);
         v.y = S(u.e[c / 3][c % 3].im);
-        p[idx(mu, par, c, i)] = v;
+        q[c * (size_t)stride] = v;
       }
     }
   }
