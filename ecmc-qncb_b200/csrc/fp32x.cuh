@@ -54,6 +54,32 @@ struct is_fp32<float> : std::true_type {};
 template <>
 struct is_fp32<f1> : std::true_type {};
 
+// Two f1 values in one register pair, with the packed operations of sm_100 (fma.rn.f32x2 and its
+// kin): each half is rounded as the f1 operator rounds it, so packed code gives the same bits as
+// the scalar code that it stands for.  By the instruction counts, an operand whose halves are one
+// register (bc), exchanged or both negated costs nothing; halves of opposite sign cost an
+// instruction, and a pair of registers that are not neighbours one or two moves.
+struct f2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ f2 pack(f1 a, f1 b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a.v), "f"(b.v));
+  return r;
+}
+__device__ __forceinline__ void unpack(f2 p, f1& a, f1& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a.v), "=f"(b.v) : "l"(p.v)); }
+__device__ __forceinline__ f2 bc(f1 a) { return pack(a, a); }
+__device__ __forceinline__ f2 fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ f2 operator*(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
 // Arithmetic type of the kernels for storage type S: FP64 storage computes in double, FP32
 // storage in f1.
 template <typename S>

@@ -297,6 +297,22 @@ __device__ __forceinline__ cx<R> conj_diff(cx<R> a, cx<R> b, cx<R> c, cx<R> d) {
             fma(-a.re, b.im, fma(-a.im, b.re, fma(c.re, d.im, c.im * d.re))));
 }
 
+// In FP32 the two components run in one packed chain, each in the order above (the same bits):
+// 9 packed instructions for 16.  Measured on 32^4 FP32 12-real: heatbath pass 66.2 -> 64.4 us.
+// (Packed products of matrices, in this form, are slower: pass 69.3 us.  A packed multiply-add
+// reads up to six registers and takes as long as the two that it stands for, and the products
+// need a sign made for every element.)
+__device__ __forceinline__ cx<f1> conj_diff(cx<f1> a, cx<f1> b, cx<f1> c, cx<f1> d) {
+  const f2 np = pack(f1(-1.0f), f1(1.0f));
+  f2 t = bc(c.im) * pack(d.im, d.re);
+  t = fma(bc(c.re), pack(d.re, d.im) * np, t);
+  t = fma(bc(-a.im), pack(b.im, b.re), t);
+  t = fma(bc(-a.re), pack(b.re, b.im) * np, t);
+  cx<f1> r;
+  unpack(t, r.re, r.im);
+  return r;
+}
+
 // Third row of an SU(3) matrix from its first two: r2 = conj(r0 x r1).
 template <typename R>
 __device__ __forceinline__ void reconstruct_row2(m3<R>& u) {
