@@ -10,6 +10,7 @@
 
 #include "../../include/qcb.h"
 #include "api_internal.h"
+#include "flow.h"
 #include "host_io.h"
 #include "kernels.h"
 
@@ -105,19 +106,6 @@ LatDev with_links(const LatDev& d, void* p) {
   return r;
 }
 
-// One RK3 step with the three fused stages: a -> b -> a -> b.  The step's input in `a`
-// is overwritten by stage 2 (stage 1 has consumed it); the result is in `b`.
-int rk3(qcb_lattice* L, const LatDev& a, const LatDev& b, double eps) {
-  qcb_ctx* c = L->ctx;
-  AlgDev z;
-  z.p = L->fz;
-  CU(launch_flow_stage(1, a, b, z, eps, c->stream, c->block), "flow stage 1");
-  CU(launch_flow_stage(2, b, a, z, eps, c->stream, c->block), "flow stage 2");
-  CU(launch_flow_stage(3, a, b, z, eps, c->stream, c->block), "flow stage 3");
-  c->launches += 3;
-  return QCB_OK;
-}
-
 // Device buffer of at least `need` doubles for the partial sums of fused measurements.
 int ensure_meas(qcb_lattice* L, size_t need) {
   if (L->meas_n >= need) return QCB_OK;
@@ -132,26 +120,91 @@ int ensure_meas(qcb_lattice* L, size_t need) {
   return QCB_OK;
 }
 
-// One RK3 step a -> b as rk3(), with the clover (Q, E) of the step's input summed inside
-// stage 1 and written to dst_dev[0..1] (FP32 whole lattices: one thread per site).
-int rk3_qe(qcb_lattice* L, const LatDev& a, const LatDev& b, double eps, double* dst_dev) {
+// The rounds of lattice d (links a, other buffer b) through the context's loop buffer.
+int loop_rounds(qcb_lattice* L, const LatDev& d, void* b, double eps, std::vector<FlowLat>* rounds) {
   qcb_ctx* c = L->ctx;
-  AlgDev z;
-  z.p = L->fz;
-  const int nb = flow_site_blocks(a);
-  const int r_ = ensure_meas(L, 2 * (size_t)nb + 512);
-  if (r_ != QCB_OK) return r_;
-  CU(launch_flow_site_qe(a, b, z, eps, L->meas, c->stream), "flow stage 1 with Q/E");
-  CU(launch_qe_from_parts(L->meas, nb, L->meas + 2 * nb, dst_dev, 1.0 / (double)a.g.Vg, c->stream), "Q/E sums");
-  CU(launch_flow_stage(2, b, a, z, eps, c->stream, c->block), "flow stage 2");
-  CU(launch_flow_stage(3, a, b, z, eps, c->stream, c->block), "flow stage 3");
-  c->launches += 6;
+  const Geom& g = d.g;
+  const size_t least = loops_bytes(g, d.prec, 2);
+  if (loops_reserve(&c->loops, loops_bytes(g, d.prec, g.L[3]), least) != cudaSuccess)
+    return fail(QCB_ERR_NOMEM, "cannot allocate the plaquette-loop work space");
+  const LoopDev k = loops_view(c->loops, 0, g, d.prec, loops_slices(g, d.prec, c->loops.bytes));
+  *rounds = flow_rounds(d, k);
+  for (FlowLat& r : *rounds) {
+    r.b = b;
+    r.acc = L->fz;
+    r.eps = eps;
+  }
   return QCB_OK;
 }
 
-int qe_async(qcb_lattice* L, const LatDev& d, double* dst_dev) {
+// The loops of every round of the links selected by swap, then (parts != nullptr) the clover
+// sums of its sites into parts[0 .. 2n), n = qe_parts(rounds), and (stage != 0) the update of
+// RK3 stage `stage`.
+uint32_t qe_parts(const std::vector<FlowLat>& rounds) {
+  uint32_t n = 0;
+  for (const FlowLat& r : rounds) n += qe_blocks(r);
+  return n;
+}
+int loop_pass(qcb_lattice* L, const std::vector<FlowLat>& rounds, int swap, int stage, double* parts) {
   qcb_ctx* c = L->ctx;
-  CU(launch_clover_qe(d, c->d_scratch, dst_dev, c->stream, c->block), "clover Q/E");
+  const int prec = L->dev.prec, nr = L->dev.nr;
+  const uint32_t n = parts ? qe_parts(rounds) : 0;
+  uint32_t first = 0;
+  for (const FlowLat& r : rounds) {
+    FlowSet s;
+    s.one = r;
+    s.blocks = loops_blocks(r);
+    CU(launch_loops(s, prec, nr, parts != nullptr, swap, 0, c->stream), "plaquette loops");
+    c->launches++;
+    if (parts) {
+      s.blocks = qe_blocks(r);
+      CU(launch_loops_qe(s, prec, nr, swap, parts, first, n, c->stream), "clover Q/E");
+      first += s.blocks;
+      c->launches++;
+    }
+    if (stage) {
+      s.blocks = update_blocks(r);
+      CU(launch_flow_update(s, prec, nr, stage, swap, 0, c->stream), "flow stage");
+      c->launches++;
+    }
+  }
+  return QCB_OK;
+}
+
+// RK3 step `step` (links in a for even steps, b for odd ones; the result is in the other).
+// With qe_dev, the clover (Q, E) of the step's input is summed from stage 1's loops and written
+// to qe_dev[0..1].
+int rk3(qcb_lattice* L, const std::vector<FlowLat>& rounds, int step, double* qe_dev) {
+  qcb_ctx* c = L->ctx;
+  const int odd = step & 1;
+  double* parts = nullptr;
+  const uint32_t n = qe_dev ? qe_parts(rounds) : 0;
+  if (qe_dev) {
+    const int r_ = ensure_meas(L, 2 * (size_t)n + 512);
+    if (r_ != QCB_OK) return r_;
+    parts = L->meas;
+  }
+  int r_ = loop_pass(L, rounds, odd, 1, parts);
+  if (r_ == QCB_OK) r_ = loop_pass(L, rounds, odd ^ 1, 2, nullptr);
+  if (r_ == QCB_OK) r_ = loop_pass(L, rounds, odd, 3, nullptr);
+  if (r_ != QCB_OK) return r_;
+  if (qe_dev) {
+    CU(launch_qe_from_parts(parts, (int)n, parts + 2 * (size_t)n, qe_dev, 1.0 / (double)L->dev.g.Vg, c->stream),
+       "Q/E sums");
+    c->launches += 3;
+  }
+  return QCB_OK;
+}
+
+// Clover (Q, E) of the rounds' links (swap as loop_pass), without a step.
+int qe_async(qcb_lattice* L, const std::vector<FlowLat>& rounds, int swap, double* dst_dev) {
+  qcb_ctx* c = L->ctx;
+  const uint32_t n = qe_parts(rounds);
+  int r_ = ensure_meas(L, 2 * (size_t)n + 512);
+  if (r_ == QCB_OK) r_ = loop_pass(L, rounds, swap, 0, L->meas);
+  if (r_ != QCB_OK) return r_;
+  CU(launch_qe_from_parts(L->meas, (int)n, L->meas + 2 * (size_t)n, dst_dev, 1.0 / (double)L->dev.g.Vg, c->stream),
+     "Q/E sums");
   c->launches += 3;
   return QCB_OK;
 }
@@ -231,6 +284,7 @@ void ctx_free(qcb_ctx* c) {
   cudaFreeHost(c->h_out);
   cudaFree(c->d_stage[0]);
   cudaFree(c->d_stage[1]);
+  cudaFree(c->loops.p);
   cudaFreeHost(c->h_stage);
   if (c->stream) cudaStreamDestroy(c->stream);
   cudaGetLastError();
@@ -813,7 +867,9 @@ int qcb_topo_qe(qcb_lattice* L, double* q, double* e) {
   qcb_ctx* c = L->ctx;
   LOCK(c);
   TRY(set_device(c));
-  TRY(qe_async(L, L->dev, c->d_out));
+  std::vector<FlowLat> rounds;
+  TRY(loop_rounds(L, L->dev, nullptr, 0.0, &rounds));
+  TRY(qe_async(L, rounds, 0, c->d_out));
   CU(cudaMemcpyAsync(c->h_out, c->d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
   TRY(check_status(c));
   *q = c->h_out[0];
@@ -833,27 +889,20 @@ int qcb_flow_measure(qcb_lattice* L, double eps, int n_steps_gf, int n_rk_steps,
   TRY(ensure_flow_space(L));
   // gf.copy(field): the flow runs on a copy (observables_mpi.cpp:320).
   CU(cudaMemcpyAsync(L->fw[0], L->dev.links, L->bytes, cudaMemcpyDeviceToDevice, c->stream), "D2D copy");
-  LatDev a = with_links(L->dev, L->fw[0]);
-  LatDev b = with_links(L->dev, L->fw[1]);
+  std::vector<FlowLat> rounds;
+  if (n_steps_gf > 0) TRY(loop_rounds(L, with_links(L->dev, L->fw[0]), L->fw[1], eps, &rounds));
   double t = 0.0;
+  int step = 0;
   const int chunk = 32;  // (t, Q, E) records staged in d_out (64 doubles) between host reads
   for (int s0 = 0; s0 < n_steps_gf; s0 += chunk) {
     const int n = (s0 + chunk <= n_steps_gf) ? chunk : n_steps_gf - s0;
     std::vector<double> ts(n);
     for (int k = 0; k < n; ++k) {
       ts[k] = t;
-      // FP32: the record is summed inside stage 1 of the group's first RK3 step, which reads
-      // the same links; otherwise (FP64, or no step follows) by the clover kernel.
-      const bool fused = a.prec == QCB_FP32 && n_rk_steps > 0;
-      if (!fused) TRY(qe_async(L, a, c->d_out + 2 * k));
-      for (int r = 0; r < n_rk_steps; ++r) {
-        if (fused && r == 0)
-          TRY(rk3_qe(L, a, b, eps, c->d_out + 2 * k));
-        else
-          TRY(rk3(L, a, b, eps));
-        LatDev tmp = a;
-        a = b;
-        b = tmp;
+      // the record is summed from the loops of the group's first RK3 step; with no step, alone
+      if (n_rk_steps == 0) TRY(qe_async(L, rounds, step & 1, c->d_out + 2 * k));
+      for (int r = 0; r < n_rk_steps; ++r, ++step) {
+        TRY(rk3(L, rounds, step, r == 0 ? c->d_out + 2 * k : nullptr));
         t += eps;
       }
     }
@@ -878,16 +927,11 @@ int qcb_flow_steps(qcb_lattice* L, double eps, int n) {
   TRY(ensure_flow_space(L));
   // Each RK3 step ping-pongs between the primary buffer and fw[0]; the result is copied
   // back to the primary buffer when it ends up in fw[0].
-  LatDev a = L->dev;
-  LatDev b = with_links(L->dev, L->fw[0]);
-  for (int r = 0; r < n; ++r) {
-    TRY(rk3(L, a, b, eps));
-    LatDev tmp = a;
-    a = b;
-    b = tmp;
-  }
-  if (a.links != L->dev.links)
-    CU(cudaMemcpyAsync(L->dev.links, a.links, L->bytes, cudaMemcpyDeviceToDevice, c->stream), "D2D copy");
+  std::vector<FlowLat> rounds;
+  if (n > 0) TRY(loop_rounds(L, L->dev, L->fw[0], eps, &rounds));
+  for (int r = 0; r < n; ++r) TRY(rk3(L, rounds, r, nullptr));
+  if (n & 1)
+    CU(cudaMemcpyAsync(L->dev.links, L->fw[0], L->bytes, cudaMemcpyDeviceToDevice, c->stream), "D2D copy");
   return QCB_OK;
 }
 
@@ -917,16 +961,9 @@ int qcb_flow_stage(qcb_lattice* L, int stage, double eps, int step) {
   TRY(ensure_flow_space(L));
   // step s ping-pongs between the links (a) and the work buffer fw[0] (b) as qcb_flow_steps:
   // stage 1 a -> b, stage 2 b -> a, stage 3 a -> b, with a and b swapped for odd s
-  const LatDev x = L->dev, y = with_links(L->dev, L->fw[0]);
-  const LatDev& a = (step & 1) ? y : x;
-  const LatDev& b = (step & 1) ? x : y;
-  AlgDev z;
-  z.p = L->fz;
-  const LatDev& src = (stage == 2) ? b : a;
-  const LatDev& dst = (stage == 2) ? a : b;
-  CU(launch_flow_stage(stage, src, dst, z, eps, c->stream, c->block), "flow stage");
-  c->launches++;
-  return QCB_OK;
+  std::vector<FlowLat> rounds;
+  TRY(loop_rounds(L, L->dev, L->fw[0], eps, &rounds));
+  return loop_pass(L, rounds, (step & 1) ^ (stage == 2 ? 1 : 0), stage, nullptr);
 }
 
 int qcb_flow_finish(qcb_lattice* L, int n_steps) {

@@ -14,16 +14,11 @@
 
 #include "api_internal.h"
 #include "batch.h"
+#include "flow.h"
 
 using namespace qcb;
 
 namespace {
-
-// Descriptor sets (n entries each) held on the device:
-enum { SET_LINKS = 0,    // links = primary (heatbath, plaquette, in-place flow with work = fw0)
-       SET_COPY_EVEN,    // links = fw0, work = fw1 (flow on a copy, even cumulative steps)
-       SET_COPY_ODD,     // links = fw1, work = fw0 (odd cumulative steps)
-       NSETS };
 
 constexpr int DEFAULT_TILE = 256;
 
@@ -34,11 +29,19 @@ struct qcb_batch {
   int n = 0, prec = 0, nr = 0;
   std::vector<qcb_lattice*> lats;
   std::vector<uint32_t> hb_tile, flow_tile;
-  BatchLat* d_desc = nullptr;  // NSETS * n
+  BatchLat* d_desc = nullptr;  // n, of the lattices' links
   BatchLat* h_desc = nullptr;  // pinned mirror
-  uint32_t* d_prefix = nullptr;  // hb (n+1) | flow (n+1) | reduction (n+1)
+  uint32_t* d_prefix = nullptr;  // hb (n+1) | plaquette (n+1)
   std::vector<uint32_t> h_prefix;
-  uint32_t per_hb = 0, per_flow = 0, nred = 0;
+  uint32_t per_hb = 0, nred = 0;
+  // Flow and clover (made on first use): on the links with the copy fw0 as the other buffer,
+  // and on copies (fw0 with fw1).  The plans differ in their descriptors only.
+  LoopBuf loops;
+  bool have_flow = false;
+  FlowPlan flow[2];
+  FlowLat* d_flow[2] = {nullptr, nullptr};
+  uint32_t* d_flow_prefix = nullptr;  // the plan's prefix, then its qe_prefix
+  double* d_qe = nullptr;             // clover partials
   uint32_t* d_done = nullptr;
   uint32_t* d_status = nullptr;  // [0] KP cap hits, [1] wait timeouts, [2] abort
   uint32_t* h_status = nullptr;
@@ -71,65 +74,61 @@ int bcuda(cudaError_t e, const char* what) {
 
 uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
-// Rebuild descriptors and prefix sums from the lattices and tiles; upload them.
-int upload_layout(qcb_batch* b) {
-  const int n = b->n;
-  b->h_prefix.assign(3 * (n + 1), 0);
-  uint32_t* ph = &b->h_prefix[0];
-  uint32_t* pf = &b->h_prefix[n + 1];
-  uint32_t* pr = &b->h_prefix[2 * (n + 1)];
-  for (int l = 0; l < n; ++l) {
-    const qcb_lattice* L = b->lats[l];
-    const uint32_t nth = ceil_div(L->dev.g.Vh, b->hb_tile[l]);
-    const uint32_t ntf = flow_items_per_tile(L->dev.prec) * ceil_div(L->dev.g.Vh, b->flow_tile[l]);
-    ph[l + 1] = ph[l] + nth;
-    pf[l + 1] = pf[l] + ntf;
-    pr[l + 1] = pr[l] + ceil_div(L->dev.g.V, (uint32_t)batch_red_sites());
-    for (int s = 0; s < NSETS; ++s) {
-      BatchLat& d = b->h_desc[s * n + l];
-      memset(&d, 0, sizeof d);
-      d.g = L->dev.g;
-      d.acc = L->fz;
-      d.tile = b->hb_tile[l];
-      d.ntiles = nth;
-      if (s == SET_LINKS) {
-        d.links = L->dev.links;
-        d.work = L->fw[0];
-      } else if (s == SET_COPY_EVEN) {
-        d.links = L->fw[0];
-        d.work = L->fw[1];
-      } else {
-        d.links = L->fw[1];
-        d.work = L->fw[0];
-      }
-    }
+void drop_flow(qcb_batch* b) {
+  for (FlowLat*& d : b->d_flow) {
+    cudaFree(d);
+    d = nullptr;
   }
-  b->per_hb = ph[n];
-  b->per_flow = pf[n];
-  b->nred = pr[n];
-  cudaFree(b->d_scratch);
-  b->d_scratch = nullptr;
-  BCU(cudaMalloc(&b->d_scratch, 2 * (size_t)b->nred * sizeof(double)), "batch scratch");
-  BCU(cudaMemcpyAsync(b->d_prefix, b->h_prefix.data(), b->h_prefix.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                      b->ctx->stream),
-      "prefix upload");
-  BCU(cudaMemcpyAsync(b->d_desc, b->h_desc, (size_t)NSETS * n * sizeof(BatchLat), cudaMemcpyHostToDevice,
-                      b->ctx->stream),
-      "descriptor upload");
-  BCU(cudaStreamSynchronize(b->ctx->stream), "sync");
+  cudaFree(b->d_flow_prefix);
+  cudaFree(b->d_qe);
+  b->d_flow_prefix = nullptr;
+  b->d_qe = nullptr;
+  b->have_flow = false;
   if (b->exec) {
     cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
   }
   b->have_plan = false;
+}
+
+// Rebuild descriptors and prefix sums from the lattices and tiles; upload them.
+int upload_layout(qcb_batch* b) {
+  const int n = b->n;
+  b->h_prefix.assign(2 * (n + 1), 0);
+  uint32_t* ph = &b->h_prefix[0];
+  uint32_t* pr = &b->h_prefix[n + 1];
+  for (int l = 0; l < n; ++l) {
+    const qcb_lattice* L = b->lats[l];
+    const uint32_t nth = ceil_div(L->dev.g.Vh, b->hb_tile[l]);
+    ph[l + 1] = ph[l] + nth;
+    pr[l + 1] = pr[l] + ceil_div(L->dev.g.V, (uint32_t)batch_red_sites());
+    BatchLat& d = b->h_desc[l];
+    memset(&d, 0, sizeof d);
+    d.g = L->dev.g;
+    d.links = L->dev.links;
+    d.tile = b->hb_tile[l];
+    d.ntiles = nth;
+  }
+  b->per_hb = ph[n];
+  b->nred = pr[n];
+  cudaFree(b->d_scratch);
+  b->d_scratch = nullptr;
+  BCU(cudaMalloc(&b->d_scratch, (size_t)b->nred * sizeof(double)), "batch scratch");
+  BCU(cudaMemcpyAsync(b->d_prefix, b->h_prefix.data(), b->h_prefix.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                      b->ctx->stream),
+      "prefix upload");
+  BCU(cudaMemcpyAsync(b->d_desc, b->h_desc, (size_t)n * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream),
+      "descriptor upload");
+  BCU(cudaStreamSynchronize(b->ctx->stream), "sync");
+  drop_flow(b);
   return QCB_OK;
 }
 
-// Heatbath parameters go into the SET_LINKS descriptors (host mirror + async upload).
+// Heatbath parameters go into the descriptors (host mirror + async upload).
 int set_hb_params(qcb_batch* b, const double* betas, const uint64_t* seeds, const uint64_t* sweep_offsets) {
   for (int l = 0; l < b->n; ++l) {
     if (!(betas[l] > 0.0)) return bfail(QCB_ERR_INVALID, "beta must be positive");
-    BatchLat& d = b->h_desc[SET_LINKS * b->n + l];
+    BatchLat& d = b->h_desc[l];
     d.beta = betas[l];
     d.k0 = (uint32_t)seeds[l];
     d.k1 = (uint32_t)(seeds[l] >> 32);
@@ -140,75 +139,99 @@ int set_hb_params(qcb_batch* b, const double* betas, const uint64_t* seeds, cons
   return QCB_OK;
 }
 
-// Flow descriptors use the flow tile.
-void flow_tiles_into(qcb_batch* b, int set, std::vector<BatchLat>& out) {
-  out.assign(b->h_desc + set * b->n, b->h_desc + (set + 1) * b->n);
-  for (int l = 0; l < b->n; ++l) {
-    out[l].tile = b->flow_tile[l];
-    out[l].ntiles = flow_items_per_tile(b->prec) * ceil_div(out[l].g.Vh, b->flow_tile[l]);
+// The lattices as items of a flow plan: on the links, or (copies) on fw0.
+std::vector<FlowItem> flow_items(const std::vector<qcb_lattice*>& lats, const std::vector<uint32_t>& tile, int copies) {
+  std::vector<FlowItem> items;
+  for (size_t l = 0; l < lats.size(); ++l) {
+    const qcb_lattice* L = lats[l];
+    FlowItem it;
+    it.L = L->dev;
+    it.b = L->fw[0];
+    if (copies) {
+      it.L.links = L->fw[0];
+      it.b = L->fw[1];
+    }
+    it.acc = L->fz;
+    it.eps = 0.0;
+    it.tile = tile[l];
+    it.nsteps = 1 << 30;
+    items.push_back(it);
   }
+  return items;
 }
 
-BatchRun make_run(qcb_batch* b, int set, int kind, uint32_t nlevels, int n_hits, double eps) {
-  BatchRun r;
-  r.lats = b->d_desc + set * b->n;
-  r.prefix = b->d_prefix + (kind == BATCH_HB ? 0 : (b->n + 1));
-  r.nlat = b->n;
-  r.nlevels = nlevels;
-  r.per_level = (kind == BATCH_HB) ? b->per_hb : b->per_flow;
-  r.done = b->d_done;
-  r.status = b->d_status;
-  r.n_hits = n_hits;
-  r.eps = eps;
-  return r;
+// Loop buffer, plans and their device arrays, made on first use.
+int ensure_flow_plan(qcb_batch* b) {
+  if (b->have_flow) return QCB_OK;
+  size_t want = 0, least = 0;
+  flow_plan_bytes(flow_items(b->lats, b->flow_tile, 0), &want, &least);
+  if (loops_reserve(&b->loops, want, least) != cudaSuccess)
+    return bfail(QCB_ERR_NOMEM, "cannot allocate the batch's plaquette-loop work space");
+  for (int k = 0; k < 2; ++k) {
+    b->flow[k] = flow_plan(flow_items(b->lats, b->flow_tile, k), b->loops);
+    BCU(cudaMalloc(&b->d_flow[k], b->flow[k].lats.size() * sizeof(FlowLat)), "flow descriptors");
+  }
+  std::vector<uint32_t> pre = b->flow[0].prefix;
+  pre.insert(pre.end(), b->flow[0].qe_prefix.begin(), b->flow[0].qe_prefix.end());
+  BCU(cudaMalloc(&b->d_flow_prefix, pre.size() * sizeof(uint32_t)), "flow prefix");
+  BCU(cudaMalloc(&b->d_qe, 2 * (size_t)b->flow[0].qe_prefix.back() * sizeof(double)), "clover partials");
+  BCU(cudaMemcpyAsync(b->d_flow_prefix, pre.data(), pre.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                      b->ctx->stream),
+      "flow prefix upload");
+  BCU(cudaStreamSynchronize(b->ctx->stream), "sync");
+  b->have_flow = true;
+  return QCB_OK;
 }
 
-// The flow descriptors (flow tile) live in a second device region after the NSETS sets.
-BatchLat* flow_desc(qcb_batch* b, int set) { return b->d_desc + (NSETS + set) * b->n; }
-
-int upload_flow_desc(qcb_batch* b) {
-  for (int s = 0; s < NSETS; ++s) {
-    std::vector<BatchLat> v;
-    flow_tiles_into(b, s, v);
-    BCU(cudaMemcpyAsync(flow_desc(b, s), v.data(), v.size() * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream),
-        "flow descriptor upload");
-    BCU(cudaStreamSynchronize(b->ctx->stream), "sync");
-  }
+// Step size of the next launches into the descriptors of plan k (host and device).
+int set_flow_eps(qcb_batch* b, int k, double eps) {
+  for (FlowLat& r : b->flow[k].lats) r.eps = eps;
+  BCU(cudaMemcpyAsync(b->d_flow[k], b->flow[k].lats.data(), b->flow[k].lats.size() * sizeof(FlowLat),
+                      cudaMemcpyHostToDevice, b->ctx->stream),
+      "flow descriptor upload");
   return QCB_OK;
 }
 
 int launch_hb(qcb_batch* b, int n_sweeps, int n_hits) {
   if (n_sweeps <= 0) return QCB_OK;
   BCU(cudaMemsetAsync(b->d_done, 0, b->n * sizeof(uint32_t), b->ctx->stream), "memset");
-  BatchRun r = make_run(b, SET_LINKS, BATCH_HB, 8u * (uint32_t)n_sweeps, n_hits, 0.0);
-  BCU(launch_batch(BATCH_HB, r, b->prec, b->nr, 128, 0, b->ctx->stream), "batched heatbath");
+  BatchRun r;
+  r.lats = b->d_desc;
+  r.prefix = b->d_prefix;
+  r.nlat = b->n;
+  r.nlevels = 8u * (uint32_t)n_sweeps;
+  r.per_level = b->per_hb;
+  r.done = b->d_done;
+  r.status = b->d_status;
+  r.n_hits = n_hits;
+  BCU(launch_batch(r, b->prec, b->nr, 128, 0, b->ctx->stream), "batched heatbath");
   b->ctx->launches++;
   return QCB_OK;
 }
 
-// n RK3 steps over descriptor set `set` (flow tiles).
-int launch_flow(qcb_batch* b, int set, int n_steps, double eps) {
-  if (n_steps <= 0) return QCB_OK;
-  BCU(cudaMemsetAsync(b->d_done, 0, b->n * sizeof(uint32_t), b->ctx->stream), "memset");
-  BatchRun r = make_run(b, set, BATCH_FLOW, 3u * (uint32_t)n_steps, 0, eps);
-  r.lats = flow_desc(b, set);
-  BCU(launch_batch(BATCH_FLOW, r, b->prec, b->nr, 128, 0, b->ctx->stream), "batched flow");
-  b->ctx->launches++;
+// n RK3 steps of plan k, from the links that `odd` selects.
+int launch_flow(qcb_batch* b, int k, int odd, int n_steps) {
+  BCU(run_flow_plan(b->flow[k], b->d_flow[k], b->d_flow_prefix, b->prec, b->nr, odd, n_steps, b->ctx->stream,
+                    &b->ctx->launches),
+      "batched flow");
   return QCB_OK;
 }
 
-int launch_plaq(qcb_batch* b, int set, double* out) {
-  BCU(launch_batch_plaquette(b->d_desc + set * b->n, b->d_prefix + 2 * (b->n + 1), b->n, b->nred, b->prec, b->nr,
-                             b->d_scratch, out, b->ctx->stream),
+int launch_plaq(qcb_batch* b, double* out) {
+  BCU(launch_batch_plaquette(b->d_desc, b->d_prefix + b->n + 1, b->n, b->nred, b->prec, b->nr, b->d_scratch, out,
+                             b->ctx->stream),
       "batched plaquette");
   b->ctx->launches += 2;
   return QCB_OK;
 }
-int launch_qe(qcb_batch* b, int set, double* out2) {
-  BCU(launch_batch_qe(b->d_desc + set * b->n, b->d_prefix + 2 * (b->n + 1), b->n, b->nred, b->prec, b->nr,
-                      b->d_scratch, out2, b->ctx->stream),
+int launch_qe(qcb_batch* b, int k, int odd, double* out2) {
+  BCU(run_qe_plan(b->flow[k], b->d_flow[k], b->d_flow_prefix, b->prec, b->nr, odd, b->d_qe, b->ctx->stream,
+                  &b->ctx->launches),
+      "batched clover");
+  BCU(launch_batch_qe(b->d_desc, b->d_flow_prefix + b->flow[k].prefix.size(), b->n, b->flow[k].qe_prefix.back(),
+                      b->d_qe, out2, b->ctx->stream),
       "batched clover Q/E");
-  b->ctx->launches += 2;
+  b->ctx->launches++;
   return QCB_OK;
 }
 
@@ -248,10 +271,9 @@ int batch_status(qcb_batch* b) {
 // The whole plan (heatbath, plaquette, flow on copies with records) as stream work.
 int enqueue_plan(qcb_batch* b, const qcb_batch_plan& p) {
   const int n = b->n;
-  const int per = 1 + 3 * (p.n_groups + 1);
   BTRY(launch_hb(b, p.n_sweeps, p.n_hits));
   // plaquette -> d_out[0 .. n)
-  BTRY(launch_plaq(b, SET_LINKS, b->d_out));
+  BTRY(launch_plaq(b, b->d_out));
   for (int l = 0; l < n; ++l) {
     qcb_lattice* L = b->lats[l];
     BCU(cudaMemcpyAsync(L->fw[0], L->dev.links, L->bytes, cudaMemcpyDeviceToDevice, b->ctx->stream), "copy");
@@ -259,13 +281,12 @@ int enqueue_plan(qcb_batch* b, const qcb_batch_plan& p) {
   // records: (Q, E) of group g -> d_out[n + 2 (g n + l)]
   int cum = 0;
   for (int g = 0; g <= p.n_groups; ++g) {
-    BTRY(launch_qe(b, (cum & 1) ? SET_COPY_ODD : SET_COPY_EVEN, b->d_out + n + 2 * (size_t)g * n));
+    BTRY(launch_qe(b, 1, cum & 1, b->d_out + n + 2 * (size_t)g * n));
     if (g < p.n_groups) {
-      BTRY(launch_flow(b, (cum & 1) ? SET_COPY_ODD : SET_COPY_EVEN, p.rk_per_group, p.eps));
+      BTRY(launch_flow(b, 1, cum & 1, p.rk_per_group));
       cum += p.rk_per_group;
     }
   }
-  (void)per;
   BCU(cudaMemcpyAsync(b->h_out, b->d_out, (n + 2 * (size_t)(p.n_groups + 1) * n) * sizeof(double),
                       cudaMemcpyDeviceToHost, b->ctx->stream),
       "result copy");
@@ -313,9 +334,9 @@ int qcb_batch_create(qcb_ctx* ctx, int n, qcb_lattice* const* lats, qcb_batch** 
     int r = ensure_flow_space(b->lats[l]);
     if (r != QCB_OK) return fail_all(r);
   }
-  if (cudaMalloc(&b->d_desc, 2 * (size_t)NSETS * n * sizeof(BatchLat)) != cudaSuccess ||
-      cudaMallocHost(&b->h_desc, (size_t)NSETS * n * sizeof(BatchLat)) != cudaSuccess ||
-      cudaMalloc(&b->d_prefix, 3 * (size_t)(n + 1) * sizeof(uint32_t)) != cudaSuccess ||
+  if (cudaMalloc(&b->d_desc, (size_t)n * sizeof(BatchLat)) != cudaSuccess ||
+      cudaMallocHost(&b->h_desc, (size_t)n * sizeof(BatchLat)) != cudaSuccess ||
+      cudaMalloc(&b->d_prefix, 2 * (size_t)(n + 1) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&b->d_done, (size_t)n * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&b->d_status, 4 * sizeof(uint32_t)) != cudaSuccess ||
       cudaMallocHost(&b->h_status, 4 * sizeof(uint32_t)) != cudaSuccess) {
@@ -325,7 +346,6 @@ int qcb_batch_create(qcb_ctx* ctx, int n, qcb_lattice* const* lats, qcb_batch** 
   }
   if (cudaMemset(b->d_status, 0, 4 * sizeof(uint32_t)) != cudaSuccess) return fail_all(QCB_ERR_CUDA);
   int r = upload_layout(b);
-  if (r == QCB_OK) r = upload_flow_desc(b);
   if (r != QCB_OK) return fail_all(r);
   ctx->refs++;  // under the context lock
   *out = b;
@@ -346,7 +366,8 @@ int qcb_batch_destroy(qcb_batch* b) {
 
 namespace {
 void batch_free(qcb_batch* b) {
-  if (b->exec) cudaGraphExecDestroy(b->exec);
+  drop_flow(b);
+  cudaFree(b->loops.p);
   cudaFree(b->d_desc);
   cudaFreeHost(b->h_desc);
   cudaFree(b->d_prefix);
@@ -376,8 +397,7 @@ int qcb_batch_set_tiles(qcb_batch* b, const int* hb_tile, const int* flow_tile) 
     if (hb_tile) b->hb_tile[l] = (uint32_t)hb_tile[l];
     if (flow_tile) b->flow_tile[l] = (uint32_t)flow_tile[l];
   }
-  BTRY(upload_layout(b));
-  return upload_flow_desc(b);
+  return upload_layout(b);
 }
 
 int qcb_batch_get_tiles(qcb_batch* b, int* hb_tile, int* flow_tile) {
@@ -404,7 +424,10 @@ int qcb_batch_flow_steps(qcb_batch* b, double eps, int n_steps) {
   if (n_steps < 0) return bfail(QCB_ERR_INVALID, "negative step count");
   std::lock_guard<std::mutex> lk(b->ctx->mu);
   BCU(cudaSetDevice(b->ctx->device), "cudaSetDevice");
-  BTRY(launch_flow(b, SET_LINKS, n_steps, eps));
+  if (n_steps == 0) return QCB_OK;
+  BTRY(ensure_flow_plan(b));
+  BTRY(set_flow_eps(b, 0, eps));
+  BTRY(launch_flow(b, 0, 0, n_steps));
   if (n_steps & 1)  // the result is in fw0
     for (int l = 0; l < b->n; ++l) {
       qcb_lattice* L = b->lats[l];
@@ -418,7 +441,7 @@ int qcb_batch_plaquette(qcb_batch* b, double* out) {
   std::lock_guard<std::mutex> lk(b->ctx->mu);
   BCU(cudaSetDevice(b->ctx->device), "cudaSetDevice");
   BTRY(ensure_out(b, (size_t)b->n * 2));
-  BTRY(launch_plaq(b, SET_LINKS, b->d_out));
+  BTRY(launch_plaq(b, b->d_out));
   BCU(cudaMemcpyAsync(b->h_out, b->d_out, b->n * sizeof(double), cudaMemcpyDeviceToHost, b->ctx->stream), "D2H");
   BTRY(batch_status(b));
   memcpy(out, b->h_out, b->n * sizeof(double));
@@ -430,7 +453,9 @@ int qcb_batch_topo_qe(qcb_batch* b, double* q, double* e) {
   std::lock_guard<std::mutex> lk(b->ctx->mu);
   BCU(cudaSetDevice(b->ctx->device), "cudaSetDevice");
   BTRY(ensure_out(b, (size_t)b->n * 2));
-  BTRY(launch_qe(b, SET_LINKS, b->d_out));
+  BTRY(ensure_flow_plan(b));
+  BTRY(set_flow_eps(b, 0, 0.0));
+  BTRY(launch_qe(b, 0, 0, b->d_out));
   BCU(cudaMemcpyAsync(b->h_out, b->d_out, 2 * b->n * sizeof(double), cudaMemcpyDeviceToHost, b->ctx->stream), "D2H");
   BTRY(batch_status(b));
   for (int l = 0; l < b->n; ++l) {
@@ -451,6 +476,8 @@ int qcb_batch_run(qcb_batch* b, const qcb_batch_plan* plan, const double* betas,
   const int n = b->n;
   BTRY(ensure_out(b, (size_t)n + 2 * (size_t)(p.n_groups + 1) * n));
   BTRY(set_hb_params(b, betas, seeds, sweep_offsets));
+  BTRY(ensure_flow_plan(b));
+  BTRY(set_flow_eps(b, 1, p.eps));
   bool graph = false;
   if (b->graph_ok) {
     if (!b->have_plan || !same_plan(b->plan, p) || !b->exec) {
@@ -584,60 +611,83 @@ extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
     }
     // A sub-batch of this size's lattices, timed on scratch copies: the heatbath runs on
     // fw1 (copied from the links) and the flow on fw1/fw0, so the lattices are untouched.
+    BTRY(ensure_flow_plan(b));
     const int m = (int)kv.second.size();
-    std::vector<BatchLat> dsc(m);
-    std::vector<uint32_t> pre(m + 1, 0);
+    std::vector<qcb_lattice*> lats(m);
     for (int j = 0; j < m; ++j) {
-      qcb_lattice* L = b->lats[kv.second[j]];
+      qcb_lattice* L = lats[j] = b->lats[kv.second[j]];
       BCU(cudaMemcpyAsync(L->fw[1], L->dev.links, L->bytes, cudaMemcpyDeviceToDevice, b->ctx->stream), "copy");
     }
+    std::vector<BatchLat> dsc(m);
+    std::vector<uint32_t> pre(m + 1, 0);
     BatchLat* d_dsc = nullptr;
+    FlowLat* d_flow = nullptr;
     uint32_t* d_pre = nullptr;
+    const size_t rounds = b->flow[0].lats.size() + (size_t)m;
     BCU(cudaMalloc(&d_dsc, m * sizeof(BatchLat)), "tune alloc");
-    BCU(cudaMalloc(&d_pre, (m + 1) * sizeof(uint32_t)), "tune alloc");
+    BCU(cudaMalloc(&d_flow, rounds * sizeof(FlowLat)), "tune alloc");
+    BCU(cudaMalloc(&d_pre, 6 * rounds * sizeof(uint32_t)), "tune alloc");
     float best_hb = 1e30f, best_fl = 1e30f;
     int arg_hb = DEFAULT_TILE, arg_fl = DEFAULT_TILE;
     for (int kind = 0; kind < 2; ++kind)
       for (int cand : cands) {
-        for (int j = 0; j < m; ++j) {
-          qcb_lattice* L = b->lats[kv.second[j]];
-          BatchLat& d = dsc[j];
-          memset(&d, 0, sizeof d);
-          d.g = L->dev.g;
-          d.links = L->fw[1];
-          d.work = L->fw[0];
-          d.acc = L->fz;
-          d.beta = 6.0;
-          d.k0 = 12345u;
-          d.tile = (uint32_t)cand;
-          d.ntiles = (kind == 0 ? 1u : flow_items_per_tile(L->dev.prec)) * ceil_div(d.g.Vh, (uint32_t)cand);
-          pre[j + 1] = pre[j] + d.ntiles;
-        }
-        if (cand > 2 * (int)dsc[0].g.Vh && cand != cands[0]) continue;  // larger than the lattice
-        BCU(cudaMemcpyAsync(d_dsc, dsc.data(), m * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream), "H2D");
-        BCU(cudaMemcpyAsync(d_pre, pre.data(), (m + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, b->ctx->stream),
-            "H2D");
+        if (cand > 2 * (int)lats[0]->dev.g.Vh && cand != cands[0]) continue;  // larger than the lattice
         BatchRun r;
-        r.lats = d_dsc;
-        r.prefix = d_pre;
-        r.nlat = m;
-        r.per_level = pre[m];
-        r.done = b->d_done;
-        r.status = b->d_status;
-        r.n_hits = 1;
-        r.eps = 0.02;
-        r.nlevels = kind == 0 ? 16 : 6;  // 2 sweeps / 2 RK3 steps
+        FlowPlan fp;
+        if (kind == 0) {
+          for (int j = 0; j < m; ++j) {
+            BatchLat& d = dsc[j];
+            memset(&d, 0, sizeof d);
+            d.g = lats[j]->dev.g;
+            d.links = lats[j]->fw[1];
+            d.beta = 6.0;
+            d.k0 = 12345u;
+            d.tile = (uint32_t)cand;
+            d.ntiles = ceil_div(d.g.Vh, (uint32_t)cand);
+            pre[j + 1] = pre[j] + d.ntiles;
+          }
+          r.lats = d_dsc;
+          r.prefix = d_pre;
+          r.nlat = m;
+          r.per_level = pre[m];
+          r.done = b->d_done;
+          r.status = b->d_status;
+          r.n_hits = 1;
+          r.nlevels = 16;  // 2 sweeps
+          BCU(cudaMemcpyAsync(d_dsc, dsc.data(), m * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream), "H2D");
+          BCU(cudaMemcpyAsync(d_pre, pre.data(), (m + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, b->ctx->stream),
+              "H2D");
+        } else {
+          std::vector<FlowItem> items = flow_items(lats, std::vector<uint32_t>(m, (uint32_t)cand), 0);
+          for (int j = 0; j < m; ++j) {
+            items[j].L.links = lats[j]->fw[1];
+            items[j].b = lats[j]->fw[0];
+            items[j].eps = 0.02;
+          }
+          fp = flow_plan(items, b->loops);
+          BCU(cudaMemcpyAsync(d_flow, fp.lats.data(), fp.lats.size() * sizeof(FlowLat), cudaMemcpyHostToDevice,
+                              b->ctx->stream),
+              "H2D");
+          BCU(cudaMemcpyAsync(d_pre, fp.prefix.data(), fp.prefix.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                              b->ctx->stream),
+              "H2D");
+        }
         float best = 1e30f;
         for (int rep = 0; rep < 3; ++rep) {
           BCU(cudaMemsetAsync(b->d_done, 0, m * sizeof(uint32_t), b->ctx->stream), "memset");
           BCU(cudaEventRecord(e0, b->ctx->stream), "event");
-          BCU(launch_batch(kind == 0 ? BATCH_HB : BATCH_FLOW, r, b->prec, b->nr, 128, 0, b->ctx->stream), "tune launch");
+          if (kind == 0) {
+            BCU(launch_batch(r, b->prec, b->nr, 128, 0, b->ctx->stream), "tune launch");
+            b->ctx->launches++;
+          } else {  // 2 RK3 steps
+            BCU(run_flow_plan(fp, d_flow, d_pre, b->prec, b->nr, 0, 2, b->ctx->stream, &b->ctx->launches),
+                "tune launch");
+          }
           BCU(cudaEventRecord(e1, b->ctx->stream), "event");
           BCU(cudaEventSynchronize(e1), "event sync");
           float ms = 0;
           BCU(cudaEventElapsedTime(&ms, e0, e1), "elapsed");
           if (rep > 0) best = std::min(best, ms);
-          b->ctx->launches++;
         }
         if (kind == 0 && best < best_hb) {
           best_hb = best;
@@ -649,6 +699,7 @@ extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
         }
       }
     cudaFree(d_dsc);
+    cudaFree(d_flow);
     cudaFree(d_pre);
     cache[khb] = arg_hb;
     cache[kfl] = arg_fl;
@@ -663,6 +714,5 @@ extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
   write_cache(cache_path, cache);
   b->hb_tile = hb;
   b->flow_tile = fl;
-  BTRY(upload_layout(b));
-  return upload_flow_desc(b);
+  return upload_layout(b);
 }

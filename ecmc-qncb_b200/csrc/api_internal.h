@@ -4,6 +4,7 @@
 #include <string>
 
 #include "../../include/qcb.h"
+#include "flow.h"
 #include "kernels.h"
 
 struct qcb_ctx {
@@ -18,6 +19,9 @@ struct qcb_ctx {
   double* d_stage[2] = {nullptr, nullptr};
   size_t stage_bytes = 0;
   double* h_stage = nullptr;  // pinned, for file I/O
+  // Plaquette loops of the flow and the clover, shared by the context's lattices (its calls
+  // run in stream order); allocated on first use, at most LOOPS_MAX_BYTES or two time slices.
+  qcb::LoopBuf loops;
   uint64_t launches = 0;
   std::mutex mu;
   // Objects created on this context (lattices, batches, servers).  qcb_ctx_destroy with

@@ -1,0 +1,54 @@
+// flow_launch.cuh — what the kernels of the loops, the flow update and the clover share: which
+// lattice a block works on, and their launch.
+#pragma once
+#include "dispatch.cuh"
+#include "flow.h"
+#include "loops.cuh"
+#include "sync.cuh"
+
+namespace qcb {
+
+constexpr int FLOW_THREADS = 128;
+
+// Sites of one parity per block of the kernels that run one thread per site.
+__host__ __device__ __forceinline__ uint32_t site_tile(const FlowLat& r) {
+  return r.tile > (uint32_t)FLOW_THREADS ? r.tile : (uint32_t)FLOW_THREADS;
+}
+
+// The lattice l with prefix[l] <= b < prefix[l + 1], found by a whole warp: one load and one
+// ballot for each 32 lattices.
+__device__ __forceinline__ int lattice_of(const uint32_t* __restrict__ prefix, int nlat, uint32_t b) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < nlat; base += 32) {
+    const uint32_t end = base + lane < nlat ? __ldg(&prefix[base + lane + 1]) : 0xFFFFFFFFu;
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, end <= b);
+    if (m != 0xFFFFFFFFu) return base + __popc(m);
+  }
+  return nlat - 1;
+}
+
+template <typename S, int NR>
+__device__ __forceinline__ Links<S, NR> flow_links(const FlowLat& L, int swap) {
+  Links<S, NR> f;
+  f.p = reinterpret_cast<typename Links<S, NR>::V*>(swap ? L.b : L.a);
+  f.stride = L.g.stride;
+  return f;
+}
+
+// Programmatic stream serialization: the kernel's blocks become resident while the previous
+// kernel of the stream drains, and wait for it before they read (pdl_wait).
+template <typename... P, typename... A>
+cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, int block, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+}  // namespace qcb

@@ -1,5 +1,4 @@
-// flow_link.cuh — one link of one fused Wilson-flow RK3 stage (shared by the
-// single-lattice stage kernel and the persistent batched kernel).
+// flow_link.cuh — one link of one Wilson-flow RK3 stage, from its force.
 //
 // Reference: GradientFlow (src/flow/gradient_flow.cpp:15-114):
 //   Z   = -P_TA(U A)                         (force, gradient_flow.cpp:15-34)
@@ -8,7 +7,7 @@
 //   s3: X = 3/4 eps Z2 - eps acc                                   (compute_w3, :96-114)
 //   U' = exp(X) U   with Luescher's exponential (src/su3/utils.cpp:145-193)
 #pragma once
-#include "staple.cuh"
+#include "layout.cuh"
 
 namespace qcb {
 
@@ -39,18 +38,18 @@ __device__ __forceinline__ m3<R> flow_product(const m3<R>& E, const m3<R>& U) {
     return mul_nn(E, U);
 }
 
-// The stage-dependent part of one link's stage: X from the force Z and the accumulator,
-// and the accumulator update.
-template <typename ACC, typename R, int MU>
-__device__ __forceinline__ alg8<R> flow_x(const ACC& acc, const alg8<R>& Z, R eps, int stage, int par, uint32_t i) {
+// The stage-dependent part: X from the force Z and the accumulator Z0 (unused in stage 1), and
+// the accumulator's update.
+template <int STAGE, typename ACC, typename R>
+__device__ __forceinline__ alg8<R> flow_x(const ACC& acc, const alg8<R>& Z, const alg8<R>& Z0, R eps, int mu, int par,
+                                          uint32_t i) {
   alg8<R> X;
-  if (stage == 1) {
+  if constexpr (STAGE == 1) {
     const R c = R(0.25) * eps;
 #pragma unroll
     for (int k = 0; k < 8; ++k) X.a[k] = c * Z.a[k];
-    acc.template store<R>(MU, par, i, Z);
-  } else if (stage == 2) {
-    const alg8<R> Z0 = acc.template load<R>(MU, par, i);
+    acc.template store<R>(mu, par, i, Z);
+  } else if constexpr (STAGE == 2) {
     const R c1 = R(8.0 / 9.0) * eps, c0 = R(17.0 / 36.0) * eps;
     alg8<R> N;
 #pragma unroll
@@ -58,74 +57,13 @@ __device__ __forceinline__ alg8<R> flow_x(const ACC& acc, const alg8<R>& Z, R ep
       X.a[k] = fma(c1, Z.a[k], -(c0 * Z0.a[k]));
       N.a[k] = fma(R(8.0 / 9.0), Z.a[k], -(R(17.0 / 36.0) * Z0.a[k]));
     }
-    acc.template store<R>(MU, par, i, N);
+    acc.template store<R>(mu, par, i, N);
   } else {
-    const alg8<R> Z0 = acc.template load<R>(MU, par, i);
     const R c1 = R(0.75) * eps;
 #pragma unroll
     for (int k = 0; k < 8; ++k) X.a[k] = fma(c1, Z.a[k], -(eps * Z0.a[k]));
   }
   return X;
-}
-
-// Stage `stage` (1, 2, 3) of one link U_MU(x), x = (par, i): src -> dst.  Inlined with a
-// constant stage in the per-stage kernels; the persistent batch kernel passes it at run time.
-template <typename F, typename ACC, typename R, int MU>
-__device__ __forceinline__ void flow_link(const Geom& g, const F& src, const F& dst, const ACC& acc, R eps, int stage,
-                                          int par, uint32_t i) {
-  const Coord x = cb_coord(g, par, i);
-  if (!own_site(g, x.c[3])) return;  // halo slice of a slab
-  const m3<R> A = staple_sum_best<F, R, MU>(g, src, x, par, i);
-  const m3<R> U = src.template load<R>(MU, par, i);
-  // Z = P_TA(-U A) = -P_TA(U A)
-  alg8<R> Z = proj_ta(mul_nn(U, A));
-#pragma unroll
-  for (int k = 0; k < 8; ++k) Z.a[k] = -Z.a[k];
-  const alg8<R> X = flow_x<ACC, R, MU>(acc, Z, eps, stage, par, i);
-  const m3<R> E = exp_su3(X);
-  m3<R> Un = flow_product<F, R>(E, U);
-  flow_reunit<R>(Un, stage);
-  dst.template store<R>(MU, par, i, Un);
-}
-
-// Runtime-direction, runtime-stage variant (one code body for every mu and stage).
-template <typename F, typename ACC, typename R>
-__device__ __forceinline__ void flow_link_rt(const Geom& g, const F& src, const F& dst, const ACC& acc, R eps, int stage,
-                                             int mu, int par, uint32_t i) {
-  const Coord x = cb_coord(g, par, i);
-  if (!own_site(g, x.c[3])) return;  // halo slice of a slab
-  const m3<R> A = staple_sum_rt<F, R>(g, src, x, mu, par, i);
-  const m3<R> U = src.template load<R>(mu, par, i);
-  alg8<R> Z = proj_ta(mul_nn(U, A));
-#pragma unroll
-  for (int k = 0; k < 8; ++k) Z.a[k] = -Z.a[k];
-  alg8<R> X;
-  if (stage == 1) {
-    const R c = R(0.25) * eps;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) X.a[k] = c * Z.a[k];
-    acc.template store<R>(mu, par, i, Z);
-  } else {
-    const alg8<R> Z0 = acc.template load<R>(mu, par, i);
-    if (stage == 2) {
-      const R c1 = R(8.0 / 9.0) * eps, c0 = R(17.0 / 36.0) * eps;
-      alg8<R> N;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        X.a[k] = fma(c1, Z.a[k], -(c0 * Z0.a[k]));
-        N.a[k] = fma(R(8.0 / 9.0), Z.a[k], -(R(17.0 / 36.0) * Z0.a[k]));
-      }
-      acc.template store<R>(mu, par, i, N);
-    } else {
-      const R c1 = R(0.75) * eps;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) X.a[k] = fma(c1, Z.a[k], -(eps * Z0.a[k]));
-    }
-  }
-  const m3<R> E = exp_su3(X);
-  m3<R> Un = flow_product<F, R>(E, U);
-  flow_reunit<R>(Un, stage);
-  dst.template store<R>(mu, par, i, Un);
 }
 
 }  // namespace qcb

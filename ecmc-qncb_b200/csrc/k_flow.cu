@@ -1,94 +1,130 @@
-// k_flow.cu — fused Wilson-flow RK3 stages.
+// k_flow.cu — the update of a Wilson-flow RK3 stage, from the loops of its source links.
 //
 // Reference: GradientFlow (src/flow/gradient_flow.cpp:15-128) runs five full-lattice loops
 // per step (compute_force, compute_w1, compute_force, compute_w2, replace_force_0,
 // compute_force, compute_w3) over three full GaugeField copies, with a halo exchange after
-// every W update.  Each stage here is one kernel, one thread per link:
-//   Z   = -P_TA(U A)                         (force, gradient_flow.cpp:15-34)
-//   s1: X = eps/4 Z0;                acc = Z0                      (compute_w1, :37-53)
-//   s2: X = 8/9 eps Z1 - 17/36 eps Z0; acc = 8/9 Z1 - 17/36 Z0    (compute_w2 + replace_force_0, :56-93)
-//   s3: X = 3/4 eps Z2 - eps acc                                   (compute_w3, :96-114)
-//   U' = exp(X) U   with Luescher's exponential (src/su3/utils.cpp:145-193)
+// every W update.  Each stage here is two kernels: the plaquette loops of the links (k_loops.cu),
+// and this one, which takes each link's force from them and applies the stage (flow_link.cuh).
 // Links are double-buffered (src -> dst) because every stage reads neighbours of the
 // previous stage; the force accumulator holds 8 reals per link.
-#include "dispatch.cuh"
+//
+// Measured per RK3 step on 32^4, against kernels that multiplied out the staples of every link
+// (twelve products each; in FP32 ten, with one product shared by a plane's two links): FP64
+// 18-real 2.65 -> 2.06 ms, FP32 12-real 1.08 -> 0.97 ms.  Of a stage, the loops take a third and the
+// update two thirds (FP32 215 us, 0.71-0.85 GB of DRAM traffic, 56% issue; FP64 420-480 us, 56% of
+// the DRAM rate).  A smaller loop buffer, whose rounds of slices would stay in L2, costs more in
+// half-filled last waves than it saves: 110, 70 and 24 MB make the FP32 step 1.05, 1.09 and 1.24 ms.
+#include "flow_launch.cuh"
 #include "flow_link.cuh"
-#include "sync.cuh"
 
 namespace qcb {
 
-// Grid (2 * tiles, 4): blockIdx.y = mu, blockIdx.x = 2 * tile + parity.  Blocks are issued
-// x-fastest, so one direction runs at a time over the whole lattice (one mu instantiation in
-// the instruction cache) and both parities of a tile run together.  Measured per RK3 step on
-// 32^4 FP32-12: 1.37 ms; a run-time-mu kernel with the eight (mu, parity) blocks of a tile
-// adjacent: 1.58 ms; chunks of 256 / 512 / 1024 tiles with the four directions of a chunk in
-// turn (to reuse the chunk's links from L2): 1.48 / 1.71 / 1.54 ms, because the direction
-// changes every one or two waves of blocks and the four instantiations then compete for the
-// instruction cache.  The flow is bound by instruction issue, not by DRAM.
-// Resident blocks per SM (the register bound): FP32 5 (96 registers) measured 1.36 ms per RK3
-// step on 32^4 FP32-12 against 1.74 ms with the compiler's own choice; FP64 3 measured
-// 2.76 ms per step on 32^4 FP64-18 against 3.02 ms with the compiler's own choice or 2.
+// Four warps work on 32 sites of one parity.  Warp nu first moves the three loops K_{mu nu}(x-nu)
+// up along U_nu(x-nu), which it loads and completes once
+// into shared memory; then warp mu sums its link's force from them and applies the stage.
 #ifndef QCB_FLOW_MINB32
 #define QCB_FLOW_MINB32 5
 #endif
 #ifndef QCB_FLOW_MINB64
 #define QCB_FLOW_MINB64 3
 #endif
-template <typename S, int NR, int STAGE>
-__global__ void __launch_bounds__(128, sizeof(S) == 4 ? QCB_FLOW_MINB32 : QCB_FLOW_MINB64) k_flow_stage(Geom g, Links<S, NR> src, Links<S, NR> dst, AlgField<S> acc,
-                                                    S eps) {
-  pdl_launch_dependents();  // launched with programmatic stream serialization
+template <typename S, int NR, int STAGE, bool MULTI>
+__global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_FLOW_MINB32 : QCB_FLOW_MINB64)
+    k_flow_update(const __grid_constant__ FlowLat one, const FlowLat* __restrict__ lats,
+                  const uint32_t* __restrict__ prefix, int nlat, int swap, int step) {
+  typedef arith_t<S> R;
+  typedef Links<S, NR> F;
+  pdl_launch_dependents();
   pdl_wait();
-  const int mu = blockIdx.y;
-  const uint32_t i = (blockIdx.x >> 1) * blockDim.x + threadIdx.x;
-  const int par = blockIdx.x & 1;
-  if (i >= g.Vh) return;
-  switch (mu) {
-    case 0: flow_link<Links<S, NR>, AlgField<S>, arith_t<S>, 0>(g, src, dst, acc, arith_t<S>(eps), STAGE, par, i); break;
-    case 1: flow_link<Links<S, NR>, AlgField<S>, arith_t<S>, 1>(g, src, dst, acc, arith_t<S>(eps), STAGE, par, i); break;
-    case 2: flow_link<Links<S, NR>, AlgField<S>, arith_t<S>, 2>(g, src, dst, acc, arith_t<S>(eps), STAGE, par, i); break;
-    default: flow_link<Links<S, NR>, AlgField<S>, arith_t<S>, 3>(g, src, dst, acc, arith_t<S>(eps), STAGE, par, i); break;
+  const int l = MULTI ? lattice_of(prefix, nlat, blockIdx.x) : 0;
+  const FlowLat& L = MULTI ? lats[l] : one;
+  if (MULTI && step >= L.nsteps) return;
+  const uint32_t b = MULTI ? blockIdx.x - __ldg(&prefix[l]) : blockIdx.x;
+  const F src = flow_links<S, NR>(L, swap), dst = flow_links<S, NR>(L, swap ^ 1);
+  AlgField<S> acc;
+  acc.p = reinterpret_cast<typename AlgField<S>::V*>(L.acc);
+  acc.stride = L.g.stride;
+  const Loops<S> K(L.k, L.g);
+  typedef typename AlgStore<S>::V V;
+  constexpr int NC = AlgStore<S>::NC;
+  __shared__ V moved[12][NC][32];  // [3 nu + k]: loop k of direction nu, moved to x
+  const uint32_t n = (uint32_t)(L.t1 - L.t0) * K.half, first = (b >> 1) * L.tile;
+  const int par = (int)(b & 1), w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const R eps = R(S(L.eps));
+  for (uint32_t k0 = 0; k0 < L.tile && first + k0 < n; k0 += 32) {
+    const uint32_t k = first + k0 + lane;
+    const uint32_t i = (uint32_t)L.t0 * K.half + k;
+    const bool on = k < n;
+    if (k0) __syncthreads();
+    alg8<R> Z, Z0;
+    m3<R> U;
+    if (on) {
+      const Coord x = cb_coord(L.g, par, i);
+      {
+        alg8<R> m[3];
+        transported<F, S, R>(src, K, x, nb_offsets(L.g, x), w, par, L.g.L[3], m);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          V v[NC];
+          S* q = reinterpret_cast<S*>(v);
+#pragma unroll
+          for (int a = 0; a < 8; ++a) q[a] = S(m[j].a[a]);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) moved[3 * w + j][c][lane] = v[c];
+        }
+      }
+      // -sum_nu of K_{mu nu}(x), mu = w
+      const uint32_t jx = K.at(i, x.c[3], x.c[3]);
+#pragma unroll
+      for (int a = 0; a < 8; ++a) Z.a[a] = R(0);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int nu = j + (j >= w);
+        const alg8<R> A = K.template load<R>(nu > w ? plane_of(w, nu) : plane_of(nu, w), par, jx);
+        add_alg(Z, A, nu > w ? R(-1) : R(1));
+      }
+      if (STAGE != 1) Z0 = acc.template load<R>(w, par, i);
+      U = src.template load<R>(w, par, i);
+    }
+    __syncthreads();
+    if (on) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int nu = j + (j >= w);
+        V v[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) v[c] = moved[3 * nu + w - (w > nu)][c][lane];
+        const S* q = reinterpret_cast<const S*>(v);
+        alg8<R> B;
+#pragma unroll
+        for (int a = 0; a < 8; ++a) B.a[a] = R(q[a]);
+        add_alg(Z, B, nu > w ? R(1) : R(-1));
+      }
+      const alg8<R> X = flow_x<STAGE, AlgField<S>, R>(acc, Z, Z0, eps, w, par, i);
+      m3<R> Un = flow_product<F, R>(exp_su3(X), U);
+      flow_reunit<R>(Un, STAGE);
+      dst.template store<R>(w, par, i, Un);
+    }
   }
 }
 
 template <typename S, int NR>
-static cudaError_t flow_impl(int stage, const LatDev& Ls, const LatDev& Ld, const AlgDev& z, double eps,
-                             cudaStream_t s, int block) {
-  Links<S, NR> src, dst;
-  src.p = reinterpret_cast<typename Links<S, NR>::V*>(Ls.links);
-  src.stride = Ls.g.stride;
-  dst.p = reinterpret_cast<typename Links<S, NR>::V*>(Ld.links);
-  dst.stride = Ld.g.stride;
-  AlgField<S> acc;
-  acc.p = reinterpret_cast<typename AlgField<S>::V*>(z.p);
-  acc.stride = Ls.g.stride;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid_for(Ls.g.Vh, block) * 2, 4);
-  cfg.blockDim = dim3(block);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  void (*kern)(Geom, Links<S, NR>, Links<S, NR>, AlgField<S>, S) =
-      stage == 1 ? k_flow_stage<S, NR, 1> : (stage == 2 ? k_flow_stage<S, NR, 2> : k_flow_stage<S, NR, 3>);
-  return cudaLaunchKernelEx(&cfg, kern, Ls.g, src, dst, acc, S(eps));
+static cudaError_t update_impl(const FlowSet& s, int stage, int swap, int step, cudaStream_t st) {
+  if (s.blocks == 0) return cudaSuccess;
+  void (*kern)(const FlowLat, const FlowLat*, const uint32_t*, int, int, int) =
+      s.lats ? (stage == 1 ? k_flow_update<S, NR, 1, true>
+                           : (stage == 2 ? k_flow_update<S, NR, 2, true> : k_flow_update<S, NR, 3, true>))
+             : (stage == 1 ? k_flow_update<S, NR, 1, false>
+                           : (stage == 2 ? k_flow_update<S, NR, 2, false> : k_flow_update<S, NR, 3, false>));
+  return pdl_launch(kern, dim3(s.blocks), FLOW_THREADS, st, s.one, s.lats, s.prefix, s.nlat, swap, step);
 }
 
-// FP32 lattices run the flow with one thread per site (k_flow_site.cu): measured per RK3 step
-// 1.297 -> 1.225 ms on 32^4 and 23.4 -> 20.3 ms on 64^4 (12-real), with DRAM traffic 1.12 x the
-// algorithmic bytes instead of 2.0 x.  FP64 keeps one thread per link.
-#ifndef QCB_FLOW_SITE
-#define QCB_FLOW_SITE 1
-#endif
-
-cudaError_t launch_flow_stage(int stage, const LatDev& src, const LatDev& dst, const AlgDev& z, double eps,
-                              cudaStream_t s, int block) {
-  if (block <= 0) block = 128;
-  if (src.prec != dst.prec || src.nr != dst.nr) return cudaErrorInvalidValue;
-  if (QCB_FLOW_SITE && src.prec == 1) return launch_flow_site(stage, src, dst, z, eps, s);
-  QCB_DISPATCH_STORE(src, flow_impl, stage, src, dst, z, eps, s, block);
+cudaError_t launch_flow_update(const FlowSet& s, int prec, int nr, int stage, int swap, int step, cudaStream_t st) {
+  if (stage < 1 || stage > 3) return cudaErrorInvalidValue;
+  LatDev probe;
+  probe.prec = prec;
+  probe.nr = nr;
+  QCB_DISPATCH_STORE(probe, update_impl, s, stage, swap, step, st);
 }
 
 }  // namespace qcb

@@ -1,0 +1,239 @@
+// k_loops.cu — the plaquette-loop field of a lattice, and the clover Q and E summed from it.
+//
+// References: clover_site, local_q_e_clover and topo_q_e_clover(_global)
+// (src/observables/observables_mpi.cpp:61-150) for Q and E; the loops also carry the force of
+// the Wilson flow (loops.cuh).
+#include "flow_launch.cuh"
+#include "reduce.cuh"
+
+namespace qcb {
+
+// ---- the loop buffer --------------------------------------------------------------------
+static size_t loops_stride(const Geom& g, int slices) {
+  return ((size_t)slices * (size_t)(g.str[3] / 2) + 63) / 64 * 64;
+}
+size_t loops_bytes(const Geom& g, int prec, int slices) {
+  return (size_t)(6 * 2 * 9) * loops_stride(g, slices) * (prec == QCB_PREC_FP64 ? 8 : 4);
+}
+int loops_slices(const Geom& g, int prec, size_t bytes) {
+  if (loops_bytes(g, prec, g.L[3]) <= bytes) return g.L[3];
+  const size_t one = loops_bytes(g, prec, 1);
+  int n = (int)(bytes / one);
+  if (n > g.L[3] - 1) n = g.L[3] - 1;
+  while (n >= 2 && loops_bytes(g, prec, n) > bytes) --n;
+  return n >= 2 ? n : 0;
+}
+cudaError_t loops_reserve(LoopBuf* buf, size_t want, size_t least) {
+  if (want > LOOPS_MAX_BYTES) want = LOOPS_MAX_BYTES;
+  if (want < least) want = least;
+  if (buf->bytes >= want || (buf->bytes >= least && buf->wanted >= want)) return cudaSuccess;
+  cudaFree(buf->p);
+  buf->p = nullptr;
+  buf->bytes = 0;
+  buf->wanted = want;
+  for (size_t n = want;; n = n / 2 > least ? n / 2 : least) {
+    if (cudaMalloc(&buf->p, n) == cudaSuccess) {
+      buf->bytes = n;
+      return cudaSuccess;
+    }
+    cudaGetLastError();
+    buf->p = nullptr;
+    if (n <= least) return cudaErrorMemoryAllocation;
+  }
+}
+LoopDev loops_view(const LoopBuf& buf, size_t off, const Geom& g, int prec, int slices) {
+  const size_t es = prec == QCB_PREC_FP64 ? 8 : 4, st = loops_stride(g, slices);
+  LoopDev k;
+  k.p = (char*)buf.p + off;
+  k.tr = (char*)buf.p + off + 6 * 2 * 8 * st * es;
+  k.stride = (uint32_t)st;
+  k.slices = slices;
+  return k;
+}
+
+std::vector<FlowLat> flow_rounds(const LatDev& L, const LoopDev& k) {
+  std::vector<FlowLat> out;
+  const Geom& g = L.g;
+  const bool whole = g.tlo == 0 && g.thi == g.L[3] - 1;
+  FlowLat r;
+  r.g = g;
+  r.a = L.links;
+  r.b = r.acc = nullptr;
+  r.k = k;
+  r.eps = 0.0;
+  r.tile = 32;
+  r.nsteps = 1 << 30;
+  const bool full = k.slices >= g.L[3];
+  if (!full && k.slices < 2) return out;  // no room: nothing can run (loops_reserve rules it out)
+  for (int t = g.tlo; t <= g.thi;) {
+    const int room = full ? g.L[3] : k.slices - 1;  // one slot holds the slice before the round
+    r.t0 = t;
+    r.t1 = t + room <= g.thi ? t + room : g.thi + 1;
+    if (full && whole) {
+      r.kt0 = 0;
+      r.kn = g.L[3];
+    } else {
+      r.kt0 = t == g.tlo ? t - 1 : t;
+      r.kn = r.t1 - r.kt0;
+    }
+    out.push_back(r);
+    t = r.t1;
+  }
+  return out;
+}
+
+static uint32_t tiles_of(const Geom& g, int slices, uint32_t tile) {
+  return 2 * (((uint32_t)slices * (uint32_t)(g.str[3] / 2) + tile - 1) / tile);  // both parities
+}
+uint32_t loops_blocks(const FlowLat& r) { return tiles_of(r.g, r.kn, site_tile(r)); }
+uint32_t qe_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, site_tile(r)); }
+uint32_t update_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, r.tile); }
+
+// ---- the loops --------------------------------------------------------------------------
+// One thread per site and grid row: row y of n takes planes y, y + n, ...; the planes run
+// through one body that is not unrolled.  Measured on 32^4 FP32 12-real: 125 us, 0.37 GB of DRAM
+// traffic (the links read and the loops written once), bound by the FP32 pipes and by the latency
+// of its sixteen links; FP64 18-real 250 us.  Six rows instead of one make a small lattice's few
+// blocks six times as many; from 2048 blocks the chip is full without that, and one row reads
+// the site's own links once for all its planes.
+template <typename S, int NR, bool TRACE>
+__device__ __forceinline__ void loops_site(const FlowLat& L, const Links<S, NR>& f, int par, uint32_t j) {
+  typedef arith_t<S> R;
+  const Loops<S> K(L.k, L.g);
+  int32_t ii = (int32_t)(j + (uint32_t)L.kt0 * K.half);
+  const bool before = ii < 0;  // the slice before 0 is the last one
+  if (before) ii += (int32_t)L.g.Vh;
+  const uint32_t i = (uint32_t)ii;
+  const Coord x = cb_coord(L.g, par, i);
+  const NbOff o = nb_offsets(L.g, x);
+  const uint32_t jx = K.at(i, x.c[3], before ? -1 : x.c[3]);
+  m3<R> U;
+  int have = -1;
+#pragma unroll 1
+  for (int p = blockIdx.y; p < 6; p += gridDim.y) {
+    const int mu = p < 3 ? 0 : (p < 5 ? 1 : 2), nu = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
+    if (mu != have) U = lead<Links<S, NR>, R>(f, mu, par, i);
+    have = mu;
+    const m3<R> W = plaquette_loop<Links<S, NR>, R>(f, U, mu, nu, par, i, cb_index((uint32_t)((int32_t)x.s + sel4(o.up, mu))),
+                                                    cb_index((uint32_t)((int32_t)x.s + sel4(o.up, nu))));
+    K.template store<R>(p, par, jx, proj_ta(W));
+    if (TRACE) K.template store_tr<R>(p, par, jx, (W.e[0][0].im + W.e[1][1].im + W.e[2][2].im) * R(1.0 / 3.0));
+  }
+}
+
+#ifndef QCB_LOOPS_MINB32
+#define QCB_LOOPS_MINB32 5
+#endif
+#ifndef QCB_LOOPS_MINB64
+#define QCB_LOOPS_MINB64 3
+#endif
+template <typename S, int NR, bool TRACE, bool MULTI>
+__global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_LOOPS_MINB32 : QCB_LOOPS_MINB64)
+    k_loops(const __grid_constant__ FlowLat one, const FlowLat* __restrict__ lats, const uint32_t* __restrict__ prefix,
+            int nlat, int swap, int step) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int l = MULTI ? lattice_of(prefix, nlat, blockIdx.x) : 0;
+  const FlowLat& L = MULTI ? lats[l] : one;
+  if (MULTI && step >= L.nsteps) return;
+  const uint32_t b = MULTI ? blockIdx.x - __ldg(&prefix[l]) : blockIdx.x;
+  const Links<S, NR> f = flow_links<S, NR>(L, swap);
+  const uint32_t n = (uint32_t)L.kn * (uint32_t)(L.g.str[3] >> 1), tile = site_tile(L), first = (b >> 1) * tile;
+  for (uint32_t k = threadIdx.x; k < tile && first + k < n; k += FLOW_THREADS)
+    loops_site<S, NR, TRACE>(L, f, (int)(b & 1), first + k);
+}
+
+template <typename S, int NR>
+static cudaError_t loops_impl(const FlowSet& s, bool trace, int swap, int step, cudaStream_t st) {
+  if (s.blocks == 0) return cudaSuccess;
+  auto kern = s.lats ? (trace ? k_loops<S, NR, true, true> : k_loops<S, NR, false, true>)
+                     : (trace ? k_loops<S, NR, true, false> : k_loops<S, NR, false, false>);
+  const unsigned rows = s.blocks >= 2048 ? 1 : (s.blocks >= 512 ? 3 : 6);
+  return pdl_launch(kern, dim3(s.blocks, rows), FLOW_THREADS, st, s.one, s.lats, s.prefix, s.nlat, swap, step);
+}
+
+cudaError_t launch_loops(const FlowSet& s, int prec, int nr, bool trace, int swap, int step, cudaStream_t st) {
+  LatDev probe;
+  probe.prec = prec;
+  probe.nr = nr;
+  QCB_DISPATCH_STORE(probe, loops_impl, s, trace, swap, step, st);
+}
+
+// ---- Q and E ------------------------------------------------------------------------------
+// Unscaled clover sums q_site = tr F01 F23 - tr F02 F13 + tr F03 F12 and e_site = sum_{mu<nu}
+// |F_mu nu|^2 (the 1/(4 pi^2) and 1/2 are applied to the totals).  The six planes run through
+// one body, in the pairs (01, 23), (02, 13), (03, 12); each pair's share is added in FP64.
+// Three transports a plane where four leaves were nine products: Q and E of 32^4 alone, loops
+// included, FP32 12-real 572 -> 370 us, FP64 18-real 1301 -> 720 us; with the loops already there
+// for an RK3 step, FP32 210 us more.
+template <typename S, int NR>
+__device__ __forceinline__ void qe_site(const FlowLat& L, const Links<S, NR>& f, int par, uint32_t i, double* q,
+                                        double* e) {
+  typedef arith_t<S> R;
+  const Loops<S> K(L.k, L.g);
+  const Coord x = cb_coord(L.g, par, i);
+  const NbOff o = nb_offsets(L.g, x);
+  ah9<R> prev;
+#pragma unroll 1
+  for (int p = 0; p < 6; ++p) {
+    const int h = p >> 1;
+    const int mu = (p & 1) == 0 ? 0 : (h == 0 ? 2 : 1), nu = (p & 1) == 0 ? h + 1 : (h == 2 ? 2 : 3);
+    const ah9<R> F = clover_plane<Links<S, NR>, S, R>(f, K, x, o, mu, nu, par, i, L.g.L[3]);
+    *e += (double)sqnorm_ah(F);
+    if (p & 1) {
+      const double t = (double)re_tr_ah(prev, F);
+      *q += h == 1 ? -t : t;
+    } else {
+      prev = F;
+    }
+  }
+}
+
+#ifndef QCB_QE_MINB32
+#define QCB_QE_MINB32 5
+#endif
+#ifndef QCB_QE_MINB64
+#define QCB_QE_MINB64 3
+#endif
+template <typename S, int NR, bool MULTI>
+__global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_QE_MINB32 : QCB_QE_MINB64)
+    k_loops_qe(const __grid_constant__ FlowLat one, const FlowLat* __restrict__ lats,
+               const uint32_t* __restrict__ prefix, int nlat, int swap, double* __restrict__ parts, uint32_t first,
+               uint32_t nparts) {
+  __shared__ double sh[FLOW_THREADS / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int l = MULTI ? lattice_of(prefix, nlat, blockIdx.x) : 0;
+  const FlowLat& L = MULTI ? lats[l] : one;
+  const uint32_t b = MULTI ? blockIdx.x - __ldg(&prefix[l]) : blockIdx.x;
+  const Links<S, NR> f = flow_links<S, NR>(L, swap);
+  const uint32_t half = (uint32_t)(L.g.str[3] >> 1), n = (uint32_t)(L.t1 - L.t0) * half, tile = site_tile(L),
+                 at = (b >> 1) * tile;
+  double q = 0.0, e = 0.0;
+  for (uint32_t k = threadIdx.x; k < tile && at + k < n; k += FLOW_THREADS)
+    qe_site<S, NR>(L, f, (int)(b & 1), (uint32_t)L.t0 * half + at + k, &q, &e);
+  const double bq = block_sum<FLOW_THREADS>(q, sh);
+  const double be = block_sum<FLOW_THREADS>(e, sh);
+  if (threadIdx.x == 0) {
+    parts[first + blockIdx.x] = bq;
+    parts[nparts + first + blockIdx.x] = be;
+  }
+}
+
+template <typename S, int NR>
+static cudaError_t loops_qe_impl(const FlowSet& s, int swap, double* parts, uint32_t first, uint32_t n,
+                                 cudaStream_t st) {
+  if (s.blocks == 0) return cudaSuccess;
+  auto kern = s.lats ? k_loops_qe<S, NR, true> : k_loops_qe<S, NR, false>;
+  return pdl_launch(kern, dim3(s.blocks), FLOW_THREADS, st, s.one, s.lats, s.prefix, s.nlat, swap, parts, first, n);
+}
+
+cudaError_t launch_loops_qe(const FlowSet& s, int prec, int nr, int swap, double* parts, uint32_t first, uint32_t n,
+                            cudaStream_t st) {
+  LatDev probe;
+  probe.prec = prec;
+  probe.nr = nr;
+  QCB_DISPATCH_STORE(probe, loops_qe_impl, s, swap, parts, first, n, st);
+}
+
+}  // namespace qcb

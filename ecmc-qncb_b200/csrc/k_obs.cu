@@ -1,11 +1,7 @@
-// k_obs.cu — mean plaquette and clover Q/E reductions.
+// k_obs.cu — mean plaquette reduction, and the sums of per-block partials.
 //
-// References:
-//   mean_plaquette_local / _global (src/observables/observables_mpi.cpp:8-43): serial sum of
-//   Re tr(U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag)/3 over x and mu < nu, / (6V).
-//   clover_site / local_q_e_clover / topo_q_e_clover(_global) (observables_mpi.cpp:61-150):
-//   F_{mu nu} = (C - C^dag)/8 with C the sum of the four leaves at x,
-//   q = (tr F01 F23 - tr F02 F13 + tr F03 F12) / (4 pi^2), e = 1/2 sum_{mu<nu} |F|^2.
+// Reference: mean_plaquette_local / _global (src/observables/observables_mpi.cpp:8-43): serial
+// sum of Re tr(U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag)/3 over x and mu < nu, / (6V).
 // Here: one thread per site (the two parities of a checkerboard index adjacent; a slab
 // skips its halo slices), per-site value in the lattice's arithmetic type, converted to FP64; FP64 tree reduction inside each block; the block partials are
 // summed in a fixed order with Neumaier compensation by a single-block kernel.  The grid
@@ -19,9 +15,8 @@ namespace qcb {
 constexpr int RED_THREADS = 128;
 constexpr int RED_BLOCKS = 148 * 8;
 
-// Minimum resident blocks per SM of the reduction kernels: the clover site evaluation is
-// the largest per-thread body; the bound keeps FP32 at 4 x 128 threads (128 registers) and
-// FP64 at 2 x 128 threads per SM.
+// Minimum resident blocks per SM of the reduction: FP32 4 x 128 threads (128 registers), FP64
+// 2 x 128 threads.
 template <typename S>
 struct RedMinBlocks {
   static constexpr int value = sizeof(S) == 4 ? 4 : 2;
@@ -138,48 +133,10 @@ cudaError_t launch_sum_parts(const double* parts, int n, double* tmp, double* ou
   return sum_parts(parts, n, 1, tmp, out, s);
 }
 
-template <typename S, int NR>
-__global__ void __launch_bounds__(RED_THREADS, RedMinBlocks<S>::value) k_clover_qe(Geom g, Links<S, NR> f, double* __restrict__ parts) {
-  typedef S R;
-  __shared__ double sh[RED_THREADS / 32];
-  double accq = 0.0, acce = 0.0;
-  const uint64_t n = (uint64_t)g.V;
-  for (uint64_t t = (uint64_t)blockIdx.x * RED_THREADS + threadIdx.x; t < n; t += (uint64_t)gridDim.x * RED_THREADS) {
-    // both parities of a checkerboard index together: a site's neighbours (opposite
-    // parity) are then read close in time, from L2
-    const int par = (int)(t & 1);
-    const uint32_t i = (uint32_t)(t >> 1);
-    const Coord x = cb_coord(g, par, i);
-    if (!own_site(g, x.c[3])) continue;
-    R q = 0, e = 0;
-    site_qe<Links<S, NR>, R>(g, f, x, par, i, &q, &e);
-    accq += (double)q;
-    acce += (double)e;
-  }
-  double bq = block_sum<RED_THREADS>(accq, sh);
-  double be = block_sum<RED_THREADS>(acce, sh);
-  if (threadIdx.x == 0) {
-    parts[blockIdx.x] = bq;
-    parts[gridDim.x + blockIdx.x] = be;
-  }
-}
-
 // out2[0] = Q = sum q / (4 pi^2); out2[1] = E = sum e / 2 / V.
 __global__ void k_qe_scale(double* out2, double inv_vol) {
   out2[0] = out2[0] * (1.0 / (4.0 * 3.14159265358979323846 * 3.14159265358979323846));
   out2[1] = 0.5 * out2[1] * inv_vol;
-}
-
-template <typename S, int NR>
-static cudaError_t clover_impl(const LatDev& L, double* scratch, double* out2, cudaStream_t s, int) {
-  Links<S, NR> f;
-  f.p = reinterpret_cast<typename Links<S, NR>::V*>(L.links);
-  f.stride = L.g.stride;
-  const int nb = red_grid(L.g);
-  k_clover_qe<S, NR><<<nb, RED_THREADS, 0, s>>>(L.g, f, scratch);
-  k_finalize<<<1, 64, 0, s>>>(scratch, nb, 2, out2);
-  k_qe_scale<<<1, 1, 0, s>>>(out2, 1.0 / (double)L.g.Vg);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_qe_from_parts(const double* parts, int n, double* tmp, double* out2, double inv_vol,
@@ -188,10 +145,6 @@ cudaError_t launch_qe_from_parts(const double* parts, int n, double* tmp, double
   if (e != cudaSuccess) return e;
   k_qe_scale<<<1, 1, 0, s>>>(out2, inv_vol);
   return cudaGetLastError();
-}
-
-cudaError_t launch_clover_qe(const LatDev& L, double* scratch, double* out2, cudaStream_t s, int block) {
-  QCB_DISPATCH_STORE(L, clover_impl, L, scratch, out2, s, block);
 }
 
 }  // namespace qcb

@@ -1,0 +1,255 @@
+// loops.cuh — plaquette loops, their parallel transport, and what the Wilson flow and the
+// clover make of them.
+//
+// Reference: the force -P_TA(U A) of GradientFlow (src/flow/gradient_flow.cpp:15-34) with the
+// staples of GaugeField.cpp:74-97, and the clover leaves of observables_mpi.cpp:61-107.
+//
+// With L_{mu nu}(y) = U_mu(y) U_nu(y+mu) U_mu(y+nu)^dag U_nu(y)^dag, every term of both is a
+// loop at some corner of a plaquette, and a loop moved along a link is conjugated by it; P_TA
+// commutes with the conjugation.  So with K_{mu nu} = P_TA(L_{mu nu}), K_{nu mu} = -K_{mu nu}:
+//   P_TA(U_mu(x) A_mu(x)) = sum_{nu != mu} [ K_{mu nu}(x) - Ad(U_nu(x-nu)) K_{mu nu}(x-nu) ]
+//   clover at x, from its four leaves = K(x) + Ad(U_nu(x-nu)) K(x-nu)
+//     + Ad(U_mu(x-mu)) [ K(x-mu) + Ad(U_nu(x-mu-nu)) K(x-mu-nu) ],  K = K_{mu nu}
+// with Ad(U) M = U^dag M U.  Each plaquette is multiplied out once (three products) instead of
+// seven times for the flow and sixteen for the clover, and a transport of eight reals costs
+// about as much as one product.
+#pragma once
+#include <type_traits>
+
+#include "flow.h"
+#include "staple.cuh"
+
+namespace qcb {
+
+// Index of plane (mu, nu), mu < nu: 01, 02, 03, 12, 13, 23.
+__device__ __forceinline__ int plane_of(int mu, int nu) { return ((mu * (7 - mu)) >> 1) + nu - mu - 1; }
+
+// The loop field of one lattice.  Time slice tv (-1: the slice before 0) sits in ring slot
+// (tv + 1) mod slices, or at its own place when all slices fit.
+template <typename S>
+struct Loops {
+  typedef typename AlgStore<S>::V V;
+  static constexpr int NC = AlgStore<S>::NC;
+  V* p;
+  S* tr;
+  uint32_t stride, half;
+  int slices;
+  bool full;
+  __device__ __forceinline__ Loops(const LoopDev& k, const Geom& g)
+      : p(reinterpret_cast<V*>(k.p)), tr(reinterpret_cast<S*>(k.tr)), stride(k.stride),
+        half((uint32_t)g.str[3] >> 1), slices(k.slices), full(k.slices >= g.L[3]) {}
+  // place of checkerboard site i of time t, read as slice tv
+  __device__ __forceinline__ uint32_t at(uint32_t i, int t, int tv) const {
+    if (full) return i;
+    return i + (uint32_t)((tv + 1) % slices - t) * half;
+  }
+  __device__ __forceinline__ size_t idx(int plane, int par, int c, uint32_t j) const {
+    return ((size_t)((plane * 2 + par) * NC + c)) * stride + j;
+  }
+  template <typename R>
+  __device__ __forceinline__ alg8<R> load(int plane, int par, uint32_t j) const {
+    V v[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = __ldg(&p[idx(plane, par, c, j)]);
+    const S* q = reinterpret_cast<const S*>(v);
+    alg8<R> z;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) z.a[k] = R(q[k]);
+    return z;
+  }
+  template <typename R>
+  __device__ __forceinline__ void store(int plane, int par, uint32_t j, const alg8<R>& z) const {
+    V v[NC];
+    S* q = reinterpret_cast<S*>(v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) q[k] = S(z.a[k]);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) p[idx(plane, par, c, j)] = v[c];
+  }
+  template <typename R>
+  __device__ __forceinline__ R load_tr(int plane, int par, uint32_t j) const {
+    return R(__ldg(&tr[(size_t)(plane * 2 + par) * stride + j]));
+  }
+  template <typename R>
+  __device__ __forceinline__ void store_tr(int plane, int par, uint32_t j, R v) const {
+    tr[(size_t)(plane * 2 + par) * stride + j] = S(v);
+  }
+};
+
+// The leading link of a product: its stored rows (12-real), or all of it.
+template <typename F, typename R>
+__device__ __forceinline__ m3<R> lead(const F& f, int mu, int par, uint32_t i) {
+  if constexpr (F::NREAL == 12)
+    return f.template load_rows01<R>(mu, par, i);
+  else
+    return f.template load<R>(mu, par, i);
+}
+
+// L_{mu nu} = (U_mu(x) U_nu(x+mu)) (U_nu(x) U_mu(x+nu))^dag.  12-real storage: rows 0 and 1 of
+// the three products from the stored rows of their first factors; row 2 of the second and of L
+// from the cross product (each is in SU(3)).
+template <typename F, typename R>
+__device__ __forceinline__ m3<R> plaquette_loop(const F& f, const m3<R>& Umu, int mu, int nu, int par, uint32_t i,
+                                                uint32_t ixmu, uint32_t ixnu) {
+  const int opp = par ^ 1;
+  const m3<R> Unu = lead<F, R>(f, nu, par, i);
+  if constexpr (F::NREAL == 12) {
+    const m3<R> G = mul_nn_rows01(Umu, f.template load<R>(nu, opp, ixmu));
+    m3<R> H = mul_nn_rows01(Unu, f.template load<R>(mu, opp, ixnu));
+    reconstruct_row2(H);
+    m3<R> L = mul_na_rows01(G, H);
+    reconstruct_row2(L);
+    return L;
+  } else {
+    const m3<R> G = mul_nn(Umu, f.template load<R>(nu, opp, ixmu));
+    const m3<R> H = mul_nn(Unu, f.template load<R>(mu, opp, ixnu));
+    return mul_na(G, H);
+  }
+}
+
+// i d v for real d
+template <typename R>
+__device__ __forceinline__ cx<R> times_i(R d, cx<R> v) {
+  return mk(-(d * v.im), d * v.re);
+}
+// acc - conj(a) b
+template <typename R>
+__device__ __forceinline__ cx<R> cfms_cn(cx<R> a, cx<R> b, cx<R> acc) {
+  acc.re = fma(-a.re, b.re, acc.re);
+  acc.re = fma(-a.im, b.im, acc.re);
+  acc.im = fma(-a.re, b.im, acc.im);
+  acc.im = fma(a.im, b.re, acc.im);
+  return acc;
+}
+// Im(conj(u) . b) over three components
+template <typename R>
+__device__ __forceinline__ R im_dot3(const cx<R> (&u)[3], const cx<R> (&b)[3]) {
+  R p = u[0].re * b[0].im, m = u[0].im * b[0].re;
+#pragma unroll
+  for (int k = 1; k < 3; ++k) p = fma(u[k].re, b[k].im, p), m = fma(u[k].im, b[k].re, m);
+  return p - m;
+}
+// conj(u) . b over three components
+template <typename R>
+__device__ __forceinline__ cx<R> dot3(const cx<R> (&u)[3], const cx<R> (&b)[3]) {
+  cx<R> s = mk(fma(u[0].re, b[0].re, u[0].im * b[0].im), fma(u[0].re, b[0].im, -(u[0].im * b[0].re)));
+  s = cfma_cn(u[1], b[1], s);
+  return cfma_cn(u[2], b[2], s);
+}
+
+// Ad(U) K = U^dag K U, column by column of U: element (i, j) is conj(u_i) . (K u_j).
+template <typename R>
+__device__ __forceinline__ alg8<R> transport(const m3<R>& U, const alg8<R>& K) {
+  const cx<R> a = mk(K.a[2], K.a[3]), b = mk(K.a[4], K.a[5]), c = mk(K.a[6], K.a[7]);
+  const R d2 = -(K.a[0] + K.a[1]);
+  cx<R> u[3][3], w[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) u[j][k] = U.e[k][j];
+  alg8<R> r;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    // rows of K: (i d0, a, b), (-a*, i d1, c), (-b*, -c*, i d2)
+    w[0] = cfma(b, u[j][2], cfma(a, u[j][1], times_i(K.a[0], u[j][0])));
+    w[1] = cfma(c, u[j][2], cfms_cn(a, u[j][0], times_i(K.a[1], u[j][1])));
+    w[2] = cfms_cn(c, u[j][1], cfms_cn(b, u[j][0], times_i(d2, u[j][2])));
+    if (j == 0) {
+      r.a[0] = im_dot3(u[0], w);
+    } else if (j == 1) {
+      const cx<R> o = dot3(u[0], w);
+      r.a[2] = o.re, r.a[3] = o.im;
+      r.a[1] = im_dot3(u[1], w);
+    } else {
+      const cx<R> o = dot3(u[0], w), q = dot3(u[1], w);
+      r.a[4] = o.re, r.a[5] = o.im;
+      r.a[6] = q.re, r.a[7] = q.im;
+    }
+  }
+  return r;
+}
+
+// The loops below site x in direction nu, K_{mu nu}(x-nu) of the three mu != nu (mu ascending,
+// K_{nu mu} where nu < mu), moved to x: out[k] = Ad(U_nu(x-nu)) K.
+template <typename F, typename S, typename R>
+__device__ __forceinline__ void transported(const F& f, const Loops<S>& K, const Coord& x, const NbOff& o, int nu,
+                                            int par, int Lt, alg8<R> (&out)[3]) {
+  const int opp = par ^ 1, t = x.c[3];
+  const uint32_t iy = cb_index((uint32_t)((int32_t)x.s + sel4(o.dn, nu)));
+  const uint32_t jy = nu == 3 ? K.at(iy, t == 0 ? Lt - 1 : t - 1, t - 1) : K.at(iy, t, t);
+  const int p0 = nu == 0 ? 0 : nu - 1, p1 = nu < 2 ? 3 * nu + (1 - nu) : nu + 1, p2 = nu < 2 ? 2 + 2 * nu : 5;
+  const m3<R> U = f.template load<R>(nu, opp, iy);
+  const alg8<R> k0 = K.template load<R>(p0, opp, jy), k1 = K.template load<R>(p1, opp, jy),
+                k2 = K.template load<R>(p2, opp, jy);
+  out[0] = transport(U, k0);
+  out[1] = transport(U, k1);
+  out[2] = transport(U, k2);
+}
+
+// Anti-Hermitian 3x3 matrix in 9 reals: F_kk = i d[k], F_ij = o[.] for (i,j) = (0,1),
+// (0,2), (1,2), and F_ji = -conj(F_ij).
+template <typename R>
+struct ah9 {
+  R d[3];
+  cx<R> o[3];
+};
+
+// Re tr(A B) of two anti-Hermitian matrices: -sum_k a_k b_k - 2 sum_{i<j} Re(A_ij conj B_ij).
+template <typename R>
+__device__ __forceinline__ R re_tr_ah(const ah9<R>& A, const ah9<R>& B) {
+  R s = 0, t = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    s = fma(A.d[k], B.d[k], s);
+    t = fma(A.o[k].re, B.o[k].re, fma(A.o[k].im, B.o[k].im, t));
+  }
+  return fma(R(-2), t, -s);
+}
+
+// |F|^2 = sum_ij |F_ij|^2 = sum_k d_k^2 + 2 sum_{i<j} |F_ij|^2.
+template <typename R>
+__device__ __forceinline__ R sqnorm_ah(const ah9<R>& A) {
+  R s = 0, t = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    s = fma(A.d[k], A.d[k], s);
+    t = fma(A.o[k].re, A.o[k].re, fma(A.o[k].im, A.o[k].im, t));
+  }
+  return fma(R(2), t, s);
+}
+
+// a + sg b, sg = +-1
+template <typename R>
+__device__ __forceinline__ void add_alg(alg8<R>& a, const alg8<R>& b, R sg = R(1)) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) a.a[q] = fma(sg, b.a[q], a.a[q]);
+}
+// F_{mu nu}(x) = (C - C^dag) / 8 (observables_mpi.cpp:81-82), C the sum of the four leaves: a
+// quarter of the transported loops, their traces (invariant under transport) on the diagonal.
+template <typename F, typename S, typename R>
+__device__ __forceinline__ ah9<R> clover_plane(const F& f, const Loops<S>& K, const Coord& x, const NbOff& o, int mu,
+                                               int nu, int par, uint32_t i, int Lt) {
+  const int opp = par ^ 1, t = x.c[3], plane = plane_of(mu, nu);
+  const int tm = t == 0 ? Lt - 1 : t - 1;
+  const int32_t s = (int32_t)x.s, dmu = sel4(o.dn, mu), dnu = sel4(o.dn, nu);
+  const uint32_t imu = (uint32_t)(s + dmu) >> 1, inu = (uint32_t)(s + dnu) >> 1, imn = (uint32_t)(s + dmu + dnu) >> 1;
+  // only nu can be the time direction (mu < nu)
+  const int tn = nu == 3 ? tm : t, vn = nu == 3 ? t - 1 : t;
+  const uint32_t j0 = K.at(i, t, t), jmu = K.at(imu, t, t), jnu = K.at(inu, tn, vn), jmn = K.at(imn, tn, vn);
+  alg8<R> B = transport(f.template load<R>(nu, par, imn), K.template load<R>(plane, par, jmn));
+  add_alg(B, K.template load<R>(plane, opp, jmu));
+  alg8<R> A = transport(f.template load<R>(mu, opp, imu), B);
+  add_alg(A, transport(f.template load<R>(nu, opp, inu), K.template load<R>(plane, opp, jnu)));
+  add_alg(A, K.template load<R>(plane, par, j0));
+  const R tr = (K.template load_tr<R>(plane, par, j0) + K.template load_tr<R>(plane, par, jmn)) +
+               (K.template load_tr<R>(plane, opp, jmu) + K.template load_tr<R>(plane, opp, jnu));
+  ah9<R> out;
+  out.d[0] = R(0.25) * (A.a[0] + tr);
+  out.d[1] = R(0.25) * (A.a[1] + tr);
+  out.d[2] = R(0.25) * (tr - (A.a[0] + A.a[1]));
+#pragma unroll
+  for (int k = 0; k < 3; ++k) out.o[k] = mk<R>(R(0.25) * A.a[2 + 2 * k], R(0.25) * A.a[3 + 2 * k]);
+  return out;
+}
+
+}  // namespace qcb

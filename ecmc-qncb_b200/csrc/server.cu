@@ -5,8 +5,8 @@
 // HBM budget) has room for it, so later arrivals never overtake earlier ones.  Each tick
 // builds one descriptor per admitted job (a sweeps job advances by quantum_sweeps sweeps, a
 // flow job by quantum_steps RK3 steps, each lattice with its own level count), runs the
-// sweeps jobs in one persistent heatbath launch and the flow jobs in one persistent flow
-// launch, measures the jobs that finished (batched plaquette / clover reductions), copies the
+// sweeps jobs in one persistent heatbath launch and the flow jobs together stage by stage (the
+// loops and the update of all of them in one launch each), measures the jobs that finished (batched plaquette / clover reductions), copies the
 // results back, and then admits the next arrivals.
 #include <string.h>
 
@@ -21,6 +21,7 @@
 
 #include "api_internal.h"
 #include "batch.h"
+#include "flow.h"
 
 using namespace qcb;
 
@@ -121,6 +122,10 @@ struct qcb_server {
   uint32_t* h_status = nullptr;
   double* d_scratch = nullptr;
   size_t scratch_cap = 0;
+  // flow and clover: the loop buffer (outside the arena), the plans' device arrays
+  LoopBuf loops;
+  char* d_flow = nullptr;
+  size_t flow_cap = 0;
   double* d_out = nullptr;
   double* h_out = nullptr;
   int cap = 0;  // descriptor capacity (max_jobs)
@@ -154,11 +159,26 @@ void finish(qcb_server* s, Job* j, int status, double plaq, double t, double q, 
   delete j;
 }
 
+// Uploads a flow plan (its descriptors, then its prefix sums and the clover's) after `at` bytes
+// of the server's flow array, which grows as needed; *end is where the next may go.
+cudaError_t upload_plan(qcb_server* s, const FlowPlan& p, size_t at, size_t* end, FlowLat** lats, uint32_t** prefix) {
+  const size_t nl = p.lats.size() * sizeof(FlowLat), np = p.prefix.size() * sizeof(uint32_t),
+               nq = p.qe_prefix.size() * sizeof(uint32_t);
+  *lats = (FlowLat*)(s->d_flow + at);
+  *prefix = (uint32_t*)(s->d_flow + at + nl);
+  *end = (at + nl + np + nq + 255) & ~(size_t)255;
+  cudaError_t e = cudaMemcpyAsync(*lats, p.lats.data(), nl, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(*prefix, p.prefix.data(), np, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(*prefix + p.prefix.size(), p.qe_prefix.data(), nq, cudaMemcpyHostToDevice, s->stream);
+  return e;
+}
+size_t plan_bytes(const FlowPlan& p) {
+  return p.lats.size() * sizeof(FlowLat) + (p.prefix.size() + p.qe_prefix.size()) * sizeof(uint32_t) + 256;
+}
+
 // One tick over the admitted jobs.  Returns a CUDA error to fail all jobs of the tick.
-// The sweeps jobs' descriptors come first, then the flow jobs'.  The two groups run as two
-// persistent launches (heatbath kernel, then flow kernel), so each launch keeps one code
-// body in the instruction cache: on the 20 req/s stream this completes 5.9 jobs/s against
-// 5.4 for one mixed launch over both groups.
+// The sweeps jobs' descriptors come first, then the flow jobs'.
 cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finishing_status) {
   const int n = (int)act.size();
   const uint32_t tile = (uint32_t)s->cfg.tile;
@@ -169,11 +189,11 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
   const int nh = (int)order.size();
   for (int k = 0; k < n; ++k)
     if (act[k]->spec.kind != QCB_JOB_SWEEPS) order.push_back(k);
-  uint32_t lev_h = 0, lev_f = 0;
-  uint32_t* pre_h = s->h_prefix;           // nh + 1 entries
-  uint32_t* pre_f = s->h_prefix + nh + 1;  // n - nh + 1 entries
+  uint32_t lev_h = 0;
+  int steps = 0;
+  uint32_t* pre_h = s->h_prefix;  // nh + 1 entries
   pre_h[0] = 0;
-  pre_f[0] = 0;
+  std::vector<FlowItem> flows;
   std::vector<int> units(n, 0);
   for (int p = 0; p < n; ++p) {
     const int k = order[p];
@@ -190,7 +210,6 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
     if (j->spec.kind == QCB_JOB_SWEEPS) {
       const int q = std::min(s->cfg.quantum_sweeps, j->spec.n_sweeps - j->done_units);
       units[k] = q;
-      d.kind = BATCH_HB;
       d.links = L->dev.links;
       d.beta = j->spec.beta;
       d.k0 = (uint32_t)j->spec.seed;
@@ -207,53 +226,91 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
       }
       const int q = std::min(s->cfg.quantum_steps, j->spec.n_steps - j->done_units);
       units[k] = q;
-      d.kind = BATCH_FLOW;
       const bool odd = (j->done_units & 1) != 0;
       d.links = odd ? j->fw1 : j->fw0;
-      d.work = odd ? j->fw0 : j->fw1;
-      d.acc = j->acc;
-      d.ntiles = flow_items_per_tile(s->cfg.precision) * cdiv(d.g.Vh, tile);
-      d.nlev = 3u * (uint32_t)q;
-      d.eps = j->spec.eps;
+      FlowItem it;
+      it.L = L->dev;
+      it.L.links = d.links;
+      it.b = odd ? j->fw0 : j->fw1;
+      it.acc = j->acc;
+      it.eps = j->spec.eps;
+      it.tile = tile;
+      it.nsteps = q;
+      if (q > 0) flows.push_back(it);
+      steps = std::max(steps, q);
     }
-    if (d.nlev == 0) {  // nothing to run this tick (measurement only): no work items
-      d.kind = BATCH_NONE;
-      d.ntiles = 0;
-    }
-    if (p < nh) {
+    if (p < nh) {  // a job with nothing to run this tick (measurement only) has no work items
+      if (d.nlev == 0) d.ntiles = 0;
       lev_h = std::max(lev_h, d.nlev);
       pre_h[p + 1] = pre_h[p] + d.ntiles;
-    } else {
-      lev_f = std::max(lev_f, d.nlev);
-      pre_f[p - nh + 1] = pre_f[p - nh] + d.ntiles;
     }
   }
   cudaError_t e = cudaMemcpyAsync(s->d_desc, s->h_desc, n * sizeof(BatchLat), cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(s->d_prefix, s->h_prefix, (n + 2) * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
+    e = cudaMemcpyAsync(s->d_prefix, s->h_prefix, (nh + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->d_done, 0, n * sizeof(uint32_t), s->stream);
   if (e != cudaSuccess) return e;
-  auto run_of = [&](int first, int count, const uint32_t* dprefix, uint32_t nlevels, uint32_t per_level) {
-    BatchRun run;
-    run.lats = s->d_desc + first;
-    run.prefix = dprefix;
-    run.nlat = count;
-    run.nlevels = nlevels;
-    run.per_level = per_level;
-    run.done = s->d_done + first;
-    run.status = s->d_status;
-    run.n_hits = 1;  // every descriptor carries its own n_hits / eps
-    run.eps = 0.02;
-    return run;
-  };
   if (nh > 0 && lev_h > 0 && pre_h[nh] > 0) {
-    e = launch_batch(BATCH_HB, run_of(0, nh, s->d_prefix, lev_h, pre_h[nh]), s->cfg.precision, s->cfg.storage, 128,
-                     0, s->stream);
+    BatchRun run;
+    run.lats = s->d_desc;
+    run.prefix = s->d_prefix;
+    run.nlat = nh;
+    run.nlevels = lev_h;
+    run.per_level = pre_h[nh];
+    run.done = s->d_done;
+    run.status = s->d_status;
+    run.n_hits = 1;  // every descriptor carries its own n_hits
+    e = launch_batch(run, s->cfg.precision, s->cfg.storage, 128, 0, s->stream);
     if (e != cudaSuccess) return e;
   }
-  if (n > nh && lev_f > 0 && pre_f[n - nh] > 0) {
-    e = launch_batch(BATCH_FLOW, run_of(nh, n - nh, s->d_prefix + nh + 1, lev_f, pre_f[n - nh]), s->cfg.precision,
-                     s->cfg.storage, 128, 0, s->stream);
+  // the jobs that finish in this tick (a cancel is looked at once)
+  std::vector<char> last(n, 0);
+  for (int k = 0; k < n; ++k) {
+    const int total = (act[k]->spec.kind == QCB_JOB_SWEEPS) ? act[k]->spec.n_sweeps : act[k]->spec.n_steps;
+    last[k] = act[k]->done_units + units[k] >= total || act[k]->cancel;
+  }
+  // the flow jobs' steps, and the clover of those that finish
+  std::vector<FlowItem> done;
+  for (int p = nh; p < n; ++p) {
+    const Job* j = act[order[p]];
+    const int u = j->done_units + units[order[p]];
+    if (!last[order[p]]) continue;
+    FlowItem it;
+    it.L = j->spec.lat->dev;
+    it.L.links = (u & 1) ? j->fw1 : j->fw0;
+    it.b = it.acc = nullptr;
+    it.eps = 0.0;
+    it.tile = tile;
+    it.nsteps = 1;  // its loops are computed once
+    done.push_back(it);
+  }
+  FlowPlan fp, qp;
+  FlowLat* d_lats[2] = {nullptr, nullptr};
+  uint32_t* d_pre[2] = {nullptr, nullptr};
+  if (!flows.empty() || !done.empty()) {
+    size_t w0 = 0, l0 = 0, w1 = 0, l1 = 0;
+    flow_plan_bytes(flows, &w0, &l0);
+    flow_plan_bytes(done, &w1, &l1);
+    e = loops_reserve(&s->loops, std::max(w0, w1), std::max(l0, l1));
+    if (e != cudaSuccess) return e;
+    fp = flow_plan(flows, s->loops);
+    qp = flow_plan(done, s->loops);
+    const size_t need = plan_bytes(fp) + plan_bytes(qp);
+    if (need > s->flow_cap) {
+      cudaStreamSynchronize(s->stream);
+      cudaFree(s->d_flow);
+      s->d_flow = nullptr;
+      s->flow_cap = 0;
+      e = cudaMalloc(&s->d_flow, 2 * need);
+      if (e != cudaSuccess) return e;
+      s->flow_cap = 2 * need;
+    }
+    size_t end = 0;
+    e = upload_plan(s, fp, 0, &end, &d_lats[0], &d_pre[0]);
+    if (e == cudaSuccess) e = upload_plan(s, qp, end, &end, &d_lats[1], &d_pre[1]);
+    if (e != cudaSuccess) return e;
+    uint64_t launches = 0;
+    e = run_flow_plan(fp, d_lats[0], d_pre[0], s->cfg.precision, s->cfg.storage, 0, steps, s->stream, &launches);
     if (e != cudaSuccess) return e;
   }
   for (int k = 0; k < n; ++k) act[k]->done_units += units[k];
@@ -266,8 +323,7 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
   for (int p = 0; p < n; ++p) {
     const int k = order[p];
     Job* j = act[k];
-    const int total = (j->spec.kind == QCB_JOB_SWEEPS) ? j->spec.n_sweeps : j->spec.n_steps;
-    if (j->done_units < total && !j->cancel) continue;
+    if (!last[k]) continue;
     BatchLat d = s->h_desc[p];
     if (j->spec.kind == QCB_JOB_SWEEPS) {
       mh.push_back(d);
@@ -282,26 +338,23 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
   if (m1 + m2 == 0) return cudaSuccess;
   std::vector<BatchLat> md(mh);
   md.insert(md.end(), mf.begin(), mf.end());
-  std::vector<uint32_t> rp(m1 + m2 + 2, 0);  // prefix of the sweeps list, then of the flow list
+  std::vector<uint32_t> rp(m1 + 1, 0);  // prefix of the sweeps list
   for (int a = 0; a < m1; ++a) rp[a + 1] = rp[a] + cdiv(mh[a].g.V, (uint32_t)batch_red_sites());
-  const uint32_t n1 = rp[m1];
-  uint32_t* rf = &rp[m1 + 1];
-  rf[0] = 0;
-  for (int a = 0; a < m2; ++a) rf[a + 1] = rf[a] + cdiv(mf[a].g.V, (uint32_t)batch_red_sites());
-  const uint32_t n2 = rf[m2];
-  const size_t need = 2 * (size_t)std::max(n1, n2);
+  const uint32_t n1 = rp[m1], n2 = m2 ? qp.qe_prefix.back() : 0;
+  const size_t need = std::max((size_t)n1, 2 * (size_t)n2);
   if (need > s->scratch_cap) {
     // grow the reduction scratch (outside the arena; rare)
     cudaStreamSynchronize(s->stream);
     cudaFree(s->d_scratch);
     s->d_scratch = nullptr;
+    s->scratch_cap = 0;
     e = cudaMalloc(&s->d_scratch, need * sizeof(double));
     if (e != cudaSuccess) return e;
     s->scratch_cap = need;
   }
   // measurement descriptors and prefixes go after the tick's ones
   BatchLat* dm = s->d_desc + s->cap;
-  uint32_t* dp = s->d_prefix + 2 * s->cap + 4;
+  uint32_t* dp = s->d_prefix + s->cap + 2;
   e = cudaMemcpyAsync(dm, md.data(), md.size() * sizeof(BatchLat), cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(dp, rp.data(), rp.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
@@ -309,9 +362,12 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
   // plaquettes -> d_out[0 .. m1), (Q, E) pairs -> d_out[m1 .. m1 + 2 m2)
   if (m1)
     e = launch_batch_plaquette(dm, dp, m1, n1, s->cfg.precision, s->cfg.storage, s->d_scratch, s->d_out, s->stream);
-  if (e == cudaSuccess && m2)
-    e = launch_batch_qe(dm + m1, dp + m1 + 1, m2, n2, s->cfg.precision, s->cfg.storage, s->d_scratch,
-                        s->d_out + m1, s->stream);
+  if (e == cudaSuccess && m2) {
+    uint64_t launches = 0;
+    e = run_qe_plan(qp, d_lats[1], d_pre[1], s->cfg.precision, s->cfg.storage, 0, s->d_scratch, s->stream, &launches);
+    if (e == cudaSuccess)
+      e = launch_batch_qe(dm + m1, d_pre[1] + qp.prefix.size(), m2, n2, s->d_scratch, s->d_out + m1, s->stream);
+  }
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(s->h_out, s->d_out, (m1 + 2 * m2) * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
   for (int a = 0; a < m1; ++a) finishing_status[kh[a]] = a;
@@ -449,7 +505,7 @@ int qcb_server_create(qcb_ctx* ctx, const qcb_server_config* cfg, qcb_server** o
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&s->d_desc, 2 * (size_t)s->cap * sizeof(BatchLat)) != cudaSuccess ||
       cudaMallocHost(&s->h_desc, (size_t)s->cap * sizeof(BatchLat)) != cudaSuccess ||
-      cudaMalloc(&s->d_prefix, (3 * (size_t)s->cap + 8) * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&s->d_prefix, (2 * (size_t)s->cap + 8) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMallocHost(&s->h_prefix, (size_t)(s->cap + 2) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&s->d_done, (size_t)s->cap * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&s->d_status, 4 * sizeof(uint32_t)) != cudaSuccess ||
@@ -573,6 +629,8 @@ int qcb_server_destroy(qcb_server* s) {
   cudaFree(s->d_status);
   cudaFreeHost(s->h_status);
   cudaFree(s->d_scratch);
+  cudaFree(s->loops.p);
+  cudaFree(s->d_flow);
   cudaFree(s->d_out);
   cudaFreeHost(s->h_out);
   cudaStreamDestroy(s->stream);

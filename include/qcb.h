@@ -153,7 +153,9 @@ int qcb_translate(qcb_lattice* lat, const int shift[4]);
  * sum_{x, mu<nu} Re tr P_{mu nu}(x) / 3, divided by 6V.  FP64 accumulation. */
 int qcb_plaquette(qcb_lattice* lat, double* out);
 /* topo_q_e_clover_global (observables_mpi.cpp:61-150): clover charge Q (total) and energy
- * density E = (1/V) sum_x 1/2 sum_{mu<nu} |F_{mu nu}|^2 with F = (C - C^dagger)/8. */
+ * density E = (1/V) sum_x 1/2 sum_{mu<nu} |F_{mu nu}|^2 with F = (C - C^dagger)/8.  Uses the
+ * context's plaquette-loop work space, as the Wilson flow does (allocated on first use, at most
+ * 1 GiB or two time slices' loops, less when that much is not free). */
 int qcb_topo_qe(qcb_lattice* lat, double* q, double* e);
 
 /* ---- allocation-free plaquette ---------------------------------------------------------
@@ -188,10 +190,13 @@ int qcb_flow_steps(qcb_lattice* lat, double eps, int n);
 /* ---- batches of lattices ------------------------------------------------------------
  * No single counterpart in the reference (it runs one lattice per process,
  * src/bin/gauge_hb_ncb.cpp:18-201).  A batch advances many independent lattices of any
- * sizes (same context, precision and storage) in one persistent cooperative launch per
- * phase: work items (lattice, level, tile of sites) run level-major, each lattice's levels
- * in order, different lattices overlapping.  Every result is bit-identical to running the
- * lattice alone through qcb_heatbath / qcb_flow_steps with the same seed and sweep counter.
+ * sizes (same context, precision and storage).  The heatbath is one persistent cooperative
+ * launch: work items (lattice, level, tile of sites) run level-major, each lattice's levels
+ * in order, different lattices overlapping.  The flow and the clover run stage by stage, each
+ * launch covering the lattices whose plaquette loops fit into the batch's loop buffer together
+ * (at most 1 GiB, or two time slices of the largest lattice; allocated on first use).  Every
+ * result is bit-identical to running the lattice alone through qcb_heatbath / qcb_flow_steps
+ * with the same seed and sweep counter.
  * The batch borrows the lattices: they must outlive it. */
 typedef struct qcb_batch qcb_batch;
 int qcb_batch_create(qcb_ctx* ctx, int n, qcb_lattice* const* lats, qcb_batch** out);
@@ -204,9 +209,9 @@ int qcb_batch_get_tiles(qcb_batch* b, int* hb_tile, int* flow_tile);
  * sweep_offsets[l] .. sweep_offsets[l] + n_sweeps - 1 (one launch).  Asynchronous. */
 int qcb_batch_heatbath(qcb_batch* b, const double* betas, int n_sweeps, int n_hits, const uint64_t* seeds,
                        const uint64_t* sweep_offsets);
-/* n RK3 steps of size eps on every lattice, in place (one launch). */
+/* n RK3 steps of size eps on every lattice, in place. */
 int qcb_batch_flow_steps(qcb_batch* b, double eps, int n_steps);
-/* Per-lattice mean plaquette / clover (Q, E) of every lattice (one launch each). */
+/* Per-lattice mean plaquette / clover (Q, E) of every lattice. */
 int qcb_batch_plaquette(qcb_batch* b, double* out);
 int qcb_batch_topo_qe(qcb_batch* b, double* q, double* e);
 /* A whole batched workload as one CUDA graph: n_sweeps heatbath sweeps in place, the mean
@@ -288,9 +293,9 @@ int qcb_wait_selftest(qcb_ctx* ctx, double limit_s, uint32_t* timeouts, uint32_t
  * No counterpart in the reference.  A request server with continuous batching: jobs
  * (Wilson-flow measurements and generate-N-sweeps runs on resident lattices of any sizes)
  * are admitted in arrival order while the server's device work-space arena (its HBM budget)
- * and job slots allow; every tick advances every admitted job by a quantum of sweeps or RK3
- * steps in ONE persistent launch (heatbath and flow items mixed), measures the jobs that
- * finish, and admits new arrivals at the tick boundary.  A job's result does not depend on
+ * and job slots allow; every tick advances every admitted sweeps job by a quantum of sweeps in
+ * one persistent launch and every flow job by a quantum of RK3 steps, the jobs together stage by
+ * stage, measures the jobs that finish, and admits new arrivals at the tick boundary.  A job's result does not depend on
  * what else runs with it (counter-based random numbers, per-lattice arithmetic).  The
  * server runs its own scheduler thread and CUDA stream on the context's device; a job's
  * lattice is lent to the server from submission until its result is returned (a sweeps job
