@@ -10,10 +10,10 @@
 //
 // Measured per RK3 step on 32^4, against kernels that multiplied out the staples of every link
 // (twelve products each; in FP32 ten, with one product shared by a plane's two links): FP64
-// 18-real 2.65 -> 2.06 ms, FP32 12-real 1.08 -> 0.97 ms.  Of a stage, the loops take a third and the
+// 18-real 2.65 -> 1.93 ms, FP32 12-real 1.08 -> 0.92 ms.  Of a stage, the loops take a third and the
 // update two thirds (FP32 215 us, 0.71-0.85 GB of DRAM traffic, 56% issue; FP64 420-480 us, 56% of
 // the DRAM rate).  A smaller loop buffer, whose rounds of slices would stay in L2, costs more in
-// half-filled last waves than it saves: 110, 70 and 24 MB make the FP32 step 1.05, 1.09 and 1.24 ms.
+// half-filled last waves than it saves: 110, 70 and 24 MB made the FP32 step 1.05, 1.09 and 1.24 ms where 1 GiB made it 0.97.
 #include "flow_launch.cuh"
 #include "flow_link.cuh"
 
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_FLOW_MINB32
   constexpr int NC = AlgStore<S>::NC;
   __shared__ V moved[12][NC][32];  // [3 nu + k]: loop k of direction nu, moved to x
   const uint32_t n = (uint32_t)(L.t1 - L.t0) * K.half, first = (b >> 1) * L.tile;
-  const int par = (int)(b & 1), w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int par = (int)(b & 1), w = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const R eps = R(S(L.eps));
   for (uint32_t k0 = 0; k0 < L.tile && first + k0 < n; k0 += 32) {
     const uint32_t k = first + k0 + lane;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_FLOW_MINB32
       const Coord x = cb_coord(L.g, par, i);
       {
         alg8<R> m[3];
-        transported<F, S, R>(src, K, x, nb_offsets(L.g, x), w, par, L.g.L[3], m);
+        transported<F, S, R>(L.g, src, K, x, w, par, m);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           V v[NC];

@@ -172,11 +172,11 @@ __device__ __forceinline__ alg8<R> transport(const m3<R>& U, const alg8<R>& K) {
 // The loops below site x in direction nu, K_{mu nu}(x-nu) of the three mu != nu (mu ascending,
 // K_{nu mu} where nu < mu), moved to x: out[k] = Ad(U_nu(x-nu)) K.
 template <typename F, typename S, typename R>
-__device__ __forceinline__ void transported(const F& f, const Loops<S>& K, const Coord& x, const NbOff& o, int nu,
-                                            int par, int Lt, alg8<R> (&out)[3]) {
-  const int opp = par ^ 1, t = x.c[3];
-  const uint32_t iy = cb_index((uint32_t)((int32_t)x.s + sel4(o.dn, nu)));
-  const uint32_t jy = nu == 3 ? K.at(iy, t == 0 ? Lt - 1 : t - 1, t - 1) : K.at(iy, t, t);
+__device__ __forceinline__ void transported(const Geom& g, const F& f, const Loops<S>& K, const Coord& x, int nu,
+                                            int par, alg8<R> (&out)[3]) {
+  const int opp = par ^ 1, t = x.c[3], L = g.L[nu], d = g.str[nu];
+  const uint32_t iy = cb_index((uint32_t)((int32_t)x.s + (sel4(x.c, nu) == 0 ? (L - 1) * d : -d)));
+  const uint32_t jy = nu == 3 ? K.at(iy, t == 0 ? L - 1 : t - 1, t - 1) : K.at(iy, t, t);
   const int p0 = nu == 0 ? 0 : nu - 1, p1 = nu < 2 ? 3 * nu + (1 - nu) : nu + 1, p2 = nu < 2 ? 2 + 2 * nu : 5;
   const m3<R> U = f.template load<R>(nu, opp, iy);
   const alg8<R> k0 = K.template load<R>(p0, opp, jy), k1 = K.template load<R>(p1, opp, jy),

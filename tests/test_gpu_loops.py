@@ -42,6 +42,18 @@ def test_flow_step_and_clover_match_oracle(ctx, dims, prec, nr):
     f.close()
 
 
+@pytest.mark.parametrize("eps", [0.11, 0.6])
+def test_large_steps_match_oracle(ctx, eps):
+    """Steps at which some (0.11) and all (0.6) exponentials need every term of the series."""
+    dims = (4, 6, 4, 6)
+    u = orc.hot_philox(dims, 77)
+    f = qcb.GaugeField(ctx, dims)
+    f.set_links(u)
+    _lib.check(_lib.lib().qcb_flow_steps(f.h, eps, 1))
+    assert np.abs(f.get_links() - orc.flow_steps(u, dims, eps, 1)).max() < 1e-12
+    f.close()
+
+
 def test_rounds_of_time_slices_match_slabs(ctx):
     """64^3 x 10 in FP64 has 1.13 GB of loops: rounds of eight and two slices through the buffer,
     the slice before a round kept from the one before it.  Slabs of two slices hold theirs whole;
