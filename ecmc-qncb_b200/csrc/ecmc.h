@@ -16,6 +16,7 @@ struct EcmcLaunch {
   double2* links;        // FP64 array-of-structures copy: link (s, mu) = 9 double2 at (4 s + mu) * 9
   qcb_ecmc_chain* chains;
   uint32_t n_chains;
+  uint32_t per_warp;     // chains per warp (set by launch_ecmc_sample)
   int L[4];              // lattice extents
   int nb[4];             // blocks per direction (L[d] / l)
   int cum[4];            // cumulative shift of the field's frame, in [0, L[d])

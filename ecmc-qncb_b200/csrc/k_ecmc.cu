@@ -124,6 +124,21 @@ __device__ __noinline__ M haar(Stream& g) {
   return haar_from_normals(n);
 }
 
+// -log(u) theta: a budget drawn from the exponential of mean theta (out of line: rare)
+__device__ __noinline__ double exp_draw(Stream& g, double theta) { return -log(g.uni()) * theta; }
+
+// random_site (ecmc_mpi_cb.cpp:359-367): local coordinates 1 .. l-2 (padded 2 .. L-1), then the
+// direction and the sense of rotation (out of line: at the start and at site refreshes only)
+__device__ __noinline__ void random_site(Stream& g, int l, int out[6]) {
+#pragma unroll 1
+  for (int d = 0; d < 4; ++d) out[d] = 1 + (int)(g.uni() * (double)(l - 2));
+  out[4] = (int)(g.uni() * 4.0);
+  out[5] = g.uni() < 0.5 ? -1 : 1;
+}
+
+// c mod L (out of line: the divisions of the seven site computations were a fifth of the loop's code)
+__device__ __noinline__ int reduce_far(int c, int L) { return ((c % L) + L) % L; }
+
 // The block of one chain: local coordinates lc (in [-1, l] for every link a chain at an
 // active link reads; -1 and l are the neighbouring blocks' faces, the reference's halo) sit
 // at stored site b_d l + lc_d - cum_d (mod L_d), with base_d = b_d l - cum_d in
@@ -131,18 +146,22 @@ __device__ __noinline__ M haar(Stream& g) {
 struct Block {
   int L[4], base[4], l;
   __device__ __forceinline__ uint32_t site(const int lc[4]) const {
-    uint32_t s = 0;
+    int c[4];
+    bool far = false;
 #pragma unroll
-    for (int d = 3; d >= 0; --d) {
-      int c = base[d] + lc[d];
-      if (c < 0) c += L[d];
-      else if (c >= L[d]) c -= L[d];
-      // a chain only leaves [-1, l] after a lift onto a frozen link, which takes a rounding
-      // accident in the lift's tower sampling; the full reduction keeps any position in bounds
-      if ((unsigned)c >= (unsigned)L[d]) c = ((c % L[d]) + L[d]) % L[d];
-      s = s * (uint32_t)L[d] + (uint32_t)c;
+    for (int d = 0; d < 4; ++d) {
+      c[d] = base[d] + lc[d];
+      if (c[d] < 0) c[d] += L[d];
+      else if (c[d] >= L[d]) c[d] -= L[d];
+      far = far || (unsigned)c[d] >= (unsigned)L[d];
     }
-    return s;
+    // a chain only leaves [-1, l] after a lift onto a frozen link, which takes a rounding
+    // accident in the lift's tower sampling; the full reduction keeps any position in bounds
+    if (far) {
+#pragma unroll
+      for (int d = 0; d < 4; ++d) c[d] = reduce_far(c[d], L[d]);
+    }
+    return (uint32_t)c[0] + (uint32_t)L[0] * ((uint32_t)c[1] + (uint32_t)L[1] * ((uint32_t)c[2] + (uint32_t)L[2] * (uint32_t)c[3]));
   }
   // GeometryCB::is_frozen in block-local terms: the halo (outside [0, l)) and the links
   // leaving local coordinate 0 in a direction d != mu.
@@ -325,22 +344,6 @@ __device__ __noinline__ double2 lift_trace_lane(const double2* L, Factor fa, Fac
   return make_double2(t, n);
 }
 
-// su2_quaternion_to_su3 (src/su3/utils.cpp:33-45) of (x0, x1, x2, x3) in subgroup (i, j).
-__device__ M embed(const double x[4], int i, int j) {
-  M X;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) X.e[a][b] = mk(0.0, 0.0);
-  const int k = 3 - i - j;
-  X.e[k][k] = mk(1.0, 0.0);
-  X.e[i][i] = mk(x[0], x[3]);
-  X.e[j][j] = mk(x[0], -x[3]);
-  X.e[i][j] = mk(x[2], x[1]);
-  X.e[j][i] = mk(-x[2], x[1]);
-  return X;
-}
-
 // q (9 double2) = element iset of a chain's set (ecmc_set / random_SU3_epsilon,
 // src/su3/utils.cpp:66-127: set[0] = 1, set[2p+1] = the product of (sqrt(1 - eps^2), eps r/|r|)
 // embedded in (0,1), (0,2), (1,2) with r uniform in (-1/2, 1/2)^3, set[2p+2] = its adjoint),
@@ -359,8 +362,21 @@ __device__ __noinline__ void set_words(u32x4* w, uint32_t a, uint32_t b, uint32_
   *w = philox4x32_10(cc, k0, k1);
 }
 
-__device__ __noinline__ void set_elem(double2* q, double eps, uint32_t k0, uint32_t k1, uint32_t c, uint32_t call,
-                                      uint32_t gen, int iset) {
+// The quaternion (x1, x2, x3) of embedding `which` from its three uniforms.
+__device__ __forceinline__ void set_quat(const uint32_t w[3], double eps, double x[3]) {
+  double r[3];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) r[t] = ((double)w[t] + 0.5) * 2.3283064365386963e-10 - 0.5;
+  const double norm = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) x[t] = eps * r[t] / norm;
+}
+
+// With three or more lanes per chain, lane s of the first three (the others repeat them) draws the
+// words 3p + s and forms embedding s; the quaternions go round by shuffles.  x0 = sqrt(1 - eps^2).
+template <int GROUP>
+__device__ __noinline__ void set_elem(double2* q, double eps, double x0, uint32_t k0, uint32_t k1, uint32_t c,
+                                      uint32_t call, uint32_t gen, int iset, unsigned gmask, int lane0, int s3) {
   M Mx;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -368,28 +384,47 @@ __device__ __noinline__ void set_elem(double2* q, double eps, uint32_t k0, uint3
     for (int b = 0; b < 3; ++b) Mx.e[a][b] = mk(a == b ? 1.0 : 0.0, 0.0);
   if (iset != 0) {
     const uint32_t p = (uint32_t)(iset - 1) >> 1;
-    double r[12];
-    u32x4 w[3];
+    double x[3][3];
+    if (GROUP == 1) {
+      u32x4 w[3];
 #pragma unroll 1
-    for (uint32_t j = 0; j < 3; ++j) set_words(&w[j], 3 * p + j, c, call, ECMC_SETC ^ (gen & 0xFFFFu), k0, k1);
+      for (uint32_t j = 0; j < 3; ++j) set_words(&w[j], 3 * p + j, c, call, ECMC_SETC ^ (gen & 0xFFFFu), k0, k1);
+      const uint32_t w0[3] = {w[0].v[0], w[0].v[1], w[0].v[2]}, w1[3] = {w[0].v[3], w[1].v[0], w[1].v[1]},
+                     w2[3] = {w[1].v[2], w[1].v[3], w[2].v[0]};
+      set_quat(w0, eps, x[0]);
+      set_quat(w1, eps, x[1]);
+      set_quat(w2, eps, x[2]);
+    } else {
+      u32x4 w;
+      set_words(&w, 3 * p + (uint32_t)s3, c, call, ECMC_SETC ^ (gen & 0xFFFFu), k0, k1);
+      const int before = lane0 + (s3 > 0 ? s3 - 1 : 0);
+      const uint32_t b2 = __shfl_sync(gmask, w.v[2], before), b3 = __shfl_sync(gmask, w.v[3], before);
+      const uint32_t m[3] = {s3 == 0 ? w.v[0] : (s3 == 1 ? b3 : b2), s3 == 0 ? w.v[1] : (s3 == 1 ? w.v[0] : b3),
+                             s3 == 0 ? w.v[2] : (s3 == 1 ? w.v[1] : w.v[0])};
+      double y[3];
+      set_quat(m, eps, y);
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
+      for (int s = 0; s < 3; ++s)
 #pragma unroll
-      for (int t = 0; t < 4; ++t) r[4 * j + t] = ((double)w[j].v[t] + 0.5) * 2.3283064365386963e-10 - 0.5;
-    const int sub[3][2] = {{0, 1}, {0, 2}, {1, 2}};
+        for (int t = 0; t < 3; ++t) x[s][t] = __shfl_sync(gmask, y[t], lane0 + s);
+    }
+    // identity x E01 x E02 x E12, the columns' exact zeros and ones left out
+    Z Eii = mk(x0, x[0][2]), Ejj = mk(x0, -x[0][2]), Eij = mk(x[0][1], x[0][0]), Eji = mk(-x[0][1], x[0][0]);
+    Mx.e[0][0] = Eii, Mx.e[0][1] = Eij, Mx.e[1][0] = Eji, Mx.e[1][1] = Ejj;
+    Eii = mk(x0, x[1][2]), Ejj = mk(x0, -x[1][2]), Eij = mk(x[1][1], x[1][0]), Eji = mk(-x[1][1], x[1][0]);
 #pragma unroll
-    for (int s = 0; s < 3; ++s) {
-      const double norm = sqrt(r[3 * s] * r[3 * s] + r[3 * s + 1] * r[3 * s + 1] + r[3 * s + 2] * r[3 * s + 2]);
-      const double x0 = sqrt(1 - eps * eps), x1 = eps * r[3 * s] / norm, x2 = eps * r[3 * s + 1] / norm,
-                   x3 = eps * r[3 * s + 2] / norm;
-      const int i = sub[s][0], j = sub[s][1];
-      const Z Eii = mk(x0, x3), Ejj = mk(x0, -x3), Eij = mk(x2, x1), Eji = mk(-x2, x1);
+    for (int row = 0; row < 2; ++row) {
+      const Z a = Mx.e[row][0];
+      Mx.e[row][0] = cmul(a, Eii);
+      Mx.e[row][2] = cmul(a, Eij);
+    }
+    Mx.e[2][0] = Eji, Mx.e[2][2] = Ejj;
+    Eii = mk(x0, x[2][2]), Ejj = mk(x0, -x[2][2]), Eij = mk(x[2][1], x[2][0]), Eji = mk(-x[2][1], x[2][0]);
 #pragma unroll
-      for (int row = 0; row < 3; ++row) {
-        const Z a = Mx.e[row][i], b = Mx.e[row][j];
-        Mx.e[row][i] = cfma(b, Eji, cmul(a, Eii));
-        Mx.e[row][j] = cfma(b, Ejj, cmul(a, Eij));
-      }
+    for (int row = 0; row < 3; ++row) {
+      const Z a = Mx.e[row][1], b = Mx.e[row][2];
+      Mx.e[row][1] = row < 2 ? cfma(b, Eji, cmul(a, Eii)) : cmul(b, Eji);
+      Mx.e[row][2] = row < 2 ? cfma(b, Ejj, cmul(a, Eij)) : cmul(b, Ejj);
     }
   }
   const bool adj = iset != 0 && (iset & 1) == 0;
@@ -409,10 +444,9 @@ __device__ __noinline__ void set_elem(double2* q, double eps, uint32_t k0, uint3
 template <int GROUP, int MINB>
 __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunch a) {
   static_assert(GROUP == 1 || GROUP == 3 || GROUP == 6, "a chain's lanes split its six staples evenly");
-  constexpr int PER_WARP = 32 / GROUP;  // chains per warp; 32 % GROUP lanes stay idle
   const int lane = threadIdx.x & 31, slot = lane / GROUP, sub = lane - slot * GROUP, lane0 = slot * GROUP;
-  const uint32_t c = (blockIdx.x * ECMC_WARPS + (threadIdx.x >> 5)) * PER_WARP + slot;
-  if (slot >= PER_WARP || c >= a.n_chains) return;
+  const uint32_t c = (blockIdx.x * ECMC_WARPS + (threadIdx.x >> 5)) * a.per_warp + slot;
+  if (slot >= (int)a.per_warp || c >= a.n_chains) return;  // the warp's other lanes stay idle
   const unsigned gmask = GROUP == 1 ? (1u << lane) : (((1u << GROUP) - 1u) << lane0);
   qcb_ecmc_chain& rec = a.chains[c];
   Block blk;
@@ -442,14 +476,15 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
   int status = 0;  // the record keeps the bits of the latest call
   M R;
   if (!rec.initialized) {
-    // random_site (ecmc_mpi_cb.cpp:359-367): local coordinates 1 .. l-2 (padded 2 .. L-1)
+    int at[6];
+    random_site(g, l, at);
 #pragma unroll
-    for (int d = 0; d < 4; ++d) lc[d] = 1 + (int)(g.uni() * (double)(l - 2));
-    mu = (int)(g.uni() * 4.0);
-    eps = g.uni() < 0.5 ? -1 : 1;
+    for (int d = 0; d < 4; ++d) lc[d] = at[d];
+    mu = at[4];
+    eps = at[5];
     R = haar(g);
-    th_site = a.poisson ? -log(g.uni()) * a.theta_refresh_site : a.theta_refresh_site;
-    th_R = a.poisson ? -log(g.uni()) * a.theta_refresh_R : a.theta_refresh_R;
+    th_site = a.poisson ? exp_draw(g, a.theta_refresh_site) : a.theta_refresh_site;
+    th_R = a.poisson ? exp_draw(g, a.theta_refresh_R) : a.theta_refresh_R;
     tr_site = tr_R = 0.0;
     events = lifts = 0;
   } else {
@@ -466,7 +501,9 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
     events = rec.events;
     lifts = rec.lifts;
   }
-  const double theta_sample = a.poisson ? -log(g.uni()) * a.theta_sample : a.theta_sample;
+  const double set_x0 = sqrt(1 - a.epsilon_set * a.epsilon_set);
+  const int third = sub % 3;  // of the work that three lanes share
+  const double theta_sample = a.poisson ? exp_draw(g, a.theta_sample) : a.theta_sample;
   double tr_sample = 0.0;
 
 #pragma unroll 1
@@ -605,13 +642,29 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       }
       const Z ep = mk(cs, sn), em = mk(cs, -sn);
       double2* q = links + ((size_t)x * 4 + (size_t)mu) * 9;
+      if (GROUP >= 3) {
+        // a row for each of three lanes, which wait for one another before they write it and before
+        // it is read again
+        Z rr[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const Z r0 = cmul(R.e[i][0], ep), r1 = cmul(R.e[i][1], em), r2 = R.e[i][2];
+        for (int k = 0; k < 3; ++k) rr[k] = third == 0 ? R.e[0][k] : (third == 1 ? R.e[1][k] : R.e[2][k]);
+        const Z r0 = cmul(rr[0], ep), r1 = cmul(rr[1], em);
+        __syncwarp(gmask);
 #pragma unroll
         for (int j2 = 0; j2 < 3; ++j2) {
-          const Z v = cdot3(r0, T.e[0][j2], r1, T.e[1][j2], r2, t2[j2]);
-          q[3 * i + j2] = make_double2(v.re, v.im);
+          const Z v = cdot3(r0, T.e[0][j2], r1, T.e[1][j2], rr[2], t2[j2]);
+          q[3 * third + j2] = make_double2(v.re, v.im);
+        }
+        __syncwarp(gmask);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const Z r0 = cmul(R.e[i][0], ep), r1 = cmul(R.e[i][1], em), r2 = R.e[i][2];
+#pragma unroll
+          for (int j2 = 0; j2 < 3; ++j2) {
+            const Z v = cdot3(r0, T.e[0][j2], r1, T.e[1][j2], r2, t2[j2]);
+            q[3 * i + j2] = make_double2(v.re, v.im);
+          }
         }
       }
       ++events;
@@ -624,16 +677,18 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       tr_sample += d_site;
       tr_R += d_site;
       tr_site = 0.0;
-      if (a.poisson) th_site = -log(g.uni()) * a.theta_refresh_site;
+      if (a.poisson) th_site = exp_draw(g, a.theta_refresh_site);
+      int at[6];
+      random_site(g, l, at);
 #pragma unroll
-      for (int d = 0; d < 4; ++d) lc[d] = 1 + (int)(g.uni() * (double)(l - 2));
-      mu = (int)(g.uni() * 4.0);
-      eps = g.uni() < 0.5 ? -1 : 1;
+      for (int d = 0; d < 4; ++d) lc[d] = at[d];
+      mu = at[4];
+      eps = at[5];
     } else if (kind == 2) {
       tr_sample += d_R;
       tr_site += d_R;
       tr_R = 0.0;
-      if (a.poisson) th_R = -log(g.uni()) * a.theta_refresh_R;
+      if (a.poisson) th_R = exp_draw(g, a.theta_refresh_R);
       R = haar(g);
     } else {
       tr_sample += best;
@@ -654,12 +709,22 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       const bool f3 = blk.frozen(t4, nu);
       // selectVariable's uniform and the set index, in the reference's order, before the
       // plaquette: the proposal R_new = S R is known in advance and its dS rides along
-      const double r = g.uni();
-      const int iset = (int)(g.uni() * (double)ECMC_SET_SIZE);
+      double r, ui, ut = 0.0;  // ut: the acceptance's uniform, drawn only if it is needed
+      if (GROUP >= 3) {
+        const double u = chain_uniform(g.chain, g.k0, g.k1, g.n + (uint64_t)third);
+        r = __shfl_sync(gmask, u, lane0);
+        ui = __shfl_sync(gmask, u, lane0 + 1);
+        ut = __shfl_sync(gmask, u, lane0 + 2);
+        g.n += 2;
+      } else {
+        r = g.uni();
+        ui = g.uni();
+      }
+      const int iset = (int)(ui * (double)ECMC_SET_SIZE);
       // the picked element, formed once into the chain's slot (every lane of the chain writes
       // the same values and reads back its own writes)
       double2* sq = a.sx + (size_t)c * 9;
-      set_elem(sq, a.epsilon_set, a.k0, a.k1, c, a.call, set_gen, iset);
+      set_elem<GROUP>(sq, a.epsilon_set, set_x0, a.k0, a.k1, c, a.call, set_gen, iset, gmask, lane0, third);
       Herm Qn;
       {
         Z c0[3], c1[3];
@@ -676,7 +741,7 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       double tq[3], tn[3];
       const Herm Q = ds_matrix(R);
       if (GROUP >= 3) {
-        const int i3 = sub % 3, r0 = i3 == 0 ? 0 : (i3 == 1 ? (fwd ? 1 : 2) : 3);
+        const int r0 = third == 0 ? 0 : (third == 1 ? (fwd ? 1 : 2) : 3);
         const double2 v = lift_trace_lane(links, lift_factor(r0, x, s1, s2, s3, mu, nu, fwd),
                                           lift_factor(r0 + 1, x, s1, s2, s3, mu, nu, fwd),
                                           lift_factor(r0 + 2, x, s1, s2, s3, mu, nu, fwd),
@@ -705,14 +770,28 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       const double ds3 = f3 ? 0.0 : (fwd ? -tq[0] : tq[2]), dn3 = fwd ? -tn[0] : tn[2];
       const double a0 = fabs(ds0), a1 = fabs(ds1), a2 = fabs(ds2), a3 = fabs(ds3);
       const double sum = a0 + a1 + a2 + a3;
-      const double p0 = a0 / sum, p1 = a1 / sum, p2 = a2 / sum;
+      double p0, p1, p2;
+      if (GROUP >= 3) {
+        const double p = (third == 0 ? a0 : (third == 1 ? a1 : a2)) / sum;
+        p0 = __shfl_sync(gmask, p, lane0);
+        p1 = __shfl_sync(gmask, p, lane0 + 1);
+        p2 = __shfl_sync(gmask, p, lane0 + 2);
+      } else {
+        p0 = a0 / sum, p1 = a1 / sum, p2 = a2 / sum;
+      }
       // selectVariable (ecmc_mpi_cb.cpp:252-260)
       const int idx = r < p0 ? 0 : (r < p0 + p1 ? 1 : (r < p0 + p1 + p2 ? 2 : 3));
       const double ds_old = idx == 0 ? ds0 : idx == 1 ? ds1 : idx == 2 ? ds2 : ds3;
       const double ds_new = idx == 0 ? dn0 : idx == 1 ? dn1 : idx == 2 ? dn2 : dn3;
       int new_eps = -dsign(ds_old);
       bool take = fabs(ds_old) < fabs(ds_new);
-      if (!take) take = g.uni() < fabs(ds_new) / fabs(ds_old);
+      if (!take) {
+        if (GROUP >= 3)
+          ++g.n;
+        else
+          ut = g.uni();
+        take = ut < fabs(ds_new) / fabs(ds_old);
+      }
       if (take) {
         M Sx;
 #pragma unroll
@@ -791,9 +870,14 @@ __global__ void k_ecmc_counters(qcb_ecmc_chain* chains, uint32_t n, unsigned lon
 
 namespace {
 
+#ifndef ECMC_SPREAD
+#define ECMC_SPREAD 1
+#endif
 template <int GROUP, int MINB>
-cudaError_t launch_sample(const EcmcLaunch& a, cudaStream_t s) {
-  const uint32_t per_block = ECMC_WARPS * (32 / GROUP);
+cudaError_t launch_sample(EcmcLaunch a, cudaStream_t s) {
+  const uint32_t spread = (a.n_chains + 592 * ECMC_SPREAD - 1) / (592 * ECMC_SPREAD);
+  a.per_warp = spread < 32 / GROUP ? spread : 32 / GROUP;
+  const uint32_t per_block = ECMC_WARPS * a.per_warp;
   k_ecmc_sample<GROUP, MINB><<<(a.n_chains + per_block - 1) / per_block, ECMC_WARPS * 32, 0, s>>>(a);
   return cudaGetLastError();
 }
