@@ -21,7 +21,7 @@ struct qcb_ecmc {
   int lanes = 0;               // lanes per chain asked for (0: chosen by the library)
   double2* d_links = nullptr;  // FP64 array-of-structures copy of the lattice
   qcb_ecmc_chain* d_chains = nullptr;
-  double2* d_sx = nullptr;     // per chain: the set element of the current lift (9 double2)
+  double2* d_sx = nullptr;     // per chain: work slot of the current lift (ECMC_SLOT double2)
   uint32_t* d_status = nullptr;
   unsigned long long* d_count = nullptr;  // events, lifts, revs
   unsigned long long* h_count = nullptr;  // pinned: 3 counters + status word
@@ -88,7 +88,7 @@ int qcb_ecmc_create(qcb_lattice* L, const qcb_ecmc_params* p, uint64_t seed, qcb
   }
   if (cudaMalloc(&e->d_links, link_aos_bytes(L)) != cudaSuccess ||
       cudaMalloc(&e->d_chains, (size_t)e->n_chains * sizeof(qcb_ecmc_chain)) != cudaSuccess ||
-      cudaMalloc(&e->d_sx, (size_t)e->n_chains * 9 * sizeof(double2)) != cudaSuccess ||
+      cudaMalloc(&e->d_sx, (size_t)e->n_chains * ECMC_SLOT * sizeof(double2)) != cudaSuccess ||
       cudaMalloc(&e->d_status, sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&e->d_count, 3 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMallocHost(&e->h_count, 4 * sizeof(unsigned long long)) != cudaSuccess) {
@@ -139,7 +139,7 @@ int qcb_ecmc_lanes(const qcb_ecmc* e, int* lanes) {
   std::lock_guard<std::mutex> lk(c->mu);
   ECU(cudaSetDevice(c->device), "cudaSetDevice");
   const int layout = ecmc_layout(e->n_chains, e->lanes);
-  *lanes = layout == ECMC_LAYOUT_1 ? 1 : (layout == ECMC_LAYOUT_6 || layout == ECMC_LAYOUT_6C ? 6 : 3);
+  *lanes = layout;
   return QCB_OK;
 }
 

@@ -11,6 +11,8 @@ namespace qcb {
 // src/ecmc/ecmc_mpi_cb.cpp:560): the identity and 5000 pairs (M, M^dagger).
 constexpr int ECMC_SET_SIZE = 10001;
 
+constexpr int ECMC_SLOT = 15;
+
 // One sample call of every chain.
 struct EcmcLaunch {
   double2* links;        // FP64 array-of-structures copy: link (s, mu) = 9 double2 at (4 s + mu) * 9
@@ -26,16 +28,15 @@ struct EcmcLaunch {
   uint32_t k0, k1;       // Philox key (seed)
   uint32_t call;         // sample calls made so far (keys the chains' sets)
   double epsilon_set;    // size of the near-identity set's rotations
-  double2* sx;           // per chain: 9 double2 holding the set element of the current lift
+  double2* sx;           // per chain ECMC_SLOT double2: the current lift's set element S, columns 0, 1 of S R
   uint32_t* status;      // OR of the chains' status bits
 };
 // Launch shapes of the sample kernel: lanes per chain (1, 3 or 6, each lane computing an
-// equal share of the six staples; lanes 0-2 of a group also share the lift's three products)
-// and the register budget (C: capped for more resident chains).  All give the same results,
-// bit for bit.
-enum { ECMC_LAYOUT_1 = 1, ECMC_LAYOUT_3 = 3, ECMC_LAYOUT_3C = 4, ECMC_LAYOUT_6 = 6, ECMC_LAYOUT_6C = 7 };
+// equal share of the six staples; lanes 0-2 of a group also share the link's columns and a lift's
+// draws, set element and products).  All give the same results, bit for bit.
+enum { ECMC_LAYOUT_1 = 1, ECMC_LAYOUT_3 = 3, ECMC_LAYOUT_6 = 6 };
 // The layout for n_chains chains: `lanes` 1, 3 or 6 fixes the lanes per chain, 0 lets the
-// number of chains choose them too; the register budget follows the waves of resident chains.
+// number of chains choose them.
 int ecmc_layout(uint32_t n_chains, int lanes);
 cudaError_t launch_ecmc_sample(const EcmcLaunch& a, int layout, cudaStream_t s);
 // out[0..2] += the chains' events, lifts, same-site lifts; zeroes them with reset.

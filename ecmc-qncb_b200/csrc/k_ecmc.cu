@@ -34,9 +34,10 @@ namespace {
 constexpr uint32_t ECMC_CHAIN = 0xECEC0001u, ECMC_SETC = 0xECE50000u;
 constexpr uint64_t ECMC_MAX_EVENTS = 1ull << 26;
 constexpr double PI = 3.141592653589793;  // the double nearest pi
-// Sample kernel blocks: two warps.  Register caps: none (255 per thread), or ECMC_CAPPED
-// blocks of 64 threads per SM (168 per thread).
-constexpr int ECMC_WARPS = 2, ECMC_CAPPED = 6;
+// Sample kernel blocks: two warps at 255 registers a thread (four blocks per SM).  A cap of 168
+// registers keeps 1.5 times as many chains on the chip, and its spills cost more: 65536 chains ran
+// 3.99e8 events/s against 4.95e8, 10000 chains 3.14e8 against 4.45e8.
+constexpr int ECMC_WARPS = 2;
 
 typedef m3<double> M;
 typedef cx<double> Z;
@@ -112,8 +113,8 @@ __device__ M haar_from_normals(const double n[12]) {
 // inlined: it runs at initialisation and at R refreshes only).
 __device__ __noinline__ M haar(Stream& g) {
   double n[12];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
+#pragma unroll 1
+  for (int k = 0; k < 6; ++k) {  // one copy of the logarithm and the sine: the loop's code matters
     const double u1 = g.uni(), u2 = g.uni();
     const double rad = sqrt(-2.0 * log(u1));
     double sn, cs;
@@ -136,33 +137,12 @@ __device__ __noinline__ void random_site(Stream& g, int l, int out[6]) {
   out[5] = g.uni() < 0.5 ? -1 : 1;
 }
 
-// c mod L (out of line: the divisions of the seven site computations were a fifth of the loop's code)
-__device__ __noinline__ int reduce_far(int c, int L) { return ((c % L) + L) % L; }
-
 // The block of one chain: local coordinates lc (in [-1, l] for every link a chain at an
 // active link reads; -1 and l are the neighbouring blocks' faces, the reference's halo) sit
 // at stored site b_d l + lc_d - cum_d (mod L_d), with base_d = b_d l - cum_d in
 // (-L_d, L_d - l].
 struct Block {
   int L[4], base[4], l;
-  __device__ __forceinline__ uint32_t site(const int lc[4]) const {
-    int c[4];
-    bool far = false;
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-      c[d] = base[d] + lc[d];
-      if (c[d] < 0) c[d] += L[d];
-      else if (c[d] >= L[d]) c[d] -= L[d];
-      far = far || (unsigned)c[d] >= (unsigned)L[d];
-    }
-    // a chain only leaves [-1, l] after a lift onto a frozen link, which takes a rounding
-    // accident in the lift's tower sampling; the full reduction keeps any position in bounds
-    if (far) {
-#pragma unroll
-      for (int d = 0; d < 4; ++d) c[d] = reduce_far(c[d], L[d]);
-    }
-    return (uint32_t)c[0] + (uint32_t)L[0] * ((uint32_t)c[1] + (uint32_t)L[1] * ((uint32_t)c[2] + (uint32_t)L[2] * (uint32_t)c[3]));
-  }
   // GeometryCB::is_frozen in block-local terms: the halo (outside [0, l)) and the links
   // leaving local coordinate 0 in a direction d != mu.
   __device__ __forceinline__ bool frozen(const int lc[4], int mu) const {
@@ -170,6 +150,43 @@ struct Block {
 #pragma unroll
     for (int d = 0; d < 4; ++d) f = f || lc[d] < 0 || lc[d] >= l || (d != mu && lc[d] == 0);
     return f;
+  }
+};
+
+// c mod L (out of line: a division that a chain inside its block never needs)
+__device__ __noinline__ int reduce_far(int c, int L) { return ((c % L) + L) % L; }
+
+__device__ __forceinline__ int pick(const int v[4], int d) { return d == 0 ? v[0] : (d == 1 ? v[1] : (d == 2 ? v[2] : v[3])); }
+
+// Stored site of a link and the steps from it to its neighbours in each direction (periodic).
+struct Place {
+  uint32_t s;
+  int up[4], dn[4];
+  __device__ __forceinline__ Place(const Block& b, const int lc[4]) {
+    int c[4];
+    bool far = false;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      c[d] = b.base[d] + lc[d];
+      if (c[d] < 0) c[d] += b.L[d];
+      else if (c[d] >= b.L[d]) c[d] -= b.L[d];
+      far = far || (unsigned)c[d] >= (unsigned)b.L[d];
+    }
+    // a chain only leaves [-1, l] after a lift onto a frozen link, which takes a rounding
+    // accident in the lift's tower sampling; the full reduction keeps any position in bounds
+    if (far) {
+#pragma unroll
+      for (int d = 0; d < 4; ++d) c[d] = reduce_far(c[d], b.L[d]);
+    }
+    int str = 1;
+    s = 0;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      s += (uint32_t)(c[d] * str);
+      up[d] = c[d] + 1 == b.L[d] ? (1 - b.L[d]) * str : str;
+      dn[d] = c[d] == 0 ? (b.L[d] - 1) * str : -str;
+      str *= b.L[d];
+    }
   }
 };
 
@@ -438,11 +455,17 @@ __device__ __noinline__ void set_elem(double2* q, double eps, double x0, uint32_
 // sample_persistant (ecmc_mpi_cb.cpp:496-637) for chain c: events until it has travelled
 // theta_sample; the chain record persists across calls.  GROUP lanes of one warp (1, 3 or
 // 6) run a chain together: each computes its share of the six staples and, with three or
-// more, lanes 0-2 one product each of a lift; all of them carry the chain's state and take
-// the same branches, so the group never diverges.  Every lane stores the updated link (the
-// same values), so each lane's later loads see its own stores and no barrier is needed.
-template <int GROUP, int MINB>
-__global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunch a) {
+// more, a third of the work around them (a column of T and of the updated link, a product, an
+// embedding and a uniform of a lift); all of them carry the chain's state and take the same
+// branches, so the group never diverges.
+//
+// A chain is a serial walk of about 3000 warp instructions an event.  With few chains the latency of
+// dependent FP64 operations bounds it (16^4 as 256 chains: 8 us an event); with many, instruction
+// fetch does (the loop is 5500 instructions), then the links' latency.  Events/s (1e8), before and
+// after the lanes shared this work and the neighbour sites came from steps instead of seven
+// reductions: 256 chains 0.23 -> 0.34, 4096 1.80 -> 3.15, 20736 2.59 -> 4.64, 65536 3.42 -> 4.90.
+template <int GROUP>
+__global__ void __launch_bounds__(ECMC_WARPS * 32) k_ecmc_sample(EcmcLaunch a) {
   static_assert(GROUP == 1 || GROUP == 3 || GROUP == 6, "a chain's lanes split its six staples evenly");
   const int lane = threadIdx.x & 31, slot = lane / GROUP, sub = lane - slot * GROUP, lane0 = slot * GROUP;
   const uint32_t c = (blockIdx.x * ECMC_WARPS + (threadIdx.x >> 5)) * a.per_warp + slot;
@@ -516,19 +539,39 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       ++set_gen;
       set_counter = 0;
     }
-    const uint32_t x = blk.site(lc);
-    // rows 0 and 1 of T = R^dagger U: all the reject angles need
+    const Place at_x(blk, lc);
+    const uint32_t x = at_x.s;
+    const int upmu = pick(at_x.up, mu);
+    double2* const link = links + ((size_t)x * 4 + (size_t)mu) * 9;
+    // rows 0 and 1 of T = R^dagger U: all the reject angles need.  Three lanes take a column
+    // each (all three of its rows, for the update) and exchange rows 0 and 1.
     M T;
+    Z tc[3] = {mk(0.0, 0.0), mk(0.0, 0.0), mk(0.0, 0.0)};
+    if (GROUP >= 3) {
 #pragma unroll
-    for (int j2 = 0; j2 < 3; ++j2) T.e[0][j2] = T.e[1][j2] = mk(0.0, 0.0);
+      for (int m = 0; m < 3; ++m) {
+        const double2 v = link[3 * m + third];
+        const Z u = mk(v.x, v.y);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      Z ur[3];
-      ld_row(links, x, mu, c, ur);
+        for (int i = 0; i < 3; ++i) tc[i] = cfma(conj(R.e[m][i]), u, tc[i]);
+      }
 #pragma unroll
-      for (int j2 = 0; j2 < 3; ++j2) {
-        T.e[0][j2] = cfma(conj(R.e[c][0]), ur[j2], T.e[0][j2]);
-        T.e[1][j2] = cfma(conj(R.e[c][1]), ur[j2], T.e[1][j2]);
+      for (int j2 = 0; j2 < 3; ++j2)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          T.e[i][j2] = mk(__shfl_sync(gmask, tc[i].re, lane0 + j2), __shfl_sync(gmask, tc[i].im, lane0 + j2));
+    } else {
+#pragma unroll
+      for (int j2 = 0; j2 < 3; ++j2) T.e[0][j2] = T.e[1][j2] = mk(0.0, 0.0);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        Z ur[3];
+        ld_row(links, x, mu, m, ur);
+#pragma unroll
+        for (int j2 = 0; j2 < 3; ++j2) {
+          T.e[0][j2] = cfma(conj(R.e[m][0]), ur[j2], T.e[0][j2]);
+          T.e[1][j2] = cfma(conj(R.e[m][1]), ur[j2], T.e[1][j2]);
+        }
       }
     }
     // compute_list_staples (ecmc_mpi_cb.cpp:12-36): for each nu != mu, forward then backward;
@@ -547,14 +590,11 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       // T backward, and (E'R) = R forward or D R backward, both are
       // P_ii = sum_r (Tt W^+)_ir (E'R)_ri, and (Tt W^+)_ir = sum_m conj(W1_rm) (Tt W2^+)_im
       // for W = W1 W2: one code path for both orientations, streaming every link by rows.
-      int q4[4];
-      shifted(lc, fwd ? mu : nu, fwd ? 1 : -1, -1, 0, q4);
-      const uint32_t se = blk.site(q4);
-      shifted(lc, nu, fwd ? 1 : -1, fwd ? -1 : mu, fwd ? 0 : 1, q4);
-      const uint32_t s2 = blk.site(q4);
+      const int dnnu = pick(at_x.dn, nu);
+      const uint32_t se = x + (uint32_t)(fwd ? upmu : dnnu);
+      const uint32_t s2 = x + (uint32_t)(fwd ? pick(at_x.up, nu) : dnnu + upmu);
       const int d2 = fwd ? mu : nu;
-      shifted(lc, nu, fwd ? 0 : -1, -1, 0, q4);
-      const uint32_t s1 = blk.site(q4);
+      const uint32_t s1 = x + (uint32_t)(fwd ? 0 : dnnu);
       const int d1 = fwd ? nu : mu;
       // With one lane per chain every lane of a warp is at the same staple, so the orientation
       // is a branch; with more, the two orientations run as one instruction stream.
@@ -628,42 +668,37 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
     }
     const int kind = (step == d_sample) ? 0 : (step == d_site) ? 1 : (step == d_R) ? 2 : 3;
     // update (ecmc_mpi_cb.cpp:340-356): U <- R diag(e^{i xi}, e^{-i xi}, 1) R^dagger U, the
-    // rows of T = R^dagger U: 0 and 1 from above, 2 from U; written row by row
+    // rows of T = R^dagger U: 0 and 1 from above, 2 from U
     {
       double sn, cs;
       sincos((double)eps * step, &sn, &cs);
-      Z t2[3] = {mk(0.0, 0.0), mk(0.0, 0.0), mk(0.0, 0.0)};
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        Z ur[3];
-        ld_row(links, x, mu, c, ur);
-#pragma unroll
-        for (int j2 = 0; j2 < 3; ++j2) t2[j2] = cfma(conj(R.e[c][2]), ur[j2], t2[j2]);
-      }
       const Z ep = mk(cs, sn), em = mk(cs, -sn);
-      double2* q = links + ((size_t)x * 4 + (size_t)mu) * 9;
       if (GROUP >= 3) {
-        // a row for each of three lanes, which wait for one another before they write it and before
-        // it is read again
-        Z rr[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) rr[k] = third == 0 ? R.e[0][k] : (third == 1 ? R.e[1][k] : R.e[2][k]);
-        const Z r0 = cmul(rr[0], ep), r1 = cmul(rr[1], em);
+        // a column for each of three lanes, written when all have read the link and before any
+        // reads it again
         __syncwarp(gmask);
 #pragma unroll
-        for (int j2 = 0; j2 < 3; ++j2) {
-          const Z v = cdot3(r0, T.e[0][j2], r1, T.e[1][j2], rr[2], t2[j2]);
-          q[3 * third + j2] = make_double2(v.re, v.im);
+        for (int i = 0; i < 3; ++i) {
+          const Z v = cdot3(cmul(R.e[i][0], ep), tc[0], cmul(R.e[i][1], em), tc[1], R.e[i][2], tc[2]);
+          link[3 * i + third] = make_double2(v.re, v.im);
         }
         __syncwarp(gmask);
       } else {
+        Z t2[3] = {mk(0.0, 0.0), mk(0.0, 0.0), mk(0.0, 0.0)};
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          Z ur[3];
+          ld_row(links, x, mu, m, ur);
+#pragma unroll
+          for (int j2 = 0; j2 < 3; ++j2) t2[j2] = cfma(conj(R.e[m][2]), ur[j2], t2[j2]);
+        }
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           const Z r0 = cmul(R.e[i][0], ep), r1 = cmul(R.e[i][1], em), r2 = R.e[i][2];
 #pragma unroll
           for (int j2 = 0; j2 < 3; ++j2) {
             const Z v = cdot3(r0, T.e[0][j2], r1, T.e[1][j2], r2, t2[j2]);
-            q[3 * i + j2] = make_double2(v.re, v.im);
+            link[3 * i + j2] = make_double2(v.re, v.im);
           }
         }
       }
@@ -697,15 +732,15 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       // lift_improved_fast (ecmc_mpi_cb.cpp:277-337) on plaquette j
       const int nu = (j >> 1) + ((j >> 1) >= mu ? 1 : 0);
       const bool fwd = (j & 1) == 0;
+      const int dnnu = pick(at_x.dn, nu);
+      const uint32_t s1 = x + (uint32_t)(upmu + (fwd ? 0 : dnnu)), s2 = x + (uint32_t)(fwd ? pick(at_x.up, nu) : dnnu),
+                     s3 = x + (uint32_t)(fwd ? 0 : dnnu);
       int t4[4];
       lift_link(1, fwd, lc, mu, nu, t4);
-      const uint32_t s1 = blk.site(t4);
       const bool f1 = blk.frozen(t4, nu);
       lift_link(2, fwd, lc, mu, nu, t4);
-      const uint32_t s2 = blk.site(t4);
       const bool f2 = blk.frozen(t4, mu);
       lift_link(3, fwd, lc, mu, nu, t4);
-      const uint32_t s3 = blk.site(t4);
       const bool f3 = blk.frozen(t4, nu);
       // selectVariable's uniform and the set index, in the reference's order, before the
       // plaquette: the proposal R_new = S R is known in advance and its dS rides along
@@ -723,7 +758,7 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
       const int iset = (int)(ui * (double)ECMC_SET_SIZE);
       // the picked element, formed once into the chain's slot (every lane of the chain writes
       // the same values and reads back its own writes)
-      double2* sq = a.sx + (size_t)c * 9;
+      double2* sq = a.sx + (size_t)c * ECMC_SLOT;
       set_elem<GROUP>(sq, a.epsilon_set, set_x0, a.k0, a.k1, c, a.call, set_gen, iset, gmask, lane0, third);
       Herm Qn;
       {
@@ -736,6 +771,11 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
           c1[m] = cdot3(a0, R.e[0][1], a1, R.e[1][1], a2, R.e[2][1]);
         }
         Qn = ds_matrix_cols(c0, c1);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {  // columns 0 and 1 of S R, for R if the proposal is taken
+          sq[9 + 2 * m] = make_double2(c0[m].re, c0[m].im);
+          sq[10 + 2 * m] = make_double2(c1[m].re, c1[m].im);
+        }
       }
       // traces of rot0, rotX, rot3 against Q (tq) and Qn (tn)
       double tq[3], tn[3];
@@ -793,19 +833,17 @@ __global__ void __launch_bounds__(ECMC_WARPS * 32, MINB) k_ecmc_sample(EcmcLaunc
         take = ut < fabs(ds_new) / fabs(ds_old);
       }
       if (take) {
-        M Sx;
+        Z n0[3], n1[3], n2[3];
 #pragma unroll
-        for (int cc = 0; cc < 9; ++cc) {
-          const double2 v = sq[cc];
-          Sx.e[cc / 3][cc % 3] = mk(v.x, v.y);
+        for (int i = 0; i < 3; ++i) {
+          const double2 u0 = sq[9 + 2 * i], u1 = sq[10 + 2 * i];
+          n0[i] = mk(u0.x, u0.y);
+          n1[i] = mk(u1.x, u1.y);
+          const double2 v0 = sq[3 * i], v1 = sq[3 * i + 1], v2 = sq[3 * i + 2];
+          n2[i] = cdot3(mk(v0.x, v0.y), R.e[0][2], mk(v1.x, v1.y), R.e[1][2], mk(v2.x, v2.y), R.e[2][2]);
         }
-        M Rn;
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j2 = 0; j2 < 3; ++j2)
-            Rn.e[i][j2] = cdot3(Sx.e[i][0], R.e[0][j2], Sx.e[i][1], R.e[1][j2], Sx.e[i][2], R.e[2][j2]);
-        R = Rn;
+        for (int i = 0; i < 3; ++i) R.e[i][0] = n0[i], R.e[i][1] = n1[i], R.e[i][2] = n2[i];
         new_eps = -dsign(ds_new);
       }
       const int nmu = lift_link(idx, fwd, lc, mu, nu, t4);
@@ -870,26 +908,27 @@ __global__ void k_ecmc_counters(qcb_ecmc_chain* chains, uint32_t n, unsigned lon
 
 namespace {
 
-#ifndef ECMC_SPREAD
-#define ECMC_SPREAD 1
-#endif
-template <int GROUP, int MINB>
+// Chains per warp: as many as fit, but no more than it takes to give each of the 592 schedulers a
+// warp.  A warp's chains take each other's branches (a refresh of R among five chains stalls
+// all five), so few chains run best with a warp each: 256 chains 0.26e8 -> 0.32e8 events/s; two or
+// four warps a scheduler instead of one are no faster.
+constexpr uint32_t SCHEDULERS = 148 * 4;
+template <int GROUP>
 cudaError_t launch_sample(EcmcLaunch a, cudaStream_t s) {
-  const uint32_t spread = (a.n_chains + 592 * ECMC_SPREAD - 1) / (592 * ECMC_SPREAD);
+  const uint32_t spread = (a.n_chains + SCHEDULERS - 1) / SCHEDULERS;
   a.per_warp = spread < 32 / GROUP ? spread : 32 / GROUP;
   const uint32_t per_block = ECMC_WARPS * a.per_warp;
-  k_ecmc_sample<GROUP, MINB><<<(a.n_chains + per_block - 1) / per_block, ECMC_WARPS * 32, 0, s>>>(a);
+  k_ecmc_sample<GROUP><<<(a.n_chains + per_block - 1) / per_block, ECMC_WARPS * 32, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 // Chains resident on the device at once for the kernel of GROUP lanes per chain.
-template <int GROUP, int MINB>
+template <int GROUP>
 uint32_t resident_chains() {
   int dev = 0, sms = 0, blocks = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_ecmc_sample<GROUP, MINB>, ECMC_WARPS * 32, 0) !=
-          cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_ecmc_sample<GROUP>, ECMC_WARPS * 32, 0) != cudaSuccess)
     return 0;
   return (uint32_t)sms * (uint32_t)blocks * ECMC_WARPS * (32 / GROUP);
 }
@@ -899,56 +938,44 @@ uint32_t resident_chains() {
 // A call lasts about as long as its number of waves of resident chains, each chain taking a
 // similar number of events, so shape k is expected to run at rate_k n / (cap_k ceil(n / cap_k)),
 // rate_k being its event rate with the device full.  The rates are the ones measured on B200
-// (1e8 events/s, reference default budgets, 8192 to 65536 chains); the capacities come from
-// the occupancy calculator.  Among equal estimates the earlier shape wins.  The capacities are
+// (1e8 events/s, reference default budgets, 65536 chains); the capacities come from the occupancy
+// calculator (5920 chains on six lanes, 11840 on three).  So six lanes run up to 5920 chains (4096:
+// 3.14 against 2.54 on three lanes) and three above (10000: 4.45 against 3.76).  The capacities are
 // computed once per device, for the device current at the call (callers make the lattice's
 // device current first).
 int ecmc_layout(uint32_t n_chains, int lanes) {
-  struct Shape {
-    int layout, lanes;
-    uint32_t cap;
-    double rate;
-  };
   constexpr int MAX_DEVICES = 64;
+  constexpr double RATE6 = 4.3, RATE3 = 5.0;
   static std::mutex mu;
   static bool filled[MAX_DEVICES] = {};
-  static Shape table[MAX_DEVICES][4];
+  static uint32_t caps[MAX_DEVICES][2];
   if (lanes == 1) return ECMC_LAYOUT_1;
+  if (lanes == 3) return ECMC_LAYOUT_3;
+  if (lanes == 6) return ECMC_LAYOUT_6;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) dev = 0;
-  Shape shapes[4];
+  uint32_t cap6, cap3;
   {
     std::lock_guard<std::mutex> lk(mu);
     if (!filled[dev]) {
-      const Shape t[4] = {
-          {ECMC_LAYOUT_6, 6, resident_chains<6, 1>(), 2.9},
-          {ECMC_LAYOUT_6C, 6, resident_chains<6, ECMC_CAPPED>(), 3.3},
-          {ECMC_LAYOUT_3, 3, resident_chains<3, 1>(), 3.1},
-          {ECMC_LAYOUT_3C, 3, resident_chains<3, ECMC_CAPPED>(), 3.6},
-      };
-      for (int k = 0; k < 4; ++k) table[dev][k] = t[k];
+      caps[dev][0] = resident_chains<6>();
+      caps[dev][1] = resident_chains<3>();
       filled[dev] = true;
     }
-    for (int k = 0; k < 4; ++k) shapes[k] = table[dev][k];
+    cap6 = caps[dev][0];
+    cap3 = caps[dev][1];
   }
-  int best = lanes == 3 ? ECMC_LAYOUT_3C : ECMC_LAYOUT_6;
-  double best_rate = -1.0;
-  for (const Shape& sh : shapes) {
-    if ((lanes != 0 && sh.lanes != lanes) || sh.cap == 0) continue;
-    const double waves = (double)((n_chains + sh.cap - 1) / sh.cap);
-    const double r = sh.rate * (double)n_chains / ((double)sh.cap * (waves < 1.0 ? 1.0 : waves));
-    if (r > best_rate) best_rate = r, best = sh.layout;
-  }
-  return best;
+  auto expected = [&](double rate, uint32_t cap) {
+    return cap == 0 ? 0.0 : rate * (double)n_chains / ((double)cap * (double)((n_chains + cap - 1) / cap));
+  };
+  return expected(RATE3, cap3) > expected(RATE6, cap6) ? ECMC_LAYOUT_3 : ECMC_LAYOUT_6;
 }
 
 cudaError_t launch_ecmc_sample(const EcmcLaunch& a, int layout, cudaStream_t s) {
   switch (layout) {
-    case ECMC_LAYOUT_1: return launch_sample<1, 1>(a, s);
-    case ECMC_LAYOUT_3: return launch_sample<3, 1>(a, s);
-    case ECMC_LAYOUT_3C: return launch_sample<3, ECMC_CAPPED>(a, s);
-    case ECMC_LAYOUT_6: return launch_sample<6, 1>(a, s);
-    case ECMC_LAYOUT_6C: return launch_sample<6, ECMC_CAPPED>(a, s);
+    case ECMC_LAYOUT_1: return launch_sample<1>(a, s);
+    case ECMC_LAYOUT_3: return launch_sample<3>(a, s);
+    case ECMC_LAYOUT_6: return launch_sample<6>(a, s);
     default: return cudaErrorInvalidValue;
   }
 }
