@@ -35,20 +35,4 @@ __device__ __forceinline__ Links<S, NR> flow_links(const FlowLat& L, int swap) {
   return f;
 }
 
-// Programmatic stream serialization: the kernel's blocks become resident while the previous
-// kernel of the stream drains, and wait for it before they read (pdl_wait).
-template <typename... P, typename... A>
-cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, int block, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(block);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 }  // namespace qcb

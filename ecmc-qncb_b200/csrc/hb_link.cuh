@@ -41,6 +41,29 @@ struct KpMath<f1> {
   }
 };
 
+// lambda^2 of a Kennedy-Pendleton attempt from its words 1, 2, 3 (a0 = 1 - 2 lambda^2).
+template <typename R>
+__device__ __forceinline__ R kp_lambda2(R mhalf_over_alpha, const u32x4& r) {
+  const R r1 = u01<R>(r.v[1]), r2 = u01<R>(r.v[2]), r3 = u01<R>(r.v[3]);
+  const R cs = KpMath<R>::cos2pi(r2);
+  return mhalf_over_alpha * fma(cs * cs, KpMath<R>::log(r3), KpMath<R>::log(r1));
+}
+
+// (a0, a1, a2, a3): a direction uniform on S^2 from two words.
+template <typename R>
+__device__ __forceinline__ void kp_direction(R a0, uint32_t w0, uint32_t w1, R* x) {
+  R uphi = u01<R>(w0);
+  R cth = fma(R(2), u01<R>(w1), R(-1));
+  R sth = sqrt(fmax(R(0), fma(-cth, cth, R(1))));
+  R rs = sqrt(fmax(R(0), fma(-a0, a0, R(1))));
+  R sphi, cphi;
+  KpMath<R>::sincos2pi(uphi, &sphi, &cphi);
+  x[0] = a0;
+  x[1] = rs * sth * cphi;
+  x[2] = rs * sth * sphi;
+  x[3] = rs * cth;
+}
+
 // The SU(2) draw of one subgroup update: a0 from the Kennedy-Pendleton density
 // sqrt(1-a0^2) exp(alpha a0), then (a1, a2, a3) uniform on the sphere of radius
 // sqrt(1-a0^2).  Returns false when the KP attempts hit the cap.  FP64 calls one
@@ -50,7 +73,6 @@ template <typename R>
 __device__ __forceinline__ bool kp_draw_inline(R alpha, uint32_t link, uint32_t sweep, uint32_t hsg, uint32_t k0,
                                                uint32_t k1, R* x) {
   R mhalf_over_alpha = R(-0.5) / alpha;
-  // Kennedy-Pendleton draw of a0 with density sqrt(1-a0^2) exp(alpha a0).
   R a0 = 0;
   bool ok = false;
   for (uint32_t att = 0; att < KP_CAP; ++att) {
@@ -59,13 +81,9 @@ __device__ __forceinline__ bool kp_draw_inline(R alpha, uint32_t link, uint32_t 
     c.v[1] = sweep;
     c.v[2] = hsg;
     c.v[3] = att;
-    u32x4 r = philox4x32_10(c, k0, k1);
-    R delta = u01<R>(r.v[0]);
-    R r1 = u01<R>(r.v[1]);
-    R r2 = u01<R>(r.v[2]);
-    R r3 = u01<R>(r.v[3]);
-    R cs = KpMath<R>::cos2pi(r2);
-    R lam2 = mhalf_over_alpha * fma(cs * cs, KpMath<R>::log(r3), KpMath<R>::log(r1));
+    const u32x4 r = philox4x32_10(c, k0, k1);
+    const R delta = u01<R>(r.v[0]);
+    const R lam2 = kp_lambda2(mhalf_over_alpha, r);
     if (delta * delta <= R(1) - lam2) {
       a0 = fma(R(-2), lam2, R(1));
       ok = true;
@@ -79,17 +97,8 @@ __device__ __forceinline__ bool kp_draw_inline(R alpha, uint32_t link, uint32_t 
   c.v[1] = sweep;
   c.v[2] = hsg;
   c.v[3] = 0xFFFFFFFFu;
-  u32x4 r = philox4x32_10(c, k0, k1);
-  R uphi = u01<R>(r.v[0]);
-  R cth = fma(R(2), u01<R>(r.v[1]), R(-1));
-  R sth = sqrt(fmax(R(0), fma(-cth, cth, R(1))));
-  R rs = sqrt(fmax(R(0), fma(-a0, a0, R(1))));
-  R sphi, cphi;
-  KpMath<R>::sincos2pi(uphi, &sphi, &cphi);
-  x[0] = a0;
-  x[1] = rs * sth * cphi;
-  x[2] = rs * sth * sphi;
-  x[3] = rs * cth;
+  const u32x4 r = philox4x32_10(c, k0, k1);
+  kp_direction(a0, r.v[0], r.v[1], x);
   return true;
 }
 
@@ -99,10 +108,10 @@ __device__ __noinline__ bool kp_draw(R alpha, uint32_t link, uint32_t sweep, uin
   return kp_draw_inline<R>(alpha, link, sweep, hsg, k0, k1, x);
 }
 
-// One SU(2) subgroup update of U for subgroup (a, b), block entries of W = U A.
-template <typename R, int A_, int B_>
-__device__ __forceinline__ bool cm_subgroup(m3<R>& U, const m3<R>& A, R beta, uint32_t link, uint32_t sweep,
-                                            uint32_t hsg, uint32_t k0, uint32_t k1) {
+// One SU(2) subgroup update of U for subgroup (a, b), block entries of W = U A, the draw from
+// draw(alpha, x).
+template <typename R, int A_, int B_, typename D>
+__device__ __forceinline__ bool cm_subgroup_with(m3<R>& U, const m3<R>& A, R beta, const D& draw) {
   // W_ij = sum_k U_ik A_kj for the four block entries.
   cx<R> Waa = mk<R>(0, 0), Wab = mk<R>(0, 0), Wba = mk<R>(0, 0), Wbb = mk<R>(0, 0);
 #pragma unroll
@@ -121,16 +130,9 @@ __device__ __forceinline__ bool cm_subgroup(m3<R>& U, const m3<R>& A, R beta, ui
   R ik = R(1) / kk;
   R v0 = w0 * ik, v1 = w1 * ik, v2 = w2 * ik, v3 = w3 * ik;
   R alpha = beta * kk * R(2.0) / R(3.0);
-  R x0, x1, x2, x3;
-  if constexpr (std::is_same<R, double>::value) {
-    R xq[4];
-    if (!kp_draw<R>(alpha, link, sweep, hsg, k0, k1, xq)) return false;
-    x0 = xq[0], x1 = xq[1], x2 = xq[2], x3 = xq[3];
-  } else {
-    R xq[4];
-    if (!kp_draw_inline<R>(alpha, link, sweep, hsg, k0, k1, xq)) return false;
-    x0 = xq[0], x1 = xq[1], x2 = xq[2], x3 = xq[3];
-  }
+  R xq[4];
+  if (!draw(alpha, xq)) return false;
+  const R x0 = xq[0], x1 = xq[1], x2 = xq[2], x3 = xq[3];
   // r = x * adj(v), adj(v) = (v0, -v1, -v2, -v3).
   R q0 = fma(x0, v0, fma(x1, v1, fma(x2, v2, x3 * v3)));
   R q1 = fma(-x0, v1, fma(x1, v0, fma(-x2, v3, x3 * v2)));
@@ -145,6 +147,17 @@ __device__ __forceinline__ bool cm_subgroup(m3<R>& U, const m3<R>& A, R beta, ui
     U.e[B_][k] = cfma(Xbb, ub, Xba * ua);
   }
   return true;
+}
+
+template <typename R, int A_, int B_>
+__device__ __forceinline__ bool cm_subgroup(m3<R>& U, const m3<R>& A, R beta, uint32_t link, uint32_t sweep,
+                                            uint32_t hsg, uint32_t k0, uint32_t k1) {
+  return cm_subgroup_with<R, A_, B_>(U, A, beta, [&](R alpha, R* x) {
+    if constexpr (std::is_same<R, double>::value)
+      return kp_draw<R>(alpha, link, sweep, hsg, k0, k1, x);
+    else
+      return kp_draw_inline<R>(alpha, link, sweep, hsg, k0, k1, x);
+  });
 }
 
 // n_hits Cabibbo-Marinari hits on link (MU, par, i) of field f, at site x; returns the number

@@ -1,0 +1,149 @@
+// hb_quad.cuh — one FP64 Cabibbo-Marinari heatbath update of one link by four lanes of a warp.
+//
+// A pass over a small lattice has fewer links than the chip has lanes and takes as long as one
+// link: thousands of dependent FP64 instructions.  Here lanes 0, 1, 2 of a group form a row each
+// of the staple sum, and the Kennedy-Pendleton attempts of a draw go to the lanes side by side
+// (the first accepted one counts, as in the loop of kp_draw_inline; the draws are a function of
+// their counters).  Every element and every draw is computed by the operations of hb_link.cuh in
+// their order, so the links are the same bit for bit.  Pass on 8^4, 18-real: 14.2 -> 11.3 us, on 12^4
+// 17.9 -> 13.4 us.  In FP32, and with 12-real links (whose third rows take all lanes' rows), four
+// lanes were slower on 10^4 already, and on 8^4 in FP32 (5.7 against 8.5 us).
+#pragma once
+#include "hb_link.cuh"
+
+namespace qcb {
+
+// The group of four lanes a thread belongs to.
+struct Quad {
+  unsigned mask;
+  int lane;  // 0 .. 3
+  __device__ __forceinline__ Quad() : mask(0xFu << (threadIdx.x & 28)), lane((int)(threadIdx.x & 3)) {}
+  template <typename T>
+  __device__ __forceinline__ T get(T v, int from) const {
+    return __shfl_sync(mask, v, from, 4);
+  }
+  __device__ __forceinline__ cx<double> get(cx<double> v, int from) const { return mk(get(v.re, from), get(v.im, from)); }
+};
+
+// Row `lane` (lane 3: row 2 again) of the staple sum, by the terms of staple_terms.
+template <typename F>
+__device__ __forceinline__ row3<double> staple_row(const Quad& q, const Geom& g, const F& f, const Coord& x, int mu,
+                                                   int par, uint32_t i) {
+  typedef double R;
+  const int opp = par ^ 1, row = q.lane < 2 ? q.lane : 2;
+  const NbOff o = nb_offsets(g, x);
+  const int32_t upmu = sel4(o.up, mu);
+  const uint32_t ixmu = cb_index((uint32_t)((int32_t)x.s + upmu));
+  row3<R> A;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) A.e[j] = mk<R>(0, 0);
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    const int nu = k + (k >= mu);
+    const int32_t upnu = sel4(o.up, nu), dnnu = sel4(o.dn, nu);
+    const uint32_t ixnu = cb_index((uint32_t)((int32_t)x.s + upnu));
+    const uint32_t ixmunu = cb_index((uint32_t)((int32_t)x.s + upmu + dnnu));
+    const uint32_t ixmnu = cb_index((uint32_t)((int32_t)x.s + dnnu));
+    {
+      // forward: (U_nu(x+mu) U_mu(x+nu)^dagger) U_nu(x)^dagger
+      const row3<R> u0 = f.template load_row<R>(nu, opp, ixmu, row);
+      const m3<R> U1 = f.template load<R>(mu, opp, ixnu), U2 = f.template load<R>(nu, par, i);
+      row3<R> t;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        t.e[j] = mk<R>(0, 0);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) t.e[j] = cfma_nc(u0.e[m], U1.e[j][m], t.e[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) A.e[j] = cfma_nc(t.e[m], U2.e[j][m], A.e[j]);
+    }
+    {
+      // backward: (U_nu(x+mu-nu)^dagger U_mu(x-nu)^dagger) U_nu(x-nu)
+      const row3<R> v0 = f.template load_col<R>(nu, par, ixmunu, row);
+      const m3<R> V1 = f.template load<R>(mu, opp, ixmnu), V2 = f.template load<R>(nu, opp, ixmnu);
+      row3<R> t;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        t.e[j] = mk<R>(0, 0);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) t.e[j] = cfma_cc(v0.e[m], V1.e[j][m], t.e[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) A.e[j] = cfma(t.e[m], V2.e[m][j], A.e[j]);
+    }
+  }
+  return A;
+}
+
+// The SU(2) draw of kp_draw_inline with its attempts side by side: three and the direction's
+// draw in the first round, four in each later one.
+__device__ __forceinline__ bool kp_draw_quad(const Quad& q, double alpha, uint32_t link, uint32_t sweep, uint32_t hsg,
+                                             uint32_t k0, uint32_t k1, double* x) {
+  const double mhalf_over_alpha = -0.5 / alpha;
+  double a0 = 0;
+  bool ok = false;
+  uint32_t d0 = 0, d1 = 0;  // the direction's words
+  for (uint32_t att = 0; att < KP_CAP; att += att ? 4 : 3) {
+    const bool dir = att == 0 && q.lane == 3;
+    u32x4 c;
+    c.v[0] = link;
+    c.v[1] = sweep;
+    c.v[2] = hsg;
+    c.v[3] = dir ? 0xFFFFFFFFu : att + (uint32_t)q.lane;
+    const u32x4 r = philox4x32_10(c, k0, k1);
+    if (att == 0) {
+      d0 = q.get(r.v[0], 3);
+      d1 = q.get(r.v[1], 3);
+    }
+    const double delta = u01<double>(r.v[0]);
+    const double lam2 = kp_lambda2(mhalf_over_alpha, r);
+    const bool good = !dir && att + (uint32_t)q.lane < KP_CAP && delta * delta <= 1.0 - lam2;
+    const unsigned hits = (__ballot_sync(q.mask, good) >> (threadIdx.x & 28)) & 0xFu;
+    if (hits) {
+      a0 = fma(-2.0, q.get(lam2, __ffs(hits) - 1), 1.0);
+      ok = true;
+      break;
+    }
+  }
+  if (!ok) return false;
+  kp_direction(a0, d0, d1, x);
+  return true;
+}
+
+// hb_update_at by the four lanes of q (every lane holds the link; lane 0 stores it).
+template <typename F, bool MEAS>
+__device__ __forceinline__ uint32_t hb_update_quad(const Quad& q, const Geom& g, const F& f, const Coord& x, int mu,
+                                                   int par, uint32_t i, double beta, uint32_t k0, uint32_t k1,
+                                                   uint32_t sweep, int n_hits, double* retr) {
+  typedef double R;
+  m3<R> U = f.template load<R>(mu, par, i), A;
+  {
+    const row3<R> a = staple_row(q, g, f, x, mu, par, i);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) A.e[k][j] = q.get(a.e[j], k);
+  }
+  const uint32_t link = (uint32_t)mu * g.Vg + (x.s + g.soff);
+  uint32_t fails = 0;
+  for (int h = 0; h < n_hits; ++h) {
+    const uint32_t hb = RNG_DOMAIN_HB | ((uint32_t)h << 2);
+    auto draw = [&](uint32_t sub) {
+      return [&, sub](R alpha, R* y) { return kp_draw_quad(q, alpha, link, sweep, hb | sub, k0, k1, y); };
+    };
+    fails += !cm_subgroup_with<R, 0, 1>(U, A, beta, draw(0));
+    fails += !cm_subgroup_with<R, 1, 2>(U, A, beta, draw(1));
+    fails += !cm_subgroup_with<R, 0, 2>(U, A, beta, draw(2));
+  }
+  __syncwarp(q.mask);  // the link is read by all four lanes before it is written
+  if (q.lane == 0) f.template store<R>(mu, par, i, U);
+  if constexpr (MEAS) *retr = re_tr_nn(U, A);
+  return fails;
+}
+
+}  // namespace qcb

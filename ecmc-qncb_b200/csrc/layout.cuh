@@ -219,6 +219,28 @@ struct Links {
     return u;
   }
 
+  // Row r, column r of link (mu, par, i), 18-real storage.
+  template <typename R>
+  __device__ __forceinline__ row3<R> load_row(int mu, int par, uint32_t i, int r) const {
+    static_assert(NR == 18, "a stored row");
+    return load_line<R>(p + idx(mu, par, 3 * r, i), stride);
+  }
+  template <typename R>
+  __device__ __forceinline__ row3<R> load_col(int mu, int par, uint32_t i, int r) const {
+    static_assert(NR == 18, "a stored column");
+    return load_line<R>(p + idx(mu, par, r, i), 3 * (size_t)stride);
+  }
+  template <typename R>
+  __device__ __forceinline__ row3<R> load_line(const V* q, size_t step) const {
+    row3<R> u;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const V v = ldv<LM>(q + c * step);
+      u.e[c] = mk<R>(R(v.x), R(v.y));
+    }
+    return u;
+  }
+
   template <typename R>
   __device__ __forceinline__ void store(int mu, int par, uint32_t i, const m3<R>& u) const {
     V* q = p + idx(mu, par, 0, i);

@@ -28,6 +28,19 @@ __device__ __forceinline__ R site_plaquette(const Geom& g, const F& f, const Coo
   return sum * R(1.0 / 3.0);
 }
 
+// Re tr P_{mu nu}(x) of one plane.
+template <typename F, typename R>
+__device__ __forceinline__ R plaquette_plane(const Geom& g, const F& f, const Coord& x, int par, uint32_t i, int mu,
+                                             int nu) {
+  const int opp = par ^ 1;
+  const NbOff o = nb_offsets(g, x);
+  const uint32_t xmu = cb_index((uint32_t)((int32_t)x.s + sel4(o.up, mu)));
+  const uint32_t xnu = cb_index((uint32_t)((int32_t)x.s + sel4(o.up, nu)));
+  const m3<R> T1 = mul_nn(f.template load<R>(mu, par, i), f.template load<R>(nu, opp, xmu));
+  const m3<R> T2 = mul_nn(f.template load<R>(nu, par, i), f.template load<R>(mu, opp, xnu));
+  return re_tr_na(T1, T2);
+}
+
 // Sum of Re tr P_ij(x) over the spatial planes i < j < 3 (no 1/3), for the measuring
 // heatbath pass.
 template <typename F, typename R>

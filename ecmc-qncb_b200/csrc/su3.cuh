@@ -87,6 +87,12 @@ struct m3 {
   cx<R> e[3][3];
 };
 
+// Three components: a row or a column.
+template <typename R>
+struct row3 {
+  cx<R> e[3];
+};
+
 template <typename R>
 __device__ __forceinline__ void set_zero(m3<R>& a) {
 #pragma unroll

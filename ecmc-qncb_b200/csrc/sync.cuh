@@ -5,6 +5,7 @@
 // count; a block that gives up counts a timeout in status[1] and raises the abort flag
 // status[2], which makes every other waiting block give up too, so the launch always ends.
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace qcb {
@@ -21,6 +22,22 @@ constexpr uint64_t WAIT_MAX_ITERS = 1ull << 28;
 // kernel be scheduled once every block of this one has issued it.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Programmatic stream serialization: the kernel's blocks become resident while the previous
+// kernel of the stream drains, and wait for it before they read (pdl_wait).
+template <typename... P, typename... A>
+cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, int block, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
 
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
   uint32_t v;
