@@ -91,22 +91,34 @@ void drop_flow(qcb_batch* b) {
   b->have_plan = false;
 }
 
+// Groups of 32 links in a heatbath pass over the lattices, and those of the largest lattice.
+void pass_groups(const std::vector<qcb_lattice*>& lats, uint64_t* groups, uint64_t* largest) {
+  *groups = *largest = 0;
+  for (const qcb_lattice* L : lats) {
+    const uint64_t n = ceil_div(L->dev.g.Vh, 32u);
+    *groups += n;
+    *largest = std::max(*largest, n);
+  }
+}
+
 // Rebuild descriptors and prefix sums from the lattices and tiles; upload them.
 int upload_layout(qcb_batch* b) {
   const int n = b->n;
   b->h_prefix.assign(2 * (n + 1), 0);
   uint32_t* ph = &b->h_prefix[0];
   uint32_t* pr = &b->h_prefix[n + 1];
+  uint64_t groups = 0, largest = 0;
+  pass_groups(b->lats, &groups, &largest);
   for (int l = 0; l < n; ++l) {
     const qcb_lattice* L = b->lats[l];
-    const uint32_t nth = ceil_div(L->dev.g.Vh, b->hb_tile[l]);
+    const uint32_t tile = batch_tile(b->hb_tile[l], groups, largest, b->prec), nth = ceil_div(L->dev.g.Vh, tile);
     ph[l + 1] = ph[l] + nth;
     pr[l + 1] = pr[l] + ceil_div(L->dev.g.V, (uint32_t)batch_red_sites());
     BatchLat& d = b->h_desc[l];
     memset(&d, 0, sizeof d);
     d.g = L->dev.g;
     d.links = L->dev.links;
-    d.tile = b->hb_tile[l];
+    d.tile = tile;
     d.ntiles = nth;
   }
   b->per_hb = ph[n];
@@ -618,6 +630,8 @@ extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
       qcb_lattice* L = lats[j] = b->lats[kv.second[j]];
       BCU(cudaMemcpyAsync(L->fw[1], L->dev.links, L->bytes, cudaMemcpyDeviceToDevice, b->ctx->stream), "copy");
     }
+    uint64_t groups = 0, largest = 0;
+    pass_groups(lats, &groups, &largest);
     std::vector<BatchLat> dsc(m);
     std::vector<uint32_t> pre(m + 1, 0);
     BatchLat* d_dsc = nullptr;
@@ -642,8 +656,8 @@ extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
             d.links = lats[j]->fw[1];
             d.beta = 6.0;
             d.k0 = 12345u;
-            d.tile = (uint32_t)cand;
-            d.ntiles = ceil_div(d.g.Vh, (uint32_t)cand);
+            d.tile = batch_tile((uint32_t)cand, groups, largest, b->prec);
+            d.ntiles = ceil_div(d.g.Vh, d.tile);
             pre[j + 1] = pre[j] + d.ntiles;
           }
           r.lats = d_dsc;

@@ -14,7 +14,7 @@ struct BatchLat {
   double beta;      // coupling
   uint32_t k0, k1;  // Philox key (seed)
   uint32_t sweep0;  // sweep counter of the launch's first sweep
-  uint32_t tile;    // sites per work item (any multiple of the block size)
+  uint32_t tile;    // sites per work item (a multiple of 32)
   uint32_t ntiles;  // work items of this lattice per level (0: none)
   uint32_t nlev;    // levels this lattice takes part in (0 = all levels of the launch)
   int n_hits;       // hits (0 = the launch's value)
@@ -31,6 +31,10 @@ struct BatchRun {
   uint32_t* status;  // [0] KP cap hits, [1] wait timeouts, [2] abort flag
   int n_hits;
 };
+
+// Sites per work item of a launch whose lattices hold `groups` groups of 32 links a pass, the
+// largest of them `largest`: at most `most`.
+uint32_t batch_tile(uint32_t most, uint64_t groups, uint64_t largest, int prec);
 
 // Cooperative persistent launch: the grid is the co-resident maximum (capped by max_blocks
 // when > 0) for the given block size.

@@ -8,12 +8,7 @@
 
 namespace qcb {
 
-constexpr int FLOW_THREADS = 128;
-
-// Sites of one parity per block of the kernels that run one thread per site.
-__host__ __device__ __forceinline__ uint32_t site_tile(const FlowLat& r) {
-  return r.tile > (uint32_t)FLOW_THREADS ? r.tile : (uint32_t)FLOW_THREADS;
-}
+constexpr int FLOW_THREADS = 128;  // and sites of one parity per block where a thread has a site
 
 // The lattice l with prefix[l] <= b < prefix[l + 1], found by a whole warp: one load and one
 // ballot for each 32 lattices.

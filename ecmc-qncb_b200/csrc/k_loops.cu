@@ -85,8 +85,8 @@ std::vector<FlowLat> flow_rounds(const LatDev& L, const LoopDev& k) {
 static uint32_t tiles_of(const Geom& g, int slices, uint32_t tile) {
   return 2 * (((uint32_t)slices * (uint32_t)(g.str[3] / 2) + tile - 1) / tile);  // both parities
 }
-uint32_t loops_blocks(const FlowLat& r) { return tiles_of(r.g, r.kn, site_tile(r)); }
-uint32_t qe_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, site_tile(r)); }
+uint32_t loops_blocks(const FlowLat& r) { return tiles_of(r.g, r.kn, FLOW_THREADS); }
+uint32_t qe_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, FLOW_THREADS); }
 uint32_t update_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, r.tile); }
 
 // ---- the loops --------------------------------------------------------------------------
@@ -138,9 +138,8 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_LOOPS_MINB3
   if (MULTI && step >= L.nsteps) return;
   const uint32_t b = MULTI ? blockIdx.x - __ldg(&prefix[l]) : blockIdx.x;
   const Links<S, NR> f = flow_links<S, NR>(L, swap);
-  const uint32_t n = (uint32_t)L.kn * (uint32_t)(L.g.str[3] >> 1), tile = site_tile(L), first = (b >> 1) * tile;
-  for (uint32_t k = threadIdx.x; k < tile && first + k < n; k += FLOW_THREADS)
-    loops_site<S, NR, TRACE>(L, f, (int)(b & 1), first + k);
+  const uint32_t n = (uint32_t)L.kn * (uint32_t)(L.g.str[3] >> 1), k = (b >> 1) * FLOW_THREADS + threadIdx.x;
+  if (k < n) loops_site<S, NR, TRACE>(L, f, (int)(b & 1), k);
 }
 
 template <typename S, int NR>
@@ -207,11 +206,10 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_QE_MINB32 :
   const FlowLat& L = MULTI ? lats[l] : one;
   const uint32_t b = MULTI ? blockIdx.x - __ldg(&prefix[l]) : blockIdx.x;
   const Links<S, NR> f = flow_links<S, NR>(L, swap);
-  const uint32_t half = (uint32_t)(L.g.str[3] >> 1), n = (uint32_t)(L.t1 - L.t0) * half, tile = site_tile(L),
-                 at = (b >> 1) * tile;
+  const uint32_t half = (uint32_t)(L.g.str[3] >> 1), n = (uint32_t)(L.t1 - L.t0) * half,
+                 k = (b >> 1) * FLOW_THREADS + threadIdx.x;
   double q = 0.0, e = 0.0;
-  for (uint32_t k = threadIdx.x; k < tile && at + k < n; k += FLOW_THREADS)
-    qe_site<S, NR>(L, f, (int)(b & 1), (uint32_t)L.t0 * half + at + k, &q, &e);
+  if (k < n) qe_site<S, NR>(L, f, (int)(b & 1), (uint32_t)L.t0 * half + k, &q, &e);
   const double bq = block_sum<FLOW_THREADS>(q, sh);
   const double be = block_sum<FLOW_THREADS>(e, sh);
   if (threadIdx.x == 0) {

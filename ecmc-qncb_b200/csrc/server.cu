@@ -189,6 +189,15 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
   const int nh = (int)order.size();
   for (int k = 0; k < n; ++k)
     if (act[k]->spec.kind != QCB_JOB_SWEEPS) order.push_back(k);
+  uint64_t groups = 0, largest = 0;  // of the sweeps jobs, as the work items are sized by (batch_tile)
+  for (int p = 0; p < nh; ++p) {
+    const Job* j = act[order[p]];
+    if (j->spec.n_sweeps <= j->done_units) continue;
+    const uint64_t g = cdiv(j->spec.lat->dev.g.Vh, 32u);
+    groups += g;
+    largest = std::max(largest, g);
+  }
+  const uint32_t hb_tile = batch_tile(tile, groups, largest, s->cfg.precision);
   uint32_t lev_h = 0;
   int steps = 0;
   uint32_t* pre_h = s->h_prefix;  // nh + 1 entries
@@ -202,7 +211,7 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
     BatchLat& d = s->h_desc[p];
     memset(&d, 0, sizeof d);
     d.g = L->dev.g;
-    d.tile = tile;
+    d.tile = hb_tile;
     if (j->ready) {
       cudaError_t e = cudaStreamWaitEvent(s->stream, j->ready, 0);
       if (e != cudaSuccess) return e;
@@ -215,7 +224,7 @@ cudaError_t tick(qcb_server* s, std::vector<Job*>& act, std::vector<int>& finish
       d.k0 = (uint32_t)j->spec.seed;
       d.k1 = (uint32_t)(j->spec.seed >> 32);
       d.sweep0 = (uint32_t)(j->spec.sweep_offset + (uint64_t)j->done_units);
-      d.ntiles = cdiv(d.g.Vh, tile);
+      d.ntiles = cdiv(d.g.Vh, hb_tile);
       d.nlev = 8u * (uint32_t)q;
       d.n_hits = j->spec.n_hits;
     } else {

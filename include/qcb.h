@@ -201,8 +201,9 @@ int qcb_flow_steps(qcb_lattice* lat, double eps, int n);
 typedef struct qcb_batch qcb_batch;
 int qcb_batch_create(qcb_ctx* ctx, int n, qcb_lattice* const* lats, qcb_batch** out);
 int qcb_batch_destroy(qcb_batch* b);
-/* Sites per work item for the heatbath / flow of each lattice (multiples of 32 in
- * [32, 65536]); NULL keeps the current value (default 256). */
+/* Most sites per work item for the heatbath / flow of each lattice (multiples of 32 in
+ * [32, 65536]); NULL keeps the current value (default 256).  A launch whose warps would not all
+ * have work, or would end unevenly, takes fewer. */
 int qcb_batch_set_tiles(qcb_batch* b, const int* hb_tile, const int* flow_tile);
 int qcb_batch_get_tiles(qcb_batch* b, int* hb_tile, int* flow_tile);
 /* n_sweeps checkerboard sweeps of every lattice l at betas[l], seeds[l], sweeps
@@ -326,7 +327,7 @@ typedef struct qcb_server_config {
   int max_jobs;           /* concurrent jobs (0: 256) */
   int quantum_sweeps;     /* sweeps per sweeps-job per tick (0: 2) */
   int quantum_steps;      /* RK3 steps per flow-job per tick (0: 4) */
-  int tile;               /* sites per work item (0: 256) */
+  int tile;               /* most sites per work item (0: 256) */
 } qcb_server_config;
 typedef struct qcb_server_stats {
   uint64_t submitted, admitted, completed, ticks;
