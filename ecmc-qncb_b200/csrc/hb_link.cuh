@@ -41,27 +41,60 @@ struct KpMath<f1> {
   }
 };
 
-// lambda^2 of a Kennedy-Pendleton attempt from its words 1, 2, 3 (a0 = 1 - 2 lambda^2).
-template <typename R>
-__device__ __forceinline__ R kp_lambda2(R mhalf_over_alpha, const u32x4& r) {
-  const R r1 = u01<R>(r.v[1]), r2 = u01<R>(r.v[2]), r3 = u01<R>(r.v[3]);
-  const R cs = KpMath<R>::cos2pi(r2);
-  return mhalf_over_alpha * fma(cs * cs, KpMath<R>::log(r3), KpMath<R>::log(r1));
+__device__ __forceinline__ u32x4 kp_words(uint32_t link, uint32_t sweep, uint32_t hsg, uint32_t n, uint32_t k0,
+                                          uint32_t k1) {
+  u32x4 c;
+  c.v[0] = link;
+  c.v[1] = sweep;
+  c.v[2] = hsg;
+  c.v[3] = n;
+  return philox4x32_10(c, k0, k1);
 }
 
-// (a0, a1, a2, a3): a direction uniform on S^2 from two words.
+// What a Kennedy-Pendleton attempt takes from its words alone: delta^2 and
+// cos^2(2 pi r2) log r3 + log r1.
 template <typename R>
-__device__ __forceinline__ void kp_direction(R a0, uint32_t w0, uint32_t w1, R* x) {
-  R uphi = u01<R>(w0);
-  R cth = fma(R(2), u01<R>(w1), R(-1));
-  R sth = sqrt(fmax(R(0), fma(-cth, cth, R(1))));
-  R rs = sqrt(fmax(R(0), fma(-a0, a0, R(1))));
-  R sphi, cphi;
-  KpMath<R>::sincos2pi(uphi, &sphi, &cphi);
+__device__ __forceinline__ void kp_attempt(const u32x4& r, R* d2, R* lg) {
+  const R delta = u01<R>(r.v[0]), r1 = u01<R>(r.v[1]), r2 = u01<R>(r.v[2]), r3 = u01<R>(r.v[3]);
+  const R cs = KpMath<R>::cos2pi(r2);
+  *d2 = delta * delta;
+  *lg = fma(cs * cs, KpMath<R>::log(r3), KpMath<R>::log(r1));
+}
+
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ f1 mul_rn(f1 a, f1 b) { return a * b; }
+
+// lambda^2 of the attempt (a0 = 1 - 2 lambda^2), and whether it is accepted.
+template <typename R>
+__device__ __forceinline__ bool kp_accept(R mhalf_over_alpha, R d2, R lg, R* lam2) {
+  *lam2 = mul_rn(mhalf_over_alpha, lg);
+  return d2 <= R(1) - *lam2;
+}
+
+// A direction uniform on S^2 from two words.
+template <typename R>
+struct KpDirection {
+  R sth, cphi, sphi, cth;
+};
+template <typename R>
+__device__ __forceinline__ KpDirection<R> kp_direction(const u32x4& r) {
+  KpDirection<R> d;
+  const R uphi = u01<R>(r.v[0]);
+  d.cth = fma(R(2), u01<R>(r.v[1]), R(-1));
+  d.sth = sqrt(fmax(R(0), fma(-d.cth, d.cth, R(1))));
+  KpMath<R>::sincos2pi(uphi, &d.sphi, &d.cphi);
+  return d;
+}
+
+// (a0, a1, a2, a3) from lambda^2 and the direction.
+template <typename R>
+__device__ __forceinline__ void kp_quaternion(R lam2, const KpDirection<R>& d, R* x) {
+  const R a0 = fma(R(-2), lam2, R(1));
+  const R rs = sqrt(fmax(R(0), fma(-a0, a0, R(1))));
   x[0] = a0;
-  x[1] = rs * sth * cphi;
-  x[2] = rs * sth * sphi;
-  x[3] = rs * cth;
+  x[1] = rs * d.sth * d.cphi;
+  x[2] = rs * d.sth * d.sphi;
+  x[3] = rs * d.cth;
 }
 
 // The SU(2) draw of one subgroup update: a0 from the Kennedy-Pendleton density
@@ -70,46 +103,31 @@ __device__ __forceinline__ void kp_direction(R a0, uint32_t w0, uint32_t w1, R* 
 // out-of-line copy for the three subgroups (measured 4% faster per pass on 32^4, the
 // smaller code); FP32 inlines it (no difference measured).
 template <typename R>
-__device__ __forceinline__ bool kp_draw_inline(R alpha, uint32_t link, uint32_t sweep, uint32_t hsg, uint32_t k0,
+__device__ __forceinline__ bool kp_draw_inline(R mhalf_over_alpha, uint32_t link, uint32_t sweep, uint32_t hsg, uint32_t k0,
                                                uint32_t k1, R* x) {
-  R mhalf_over_alpha = R(-0.5) / alpha;
-  R a0 = 0;
+  R lam2 = 0;
   bool ok = false;
   for (uint32_t att = 0; att < KP_CAP; ++att) {
-    u32x4 c;
-    c.v[0] = link;
-    c.v[1] = sweep;
-    c.v[2] = hsg;
-    c.v[3] = att;
-    const u32x4 r = philox4x32_10(c, k0, k1);
-    const R delta = u01<R>(r.v[0]);
-    const R lam2 = kp_lambda2(mhalf_over_alpha, r);
-    if (delta * delta <= R(1) - lam2) {
-      a0 = fma(R(-2), lam2, R(1));
+    R d2, lg;
+    kp_attempt<R>(kp_words(link, sweep, hsg, att, k0, k1), &d2, &lg);
+    if (kp_accept(mhalf_over_alpha, d2, lg, &lam2)) {
       ok = true;
       break;
     }
   }
   if (!ok) return false;
-  // Uniform direction on S^2 for (a1, a2, a3).
-  u32x4 c;
-  c.v[0] = link;
-  c.v[1] = sweep;
-  c.v[2] = hsg;
-  c.v[3] = 0xFFFFFFFFu;
-  const u32x4 r = philox4x32_10(c, k0, k1);
-  kp_direction(a0, r.v[0], r.v[1], x);
+  kp_quaternion(lam2, kp_direction<R>(kp_words(link, sweep, hsg, 0xFFFFFFFFu, k0, k1)), x);
   return true;
 }
 
 template <typename R>
-__device__ __noinline__ bool kp_draw(R alpha, uint32_t link, uint32_t sweep, uint32_t hsg, uint32_t k0, uint32_t k1,
+__device__ __noinline__ bool kp_draw(R mhalf_over_alpha, uint32_t link, uint32_t sweep, uint32_t hsg, uint32_t k0, uint32_t k1,
                                      R* x) {
-  return kp_draw_inline<R>(alpha, link, sweep, hsg, k0, k1, x);
+  return kp_draw_inline<R>(mhalf_over_alpha, link, sweep, hsg, k0, k1, x);
 }
 
 // One SU(2) subgroup update of U for subgroup (a, b), block entries of W = U A, the draw from
-// draw(alpha, x).
+// draw(-1 / (2 alpha), x).
 template <typename R, int A_, int B_, typename D>
 __device__ __forceinline__ bool cm_subgroup_with(m3<R>& U, const m3<R>& A, R beta, const D& draw) {
   // W_ij = sum_k U_ik A_kj for the four block entries.
@@ -131,7 +149,7 @@ __device__ __forceinline__ bool cm_subgroup_with(m3<R>& U, const m3<R>& A, R bet
   R v0 = w0 * ik, v1 = w1 * ik, v2 = w2 * ik, v3 = w3 * ik;
   R alpha = beta * kk * R(2.0) / R(3.0);
   R xq[4];
-  if (!draw(alpha, xq)) return false;
+  if (!draw(R(-0.5) / alpha, xq)) return false;
   const R x0 = xq[0], x1 = xq[1], x2 = xq[2], x3 = xq[3];
   // r = x * adj(v), adj(v) = (v0, -v1, -v2, -v3).
   R q0 = fma(x0, v0, fma(x1, v1, fma(x2, v2, x3 * v3)));
@@ -152,11 +170,11 @@ __device__ __forceinline__ bool cm_subgroup_with(m3<R>& U, const m3<R>& A, R bet
 template <typename R, int A_, int B_>
 __device__ __forceinline__ bool cm_subgroup(m3<R>& U, const m3<R>& A, R beta, uint32_t link, uint32_t sweep,
                                             uint32_t hsg, uint32_t k0, uint32_t k1) {
-  return cm_subgroup_with<R, A_, B_>(U, A, beta, [&](R alpha, R* x) {
+  return cm_subgroup_with<R, A_, B_>(U, A, beta, [&](R mhalf_over_alpha, R* x) {
     if constexpr (std::is_same<R, double>::value)
-      return kp_draw<R>(alpha, link, sweep, hsg, k0, k1, x);
+      return kp_draw<R>(mhalf_over_alpha, link, sweep, hsg, k0, k1, x);
     else
-      return kp_draw_inline<R>(alpha, link, sweep, hsg, k0, k1, x);
+      return kp_draw_inline<R>(mhalf_over_alpha, link, sweep, hsg, k0, k1, x);
   });
 }
 

@@ -80,38 +80,45 @@ __device__ __forceinline__ row3<double> staple_row(const Quad& q, const Geom& g,
   return A;
 }
 
-// The SU(2) draw of kp_draw_inline with its attempts side by side: three and the direction's
-// draw in the first round, four in each later one.
-__device__ __forceinline__ bool kp_draw_quad(const Quad& q, double alpha, uint32_t link, uint32_t sweep, uint32_t hsg,
-                                             uint32_t k0, uint32_t k1, double* x) {
-  const double mhalf_over_alpha = -0.5 / alpha;
-  double a0 = 0;
-  bool ok = false;
-  uint32_t d0 = 0, d1 = 0;  // the direction's words
-  for (uint32_t att = 0; att < KP_CAP; att += att ? 4 : 3) {
-    const bool dir = att == 0 && q.lane == 3;
-    u32x4 c;
-    c.v[0] = link;
-    c.v[1] = sweep;
-    c.v[2] = hsg;
-    c.v[3] = dir ? 0xFFFFFFFFu : att + (uint32_t)q.lane;
-    const u32x4 r = philox4x32_10(c, k0, k1);
-    if (att == 0) {
-      d0 = q.get(r.v[0], 3);
-      d1 = q.get(r.v[1], 3);
-    }
-    const double delta = u01<double>(r.v[0]);
-    const double lam2 = kp_lambda2(mhalf_over_alpha, r);
-    const bool good = !dir && att + (uint32_t)q.lane < KP_CAP && delta * delta <= 1.0 - lam2;
+// What lane sg of a group holds of subgroup sg's draw: two attempts and the direction.
+struct QuadWords {
+  double d2[2], lg[2];
+  KpDirection<double> dir;
+};
+__device__ __forceinline__ QuadWords kp_words_quad(const Quad& q, uint32_t link, uint32_t sweep, uint32_t hb,
+                                                   uint32_t k0, uint32_t k1) {
+  const uint32_t hsg = hb | (uint32_t)(q.lane < 2 ? q.lane : 2);
+  QuadWords d;
+#pragma unroll
+  for (uint32_t att = 0; att < 2; ++att)
+    kp_attempt<double>(kp_words(link, sweep, hsg, att, k0, k1), &d.d2[att], &d.lg[att]);
+  d.dir = kp_direction<double>(kp_words(link, sweep, hsg, 0xFFFFFFFFu, k0, k1));
+  return d;
+}
+
+// kp_draw from the words of lane sg; attempts from 2 on four at a time.
+__device__ __forceinline__ bool kp_draw_quad(const Quad& q, const QuadWords& d, double mhalf_over_alpha,
+                                             uint32_t link, uint32_t sweep, uint32_t hb, int sg, uint32_t k0,
+                                             uint32_t k1, double* x) {
+  double lam2, lam2b;
+  const bool first = kp_accept(mhalf_over_alpha, d.d2[0], d.lg[0], &lam2);
+  const bool second = kp_accept(mhalf_over_alpha, d.d2[1], d.lg[1], &lam2b);
+  if (!first) lam2 = lam2b;
+  bool ok = q.get((int)(first || second), sg) != 0;
+  for (uint32_t att = 2; !ok && att < KP_CAP; att += 4) {
+    double d2, lg, l2;
+    kp_attempt<double>(kp_words(link, sweep, hb | (uint32_t)sg, att + (uint32_t)q.lane, k0, k1), &d2, &lg);
+    const bool good = kp_accept(mhalf_over_alpha, d2, lg, &l2) && att + (uint32_t)q.lane < KP_CAP;
     const unsigned hits = (__ballot_sync(q.mask, good) >> (threadIdx.x & 28)) & 0xFu;
     if (hits) {
-      a0 = fma(-2.0, q.get(lam2, __ffs(hits) - 1), 1.0);
+      lam2 = q.get(l2, __ffs(hits) - 1);
       ok = true;
-      break;
     }
   }
   if (!ok) return false;
-  kp_direction(a0, d0, d1, x);
+  kp_quaternion(lam2, d.dir, x);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) x[k] = q.get(x[k], sg);
   return true;
 }
 
@@ -121,6 +128,8 @@ __device__ __forceinline__ uint32_t hb_update_quad(const Quad& q, const Geom& g,
                                                    int par, uint32_t i, double beta, uint32_t k0, uint32_t k1,
                                                    uint32_t sweep, int n_hits, double* retr) {
   typedef double R;
+  const uint32_t link = (uint32_t)mu * g.Vg + (x.s + g.soff);
+  QuadWords d = kp_words_quad(q, link, sweep, RNG_DOMAIN_HB, k0, k1);
   m3<R> U = f.template load<R>(mu, par, i), A;
   {
     const row3<R> a = staple_row(q, g, f, x, mu, par, i);
@@ -129,12 +138,14 @@ __device__ __forceinline__ uint32_t hb_update_quad(const Quad& q, const Geom& g,
 #pragma unroll
       for (int j = 0; j < 3; ++j) A.e[k][j] = q.get(a.e[j], k);
   }
-  const uint32_t link = (uint32_t)mu * g.Vg + (x.s + g.soff);
   uint32_t fails = 0;
   for (int h = 0; h < n_hits; ++h) {
     const uint32_t hb = RNG_DOMAIN_HB | ((uint32_t)h << 2);
-    auto draw = [&](uint32_t sub) {
-      return [&, sub](R alpha, R* y) { return kp_draw_quad(q, alpha, link, sweep, hb | sub, k0, k1, y); };
+    if (h) d = kp_words_quad(q, link, sweep, hb, k0, k1);
+    auto draw = [&](int sg) {
+      return [&, sg](R mhalf_over_alpha, R* y) {
+        return kp_draw_quad(q, d, mhalf_over_alpha, link, sweep, hb, sg, k0, k1, y);
+      };
     };
     fails += !cm_subgroup_with<R, 0, 1>(U, A, beta, draw(0));
     fails += !cm_subgroup_with<R, 1, 2>(U, A, beta, draw(1));

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128) k_hb_quad(Geom g, Links<double, 18> f, in
 }
 
 // Four lanes per link while all of a pass's links are then resident at once (148 SMs of three
-// blocks of 32 links): 12^4 (10368 links) takes 13.4 us against 17.9, 14^4 (19208) 22.2 against 18.6.
+// blocks of 32 links): 12^4 (10368 links) takes 12.1 us against 17.8, 14^4 (19208) 19.5 against 18.6.
 static bool quad_pass(const LatDev& L) {
   return L.prec == QCB_PREC_FP64 && L.nr == 18 && L.g.Vh <= 148u * 3u * 32u;
 }
