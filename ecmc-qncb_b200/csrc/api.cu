@@ -52,6 +52,11 @@ int set_device(qcb_ctx* c) {
 int qcb::check_status(qcb_ctx* c) {
   CU(cudaMemcpyAsync(c->h_status, c->d_status, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
      "status copy");
+  return wait_status(c);
+}
+
+// The same with the words already on their way to h_status (StatusCopy).
+int qcb::wait_status(qcb_ctx* c) {
   CU(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
   uint32_t kp = c->h_status[0];
   const uint32_t timeouts = c->h_status[1], aborted = c->h_status[2];
@@ -189,23 +194,23 @@ int rk3(qcb_lattice* L, const std::vector<FlowLat>& rounds, int step, double* qe
   if (r_ == QCB_OK) r_ = loop_pass(L, rounds, odd, 3, nullptr);
   if (r_ != QCB_OK) return r_;
   if (qe_dev) {
-    CU(launch_qe_from_parts(parts, (int)n, parts + 2 * (size_t)n, qe_dev, 1.0 / (double)L->dev.g.Vg, c->stream),
+    CU(launch_qe_from_parts(parts, (int)n, parts + 2 * (size_t)n, qe_dev, 1.0 / (double)L->dev.g.Vg, StatusCopy(),
+                            c->stream, &c->launches),
        "Q/E sums");
-    c->launches += 3;
   }
   return QCB_OK;
 }
 
 // Clover (Q, E) of the rounds' links (swap as loop_pass), without a step.
-int qe_async(qcb_lattice* L, const std::vector<FlowLat>& rounds, int swap, double* dst_dev) {
+int qe_async(qcb_lattice* L, const std::vector<FlowLat>& rounds, int swap, double* dst, const StatusCopy& st) {
   qcb_ctx* c = L->ctx;
   const uint32_t n = qe_parts(rounds);
   int r_ = ensure_meas(L, 2 * (size_t)n + 512);
   if (r_ == QCB_OK) r_ = loop_pass(L, rounds, swap, 0, L->meas);
   if (r_ != QCB_OK) return r_;
-  CU(launch_qe_from_parts(L->meas, (int)n, L->meas + 2 * (size_t)n, dst_dev, 1.0 / (double)L->dev.g.Vg, c->stream),
+  CU(launch_qe_from_parts(L->meas, (int)n, L->meas + 2 * (size_t)n, dst, 1.0 / (double)L->dev.g.Vg, st, c->stream,
+                          &c->launches),
      "Q/E sums");
-  c->launches += 3;
   return QCB_OK;
 }
 }  // namespace
@@ -769,7 +774,7 @@ int qcb_heatbath_plaquette(qcb_lattice* L, double beta, int n_sweeps, int n_hits
   LOCK(c);
   TRY(set_device(c));
   if (n_sweeps == 0) {
-    CU(launch_plaquette(L->dev, c->d_scratch, c->d_out, c->stream, c->block), "plaquette");
+    CU(launch_plaquette(L->dev, c->d_scratch, c->h_out, {c->d_status, c->h_status}, c->stream), "plaquette");
     c->launches += 2;
   } else {
     const int nb = hb_meas_blocks(L->dev);
@@ -790,11 +795,11 @@ int qcb_heatbath_plaquette(qcb_lattice* L, double beta, int n_sweeps, int n_hits
           c->launches++;
         }
     }
-    CU(launch_sum_parts(L->meas, 2 * nb, L->meas + 2 * nb, c->d_out, c->stream), "plaquette sum");
-    c->launches += 2;
+    CU(launch_sum_parts(L->meas, 2 * nb, L->meas + 2 * nb, c->h_out, {c->d_status, c->h_status}, c->stream,
+                        &c->launches),
+       "plaquette sum");
   }
-  CU(cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
-  TRY(check_status(c));
+  TRY(wait_status(c));
   // the measuring passes sum Re tr P; the plaquette kernel sums Re tr P / 3
   const double scale = n_sweeps == 0 ? 1.0 : 1.0 / 3.0;
   *plaq = c->h_out[0] * scale / (6.0 * (double)L->dev.g.Vg);
@@ -853,10 +858,9 @@ int qcb_plaquette(qcb_lattice* L, double* out) {
   qcb_ctx* c = L->ctx;
   LOCK(c);
   TRY(set_device(c));
-  CU(launch_plaquette(L->dev, c->d_scratch, c->d_out, c->stream, c->block), "plaquette");
+  CU(launch_plaquette(L->dev, c->d_scratch, c->h_out, {c->d_status, c->h_status}, c->stream), "plaquette");
   c->launches += 2;
-  CU(cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
-  TRY(check_status(c));
+  TRY(wait_status(c));
   *out = c->h_out[0] / (6.0 * (double)L->dev.g.Vg);
   return QCB_OK;
 }
@@ -869,9 +873,8 @@ int qcb_topo_qe(qcb_lattice* L, double* q, double* e) {
   TRY(set_device(c));
   std::vector<FlowLat> rounds;
   TRY(loop_rounds(L, L->dev, nullptr, 0.0, &rounds));
-  TRY(qe_async(L, rounds, 0, c->d_out));
-  CU(cudaMemcpyAsync(c->h_out, c->d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H");
-  TRY(check_status(c));
+  TRY(qe_async(L, rounds, 0, c->h_out, {c->d_status, c->h_status}));
+  TRY(wait_status(c));
   *q = c->h_out[0];
   *e = c->h_out[1];
   return QCB_OK;
@@ -900,7 +903,7 @@ int qcb_flow_measure(qcb_lattice* L, double eps, int n_steps_gf, int n_rk_steps,
     for (int k = 0; k < n; ++k) {
       ts[k] = t;
       // the record is summed from the loops of the group's first RK3 step; with no step, alone
-      if (n_rk_steps == 0) TRY(qe_async(L, rounds, step & 1, c->d_out + 2 * k));
+      if (n_rk_steps == 0) TRY(qe_async(L, rounds, step & 1, c->d_out + 2 * k, StatusCopy()));
       for (int r = 0; r < n_rk_steps; ++r, ++step) {
         TRY(rk3(L, rounds, step, r == 0 ? c->d_out + 2 * k : nullptr));
         t += eps;

@@ -55,4 +55,5 @@ void ctx_unref(qcb_ctx* c);
 int ensure_flow_space(qcb_lattice* L);
 // Reads and clears the context's device status words (after synchronising its stream).
 int check_status(qcb_ctx* c);
+int wait_status(qcb_ctx* c);
 }  // namespace qcb

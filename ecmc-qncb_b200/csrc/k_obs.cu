@@ -4,11 +4,12 @@
 // sum of Re tr(U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag)/3 over x and mu < nu, / (6V).
 // Here: one thread per site (the two parities of a checkerboard index adjacent; a slab
 // skips its halo slices), per-site value in the lattice's arithmetic type, converted to FP64; FP64 tree reduction inside each block; the block partials are
-// summed in a fixed order with Neumaier compensation by a single-block kernel.  The grid
+// summed in a fixed order with Neumaier compensation by k_total.  The grid
 // is a fixed multiple of the SM count (grid-stride loop), so the scratch is bounded.
 #include "dispatch.cuh"
 #include "obs_site.cuh"
 #include "reduce.cuh"
+#include "sync.cuh"
 
 namespace qcb {
 
@@ -24,26 +25,46 @@ struct RedMinBlocks {
 
 int reduce_blocks() { return RED_BLOCKS; }
 
-// Neumaier-compensated sums of nq quantities of n partials each (parts[q*n + k]), one warp
-// per quantity: lane j sums k = j, j+32, ...; lane 0 then adds the 32 lane sums in lane
-// order.  The order is fixed, so the result is deterministic.  out[q] = sum.
-__global__ void k_finalize(const double* __restrict__ parts, int n, int nq, double* __restrict__ out) {
-  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (q >= nq) return;
+// Totals of quantities of n partials each (block q: parts[q n .. q n + n)), Neumaier-compensated and
+// in a fixed order: thread j sums k = j, j + 1024, ..., then a tree of the compensated sums.  out[q] =
+// total * (q ? scale1 : scale0).  With host_status, block 0 also copies the four status words
+// there; out and host_status may be pinned host memory, and the caller then needs no copy and no
+// other launch before it synchronises.  One warp on 1184 partials, a scaling kernel and two
+// copies took 13 us behind a plaquette of 8^4 (this: 4), 16 behind a sweep.
+constexpr int TOTAL_THREADS = 1024;
+__global__ void __launch_bounds__(TOTAL_THREADS) k_total(const double* __restrict__ parts, int n, double scale0,
+                                                         double scale1, double* __restrict__ out,
+                                                         const uint32_t* __restrict__ status,
+                                                         uint32_t* __restrict__ host_status) {
+  __shared__ double ls[TOTAL_THREADS / 32], lc[TOTAL_THREADS / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const double* p = parts + (size_t)blockIdx.x * n;
   double s = 0.0, c = 0.0;
-  for (int k = lane; k < n; k += 32) neumaier_add(s, c, parts[q * n + k]);
-  __shared__ double ls[4][32], lc[4][32];
-  ls[q][lane] = s;
-  lc[q][lane] = c;
-  __syncwarp();
-  if (lane == 0) {
-    double S = 0.0, Cc = 0.0;
-    for (int j = 0; j < 32; ++j) {
-      neumaier_add(S, Cc, ls[q][j]);
-      Cc += lc[q][j];
+  for (int k = threadIdx.x; k < n; k += TOTAL_THREADS) neumaier_add(s, c, p[k]);
+  auto tree = [&]() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double s2 = __shfl_down_sync(0xffffffffu, s, o), c2 = __shfl_down_sync(0xffffffffu, c, o);
+      neumaier_add(s, c, s2);
+      c += c2;
     }
-    out[q] = S + Cc;
+  };
+  tree();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) ls[w] = s, lc[w] = c;
+  __syncthreads();
+  if (w == 0) {
+    s = ls[lane], c = lc[lane];
+    tree();
+    if (lane == 0) out[blockIdx.x] = (s + c) * (blockIdx.x ? scale1 : scale0);
+    if (host_status && blockIdx.x == 0 && lane < 4) host_status[lane] = status[lane];
   }
+}
+
+static cudaError_t total(const double* parts, int n, int nq, double scale0, double scale1, double* out,
+                         const StatusCopy& st, cudaStream_t s) {
+  return pdl_launch(k_total, dim3(nq), TOTAL_THREADS, s, parts, n, scale0, scale1, out, st.device, st.host);
 }
 
 // Reduction grid: one block per RED_THREADS sites, at most RED_BLOCKS.
@@ -70,35 +91,24 @@ __global__ void __launch_bounds__(RED_THREADS, RedMinBlocks<S>::value) k_plaquet
 }
 
 template <typename S, int NR>
-static cudaError_t plaquette_impl(const LatDev& L, double* scratch, double* out, cudaStream_t s, int) {
+static cudaError_t plaquette_impl(const LatDev& L, int nb, double* scratch, double* out, const StatusCopy& st,
+                                  cudaStream_t s) {
   Links<S, NR> f;
   f.p = reinterpret_cast<typename Links<S, NR>::V*>(L.links);
   f.stride = L.g.stride;
-  const int nb = red_grid(L.g);
   k_plaquette<S, NR><<<nb, RED_THREADS, 0, s>>>(L.g, f, scratch);
-  k_finalize<<<1, 32, 0, s>>>(scratch, nb, 1, out);
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : total(scratch, nb, 1, 1.0, 1.0, out, st, s);
 }
 
-cudaError_t launch_plaquette(const LatDev& L, double* scratch, double* out, cudaStream_t s, int block) {
-  QCB_DISPATCH_STORE(L, plaquette_impl, L, scratch, out, s, block);
+cudaError_t launch_plaquette(const LatDev& L, double* scratch, double* out, const StatusCopy& st, cudaStream_t s) {
+  QCB_DISPATCH_STORE(L, plaquette_impl, L, red_grid(L.g), scratch, out, st, s);
 }
 
 // Same reduction with a caller-chosen number of blocks (partials written to scratch[0..nblocks)).
-template <typename S, int NR>
-static cudaError_t plaquette_partials_impl(const LatDev& L, int nblocks, double* scratch, double* out,
-                                           cudaStream_t s) {
-  Links<S, NR> f;
-  f.p = reinterpret_cast<typename Links<S, NR>::V*>(L.links);
-  f.stride = L.g.stride;
-  k_plaquette<S, NR><<<nblocks, RED_THREADS, 0, s>>>(L.g, f, scratch);
-  k_finalize<<<1, 32, 0, s>>>(scratch, nblocks, 1, out);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_plaquette_partials(const LatDev& L, int nblocks, double* scratch, double* out, cudaStream_t s) {
   if (nblocks < 1) return cudaErrorInvalidValue;
-  QCB_DISPATCH_STORE(L, plaquette_partials_impl, L, nblocks, scratch, out, s);
+  QCB_DISPATCH_STORE(L, plaquette_impl, L, nblocks, scratch, out, StatusCopy(), s);
 }
 
 int reduce_threads() { return RED_THREADS; }
@@ -117,34 +127,30 @@ __global__ void __launch_bounds__(RED_THREADS) k_sum_chunks(const double* __rest
   if (threadIdx.x == 0) out[blockIdx.y * gridDim.x + blockIdx.x] = b;
 }
 
-// out[q] = sum of parts[q * n .. q * n + n) for q < nq (nq <= 4), in a fixed order whatever the
-// device: chunks of at most 256 x 128 partials per block, then the single-warp Neumaier
-// finalize.  tmp holds 256 * nq doubles.
-static cudaError_t sum_parts(const double* parts, int n, int nq, double* tmp, double* out, cudaStream_t s) {
-  if (n < 1 || nq < 1 || nq > 4) return cudaErrorInvalidValue;
-  const int nb = min(256, (n + RED_THREADS - 1) / RED_THREADS);
-  const int chunk = (n + nb - 1) / nb;
+// The totals of nq <= 2 quantities, in a fixed order whatever the device: at most SUM_ONE partials by
+// k_total alone, more in chunks first (64^4's 131072: 60 us in one block, 6 in two launches).
+constexpr int SUM_ONE = 16384;
+static cudaError_t sum_parts(const double* parts, int n, int nq, double scale0, double scale1, double* tmp, double* out,
+                             const StatusCopy& st, cudaStream_t s, uint64_t* launches) {
+  if (n < 1 || nq < 1 || nq > 2) return cudaErrorInvalidValue;
+  ++*launches;
+  if (n <= SUM_ONE) return total(parts, n, nq, scale0, scale1, out, st, s);
+  ++*launches;
+  const int nb = 256, chunk = (n + nb - 1) / nb;
   k_sum_chunks<<<dim3(nb, nq), RED_THREADS, 0, s>>>(parts, n, chunk, tmp);
-  k_finalize<<<1, 32 * nq, 0, s>>>(tmp, nb, nq, out);
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : total(tmp, nb, nq, scale0, scale1, out, st, s);
 }
 
-cudaError_t launch_sum_parts(const double* parts, int n, double* tmp, double* out, cudaStream_t s) {
-  return sum_parts(parts, n, 1, tmp, out, s);
-}
-
-// out2[0] = Q = sum q / (4 pi^2); out2[1] = E = sum e / 2 / V.
-__global__ void k_qe_scale(double* out2, double inv_vol) {
-  out2[0] = out2[0] * (1.0 / (4.0 * 3.14159265358979323846 * 3.14159265358979323846));
-  out2[1] = 0.5 * out2[1] * inv_vol;
+cudaError_t launch_sum_parts(const double* parts, int n, double* tmp, double* out, const StatusCopy& st, cudaStream_t s,
+                             uint64_t* launches) {
+  return sum_parts(parts, n, 1, 1.0, 1.0, tmp, out, st, s, launches);
 }
 
 cudaError_t launch_qe_from_parts(const double* parts, int n, double* tmp, double* out2, double inv_vol,
-                                 cudaStream_t s) {
-  cudaError_t e = sum_parts(parts, n, 2, tmp, out2, s);
-  if (e != cudaSuccess) return e;
-  k_qe_scale<<<1, 1, 0, s>>>(out2, inv_vol);
-  return cudaGetLastError();
+                                 const StatusCopy& st, cudaStream_t s, uint64_t* launches) {
+  const double q = 1.0 / (4.0 * 3.14159265358979323846 * 3.14159265358979323846);
+  return sum_parts(parts, n, 2, q, 0.5 * inv_vol, tmp, out2, st, s, launches);
 }
 
 }  // namespace qcb

@@ -60,20 +60,27 @@ cudaError_t launch_hb_pass_meas(const LatDev& L, int parity, double beta, uint64
 
 // ---- observables (k_obs.cu) --------------------------------------------------------
 // Reductions write per-block partial sums into scratch (nparts doubles per quantity,
-// nparts = reduce_blocks()) and a final single-block kernel writes the FP64 total(s)
-// into out (device).
+// nparts = reduce_blocks()) and a final kernel writes the FP64 total(s) into out (device memory, or
+// pinned host memory).
 int reduce_blocks();
-cudaError_t launch_plaquette(const LatDev& L, double* scratch, double* out, cudaStream_t s, int block);
+// The status words' copy that the last kernel of a measurement makes (null: none): with it the
+// results and the status reach the host without copies of their own.
+struct StatusCopy {
+  const uint32_t* device = nullptr;
+  uint32_t* host = nullptr;
+};
+cudaError_t launch_plaquette(const LatDev& L, double* scratch, double* out, const StatusCopy& st, cudaStream_t s);
 // Plaquette sum with nblocks reduction blocks (scratch holds nblocks doubles); out[0] = sum.
 cudaError_t launch_plaquette_partials(const LatDev& L, int nblocks, double* scratch, double* out, cudaStream_t s);
 int reduce_threads();
-// out[0] = sum of parts[0 .. n) in a fixed order (two launches); tmp holds 256 doubles.
-cudaError_t launch_sum_parts(const double* parts, int n, double* tmp, double* out, cudaStream_t s);
+// out[0] = sum of parts[0 .. n) in a fixed order; tmp holds 256 doubles.
+cudaError_t launch_sum_parts(const double* parts, int n, double* tmp, double* out, const StatusCopy& st, cudaStream_t s,
+                             uint64_t* launches);
 // (Q, E) from per-block clover partials: parts[0 .. n) unscaled q sums, parts[n .. 2n) unscaled
 // e sums; out2[0] = Q = sum q / (4 pi^2), out2[1] = E = sum e / 2 * inv_vol.  tmp holds 512
 // doubles.
 cudaError_t launch_qe_from_parts(const double* parts, int n, double* tmp, double* out2, double inv_vol,
-                                 cudaStream_t s);
+                                 const StatusCopy& st, cudaStream_t s, uint64_t* launches);
 
 // Sets the calling thread's qcb_last_error() message; returns code.
 int set_error(int code, const char* msg);
