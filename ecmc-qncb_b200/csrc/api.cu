@@ -777,26 +777,22 @@ int qcb_heatbath_plaquette(qcb_lattice* L, double beta, int n_sweeps, int n_hits
     CU(launch_plaquette(L->dev, c->d_scratch, c->h_out, {c->d_status, c->h_status}, c->stream), "plaquette");
     c->launches += 2;
   } else {
-    const int nb = hb_meas_blocks(L->dev);
-    TRY(ensure_meas(L, 2 * (size_t)nb + 256));
+    const int np = hb_meas_parts(L->dev);
+    TRY(ensure_meas(L, (size_t)np + 256));
     for (int s = 0; s < n_sweeps; ++s) {
       const uint32_t sweep = (uint32_t)(sweep_offset + (uint64_t)s);
       const bool last = s == n_sweeps - 1;
-      for (int mu = 0; mu < 4; ++mu)
+      for (int mu = 0; mu < (last ? 3 : 4); ++mu)
         for (int par = 0; par < 2; ++par) {
-          if (last && mu == 3) {
-            CU(launch_hb_pass_meas(L->dev, par, beta, seed, sweep, n_hits, c->d_status, L->meas + (size_t)par * nb,
-                                   c->stream),
-               "measuring heatbath pass");
-          } else {
-            CU(launch_hb_pass(L->dev, mu, par, beta, seed, sweep, n_hits, c->d_status, c->stream, c->block),
-               "heatbath pass");
-          }
+          CU(launch_hb_pass(L->dev, mu, par, beta, seed, sweep, n_hits, c->d_status, c->stream, c->block),
+             "heatbath pass");
           c->launches++;
         }
+      if (last)
+        CU(launch_hb_meas(L->dev, beta, seed, sweep, n_hits, c->d_status, L->meas, c->stream, c->block, &c->launches),
+           "measuring heatbath passes");
     }
-    CU(launch_sum_parts(L->meas, 2 * nb, L->meas + 2 * nb, c->h_out, {c->d_status, c->h_status}, c->stream,
-                        &c->launches),
+    CU(launch_sum_parts(L->meas, np, L->meas + np, c->h_out, {c->d_status, c->h_status}, c->stream, &c->launches),
        "plaquette sum");
   }
   TRY(wait_status(c));

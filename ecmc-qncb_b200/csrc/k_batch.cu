@@ -227,31 +227,30 @@ cudaError_t launch_wait_probe(const uint32_t* flag, uint32_t* status, uint64_t l
 }
 
 // ---- batched observables --------------------------------------------------------------------
-// Plaquette: one reduction item per (lattice, tile of RED_SITES sites, both parities: item site
-// t is checkerboard index t >> 1 of parity t & 1), partial sums parts[item].  Plaquette and
+// Plaquette: one reduction item per (lattice, tile of RED_SITES sites, half of each parity), partial
+// sums parts[item].  Plaquette and
 // clover partials are then added by one block per lattice in a fixed order with Neumaier
 // compensation.
 constexpr int RED_SITES = 128;
 int batch_red_sites() { return RED_SITES; }
 
 template <typename S, int NR>
-__global__ void __launch_bounds__(RED_SITES, sizeof(S) == 4 ? 4 : 2) k_batch_plaquette(const BatchLat* __restrict__ lats,
+__global__ void __launch_bounds__(RED_SITES, sizeof(S) == 4 ? 5 : 3) k_batch_plaquette(const BatchLat* __restrict__ lats,
                                                          const uint32_t* __restrict__ rprefix, int nlat,
                                                          double* __restrict__ parts) {
   __shared__ double sh[RED_SITES / 32];
   const uint32_t item = blockIdx.x;
   const int l = find_lattice(rprefix, nlat, item);
   const BatchLat& B = lats[l];
-  const uint32_t t = (item - rprefix[l]) * RED_SITES + threadIdx.x;
+  const uint32_t i = block_site(item - rprefix[l]);
+  const int par = block_parity();
   Links<S, NR> f;
   f.p = reinterpret_cast<typename Links<S, NR>::V*>(B.links);
   f.stride = B.g.stride;
   double v = 0.0;
-  if (t < B.g.V) {
-    const int par = (int)(t & 1);  // both parities of a checkerboard index together
-    const uint32_t i = t >> 1;
+  if (i < B.g.Vh) {
     const Coord x = cb_coord(B.g, par, i);
-    v = (double)site_plaquette<Links<S, NR>, arith_t<S>>(B.g, f, x, par, i);
+    v = site_plaquettes<Links<S, NR>, arith_t<S>>(B.g, f, x, par, i, 0, 1, 6) * (1.0 / 3.0);
   }
   const double b = block_sum<RED_SITES>(v, sh);
   if (threadIdx.x == 0) parts[item] = b;

@@ -122,35 +122,45 @@ static cudaError_t hb_pass_impl(const LatDev& L, int mu, int par, double beta, u
   }
 }
 
-// Pass (mu = 3, par) of a measured sweep (whole lattices only): the updates of k_hb_pass, and
-// per block the FP64 sum of the spatial plaquettes of its sites (parity par), plus for par = 1
-// Re tr(U_3 A_3) of each updated link.  After the pass of parity 0 the spatial links and the
-// even U_3 links are final, so the pass of parity 1 sees final staples; every temporal
-// plaquette holds exactly one odd U_3 link, so Re tr(U_3(x) A_3(x)) over odd x counts each
-// temporal plaquette once, and the spatial plaquettes of both parities count each spatial one
-// once.
+// The last pass (mu = 3, parity 1) of a measured sweep (whole lattices only).  Blocks 0 .. nb - 1: the
+// updates of k_hb_pass, and per block the FP64 sum of Re tr(U_3 A_3) of its updated links.  After
+// the pass of parity 0 the spatial links and the even U_3 links are final, so this pass sees final
+// staples; every temporal plaquette holds exactly one odd U_3 link and is counted once.  The other
+// blocks sum the spatial plaquettes, `rows` blocks side by side for the three planes of 128 sites.
+// (Summed by the update's threads behind their links, in both passes, they cost on 32^4 FP64
+// 18-real 354 us on top of the passes and FP32 12-real 92, more than all six planes of k_plaquette
+// do; in blocks of their own 210 and 50.)
 template <typename S, int NR>
-__global__ void __launch_bounds__(128, HbMinBlocks<S>::value) k_hb_pass_meas(Geom g, Links<S, NR> f, int par, S beta,
+__global__ void __launch_bounds__(128, HbMinBlocks<S>::value) k_hb_pass_meas(Geom g, Links<S, NR> f, S beta,
                                                                             uint32_t k0, uint32_t k1, uint32_t sweep,
-                                                                            int n_hits, uint32_t* status,
-                                                                            double* __restrict__ parts) {
+                                                                            int n_hits, uint32_t* status, int nb,
+                                                                            int rows, double* __restrict__ parts) {
+  typedef arith_t<S> R;
   __shared__ double sh[4];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   double v = 0.0;
-  uint32_t fails = 0;
-  if (i < g.Vh) {
-    const Coord x = cb_coord(g, par, i);
-    arith_t<S> retr = 0;
-    fails = hb_update_at<Links<S, NR>, arith_t<S>, NR, 3, true>(g, f, x, par, i, arith_t<S>(beta), k0, k1, sweep, n_hits, &retr);
-    v = (double)site_plaquette_spatial<Links<S, NR>, arith_t<S>>(g, f, x, par, i);
-    if (par) v += (double)retr;
+  if ((int)blockIdx.x < nb) {
+    const uint32_t i = blockIdx.x * 128 + threadIdx.x;
+    R retr = 0;
+    uint32_t fails = 0;
+    if (i < g.Vh)
+      fails = hb_update_at<Links<S, NR>, R, NR, 3, true>(g, f, cb_coord(g, 1, i), 1, i, R(beta), k0, k1, sweep, n_hits,
+                                                         &retr);
+    if (fails) atomicAdd(status, fails);
+    v = (double)retr;
+  } else {
+    const uint32_t b = blockIdx.x - (uint32_t)nb, i = block_site(b / rows);
+    const int par = block_parity();
+    if (i < g.Vh)
+      v = site_plaquettes<Links<S, NR>, R>(g, f, cb_coord(g, par, i), par, i, (int)(b % rows), rows, 3);
   }
-  if (fails) atomicAdd(status, fails);
   const double b = block_sum<128>(v, sh);
   if (threadIdx.x == 0) parts[blockIdx.x] = b;
 }
 
-// The same with four lanes per link: lanes 0, 1, 2 take one spatial plane each.
+// Both passes mu = 3 with four lanes per link: lanes 0, 1, 2 also take one spatial plane each of the
+// pass's sites.
 __global__ void __launch_bounds__(128) k_hb_quad_meas(Geom g, Links<double, 18> f, int par, double beta, uint32_t k0,
                                                       uint32_t k1, uint32_t sweep, int n_hits, uint32_t* status,
                                                       double* __restrict__ parts) {
@@ -177,30 +187,6 @@ __global__ void __launch_bounds__(128) k_hb_quad_meas(Geom g, Links<double, 18> 
   if (threadIdx.x == 0) parts[blockIdx.x] = b;
 }
 
-template <typename S, int NR>
-static cudaError_t hb_meas_impl(const LatDev& L, int par, double beta, uint64_t seed, uint32_t sweep, int n_hits,
-                                uint32_t* status, double* parts, cudaStream_t s) {
-  Links<S, NR> f;
-  f.p = reinterpret_cast<typename Links<S, NR>::V*>(L.links);
-  f.stride = L.g.stride;
-  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-  if constexpr (sizeof(S) == 8 && NR == 18)
-    if (quad_pass(L))
-      return pdl_launch(k_hb_quad_meas, dim3(grid_for(4 * (uint64_t)L.g.Vh, 128)), 128, s, L.g, f, par, beta, k0, k1,
-                        sweep, n_hits, status, parts);
-  k_hb_pass_meas<S, NR><<<grid_for(L.g.Vh, 128), 128, 0, s>>>(L.g, f, par, S(beta), k0, k1, sweep, n_hits, status,
-                                                              parts);
-  return cudaGetLastError();
-}
-
-int hb_meas_blocks(const LatDev& L) { return (int)grid_for((quad_pass(L) ? 4 : 1) * (uint64_t)L.g.Vh, 128); }
-
-cudaError_t launch_hb_pass_meas(const LatDev& L, int parity, double beta, uint64_t seed, uint32_t sweep, int n_hits,
-                                uint32_t* status, double* parts, cudaStream_t s) {
-  if (L.g.tlo != 0 || L.g.thi != L.g.L[3] - 1) return cudaErrorInvalidValue;  // whole lattices only
-  QCB_DISPATCH_STORE(L, hb_meas_impl, L, parity, beta, seed, sweep, n_hits, status, parts, s);
-}
-
 cudaError_t launch_hb_pass(const LatDev& L, int mu, int parity, double beta, uint64_t seed, uint32_t sweep,
                            int n_hits, uint32_t* status, cudaStream_t s, int block, const int* frozen) {
   if (block <= 0) block = 128;
@@ -210,6 +196,45 @@ cudaError_t launch_hb_pass(const LatDev& L, int mu, int parity, double beta, uin
     for (int d = 0; d < 4; ++d) fm.shift[d] = frozen[1 + d];
   }
   QCB_DISPATCH_STORE(L, hb_pass_impl, L, mu, parity, beta, seed, sweep, n_hits, status, s, block, fm);
+}
+
+// Planes side by side while all blocks then fit on the chip at once.
+static int spatial_rows(const LatDev& L) { return 3 * grid_for(L.g.Vh, 64) <= 148 * 3 ? 3 : 1; }
+int hb_meas_parts(const LatDev& L) {
+  return quad_pass(L) ? 2 * (int)grid_for(4 * (uint64_t)L.g.Vh, 128)
+                      : (int)grid_for(L.g.Vh, 128) + spatial_rows(L) * (int)grid_for(L.g.Vh, 64);
+}
+
+template <typename S, int NR>
+static cudaError_t hb_meas_impl(const LatDev& L, double beta, uint64_t seed, uint32_t sweep, int n_hits,
+                                uint32_t* status, double* parts, cudaStream_t s, int block, uint64_t* launches) {
+  Links<S, NR> f;
+  f.p = reinterpret_cast<typename Links<S, NR>::V*>(L.links);
+  f.stride = L.g.stride;
+  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
+  cudaError_t e = cudaSuccess;
+  if constexpr (sizeof(S) == 8 && NR == 18)
+    if (quad_pass(L)) {
+      const dim3 grid(grid_for(4 * (uint64_t)L.g.Vh, 128));
+      for (int par = 0; par < 2 && e == cudaSuccess; ++par)
+        e = pdl_launch(k_hb_quad_meas, grid, 128, s, L.g, f, par, beta, k0, k1, sweep, n_hits, status,
+                       parts + (size_t)par * grid.x);
+      *launches += 2;
+      return e;
+    }
+  e = launch_hb_pass(L, 3, 0, beta, seed, sweep, n_hits, status, s, block, nullptr);
+  const int nb = (int)grid_for(L.g.Vh, 128), rows = spatial_rows(L);
+  if (e == cudaSuccess)
+    e = pdl_launch(k_hb_pass_meas<S, NR>, dim3(hb_meas_parts(L)), 128, s, L.g, f, S(beta), k0, k1, sweep, n_hits, status,
+                   nb, rows, parts);
+  *launches += 2;
+  return e;
+}
+
+cudaError_t launch_hb_meas(const LatDev& L, double beta, uint64_t seed, uint32_t sweep, int n_hits, uint32_t* status,
+                           double* parts, cudaStream_t s, int block, uint64_t* launches) {
+  if (L.g.tlo != 0 || L.g.thi != L.g.L[3] - 1) return cudaErrorInvalidValue;  // whole lattices only
+  QCB_DISPATCH_STORE(L, hb_meas_impl, L, beta, seed, sweep, n_hits, status, parts, s, block, launches);
 }
 
 }  // namespace qcb

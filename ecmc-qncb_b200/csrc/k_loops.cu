@@ -83,11 +83,11 @@ std::vector<FlowLat> flow_rounds(const LatDev& L, const LoopDev& k) {
 }
 
 static uint32_t tiles_of(const Geom& g, int slices, uint32_t tile) {
-  return 2 * (((uint32_t)slices * (uint32_t)(g.str[3] / 2) + tile - 1) / tile);  // both parities
+  return ((uint32_t)slices * (uint32_t)(g.str[3] / 2) + tile - 1) / tile;
 }
-uint32_t loops_blocks(const FlowLat& r) { return tiles_of(r.g, r.kn, FLOW_THREADS); }
-uint32_t qe_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, FLOW_THREADS); }
-uint32_t update_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, r.tile); }
+uint32_t loops_blocks(const FlowLat& r) { return tiles_of(r.g, r.kn, FLOW_THREADS / 2); }
+uint32_t qe_blocks(const FlowLat& r) { return tiles_of(r.g, r.t1 - r.t0, FLOW_THREADS / 2); }
+uint32_t update_blocks(const FlowLat& r) { return 2 * tiles_of(r.g, r.t1 - r.t0, r.tile); }  // both parities
 
 // ---- the loops --------------------------------------------------------------------------
 // One thread per site and grid row: row y of n takes planes y, y + n, ...; the planes run
@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_LOOPS_MINB3
   if (MULTI && step >= L.nsteps) return;
   const uint32_t b = MULTI ? blockIdx.x - __ldg(&prefix[l]) : blockIdx.x;
   const Links<S, NR> f = flow_links<S, NR>(L, swap);
-  const uint32_t n = (uint32_t)L.kn * (uint32_t)(L.g.str[3] >> 1), k = (b >> 1) * FLOW_THREADS + threadIdx.x;
-  if (k < n) loops_site<S, NR, TRACE>(L, f, (int)(b & 1), k);
+  const uint32_t n = (uint32_t)L.kn * (uint32_t)(L.g.str[3] >> 1), k = block_site(b);
+  if (k < n) loops_site<S, NR, TRACE>(L, f, block_parity(), k);
 }
 
 template <typename S, int NR>
@@ -207,9 +207,9 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_QE_MINB32 :
   const uint32_t b = MULTI ? blockIdx.x - __ldg(&prefix[l]) : blockIdx.x;
   const Links<S, NR> f = flow_links<S, NR>(L, swap);
   const uint32_t half = (uint32_t)(L.g.str[3] >> 1), n = (uint32_t)(L.t1 - L.t0) * half,
-                 k = (b >> 1) * FLOW_THREADS + threadIdx.x;
+                 k = block_site(b);
   double q = 0.0, e = 0.0;
-  if (k < n) qe_site<S, NR>(L, f, (int)(b & 1), (uint32_t)L.t0 * half + k, &q, &e);
+  if (k < n) qe_site<S, NR>(L, f, block_parity(), (uint32_t)L.t0 * half + k, &q, &e);
   const double bq = block_sum<FLOW_THREADS>(q, sh);
   const double be = block_sum<FLOW_THREADS>(e, sh);
   if (threadIdx.x == 0) {

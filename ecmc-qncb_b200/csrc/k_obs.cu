@@ -2,10 +2,11 @@
 //
 // Reference: mean_plaquette_local / _global (src/observables/observables_mpi.cpp:8-43): serial
 // sum of Re tr(U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag)/3 over x and mu < nu, / (6V).
-// Here: one thread per site (the two parities of a checkerboard index adjacent; a slab
-// skips its halo slices), per-site value in the lattice's arithmetic type, converted to FP64; FP64 tree reduction inside each block; the block partials are
+// Here: one thread per site (a slab skips its halo slices), per-site value in the lattice's arithmetic type, converted to FP64; FP64 tree reduction inside each block; the block partials are
 // summed in a fixed order with Neumaier compensation by k_total.  The grid
 // is a fixed multiple of the SM count (grid-stride loop), so the scratch is bounded.
+#include <algorithm>
+
 #include "dispatch.cuh"
 #include "obs_site.cuh"
 #include "reduce.cuh"
@@ -14,13 +15,14 @@
 namespace qcb {
 
 constexpr int RED_THREADS = 128;
-constexpr int RED_BLOCKS = 148 * 8;
+// One block per 64 checkerboard indices up to 60 per SM (32^4: 8192), from there a grid-stride loop.
+constexpr int RED_BLOCKS = 148 * 60;
 
-// Minimum resident blocks per SM of the reduction: FP32 4 x 128 threads (128 registers), FP64
-// 2 x 128 threads.
+// Minimum resident blocks per SM of the reduction (32^4: FP32 5 114 us, 4 121; FP64 3 224 us, 2 267,
+// 4 235).
 template <typename S>
 struct RedMinBlocks {
-  static constexpr int value = sizeof(S) == 4 ? 4 : 2;
+  static constexpr int value = sizeof(S) == 4 ? 5 : 3;
 };
 
 int reduce_blocks() { return RED_BLOCKS; }
@@ -67,45 +69,47 @@ static cudaError_t total(const double* parts, int n, int nq, double scale0, doub
   return pdl_launch(k_total, dim3(nq), TOTAL_THREADS, s, parts, n, scale0, scale1, out, st.device, st.host);
 }
 
-// Reduction grid: one block per RED_THREADS sites, at most RED_BLOCKS.
-static int red_grid(const Geom& g) {
-  const uint64_t want = ((uint64_t)g.V + RED_THREADS - 1) / RED_THREADS;
-  return (int)(want < (uint64_t)RED_BLOCKS ? want : (uint64_t)RED_BLOCKS);
-}
-
+// Per block, the sum of Re tr P / 3 over planes blockIdx.y, blockIdx.y + gridDim.y, ... of its sites.
 template <typename S, int NR>
-__global__ void __launch_bounds__(RED_THREADS, RedMinBlocks<S>::value) k_plaquette(Geom g, Links<S, NR> f, double* __restrict__ parts) {
+__global__ void __launch_bounds__(RED_THREADS, RedMinBlocks<S>::value) k_plaquette(Geom g, Links<S, NR> f,
+                                                                                   double* __restrict__ parts) {
   __shared__ double sh[RED_THREADS / 32];
+  pdl_launch_dependents();
+  pdl_wait();
   double acc = 0.0;
-  const uint64_t n = (uint64_t)g.V;
-  for (uint64_t t = (uint64_t)blockIdx.x * RED_THREADS + threadIdx.x; t < n; t += (uint64_t)gridDim.x * RED_THREADS) {
-    // both parities of a checkerboard index together: a site's neighbours (opposite
-    // parity) are then read close in time, from L2
-    const int par = (int)(t & 1);
-    const uint32_t i = (uint32_t)(t >> 1);
+  const int par = block_parity();
+  for (uint32_t b = blockIdx.x; b * 64 < g.Vh; b += gridDim.x) {
+    const uint32_t i = block_site(b);
+    if (i >= g.Vh) continue;
     const Coord x = cb_coord(g, par, i);
-    if (own_site(g, x.c[3])) acc += (double)site_plaquette<Links<S, NR>, arith_t<S>>(g, f, x, par, i);
+    if (own_site(g, x.c[3]))
+      acc += site_plaquettes<Links<S, NR>, arith_t<S>>(g, f, x, par, i, blockIdx.y, gridDim.y, 6);
   }
-  double b = block_sum<RED_THREADS>(acc, sh);
-  if (threadIdx.x == 0) parts[blockIdx.x] = b;
+  const double b = block_sum<RED_THREADS>(acc * (1.0 / 3.0), sh);
+  if (threadIdx.x == 0) parts[blockIdx.y * gridDim.x + blockIdx.x] = b;
+}
+
+// Planes side by side while the sites' blocks are fewer than fill the chip.
+static dim3 plaquette_grid(const Geom& g, int most) {
+  const int nb = (int)std::min<uint64_t>(((uint64_t)g.Vh + 63) / 64, (uint64_t)most);
+  return dim3(nb, nb * 6 <= std::min(most, 148 * 8) ? 6 : 1);
 }
 
 template <typename S, int NR>
-static cudaError_t plaquette_impl(const LatDev& L, int nb, double* scratch, double* out, const StatusCopy& st,
+static cudaError_t plaquette_impl(const LatDev& L, int most, double* scratch, double* out, const StatusCopy& st,
                                   cudaStream_t s) {
   Links<S, NR> f;
   f.p = reinterpret_cast<typename Links<S, NR>::V*>(L.links);
   f.stride = L.g.stride;
-  k_plaquette<S, NR><<<nb, RED_THREADS, 0, s>>>(L.g, f, scratch);
-  const cudaError_t e = cudaGetLastError();
-  return e != cudaSuccess ? e : total(scratch, nb, 1, 1.0, 1.0, out, st, s);
+  const dim3 grid = plaquette_grid(L.g, most);
+  const cudaError_t e = pdl_launch(k_plaquette<S, NR>, grid, RED_THREADS, s, L.g, f, scratch);
+  return e != cudaSuccess ? e : total(scratch, (int)(grid.x * grid.y), 1, 1.0, 1.0, out, st, s);
 }
 
 cudaError_t launch_plaquette(const LatDev& L, double* scratch, double* out, const StatusCopy& st, cudaStream_t s) {
-  QCB_DISPATCH_STORE(L, plaquette_impl, L, red_grid(L.g), scratch, out, st, s);
+  QCB_DISPATCH_STORE(L, plaquette_impl, L, RED_BLOCKS, scratch, out, st, s);
 }
 
-// Same reduction with a caller-chosen number of blocks (partials written to scratch[0..nblocks)).
 cudaError_t launch_plaquette_partials(const LatDev& L, int nblocks, double* scratch, double* out, cudaStream_t s) {
   if (nblocks < 1) return cudaErrorInvalidValue;
   QCB_DISPATCH_STORE(L, plaquette_impl, L, nblocks, scratch, out, StatusCopy(), s);

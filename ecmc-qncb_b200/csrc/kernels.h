@@ -48,15 +48,12 @@ cudaError_t launch_translate(const LatDev& dst, const LatDev& src, const int shi
 cudaError_t launch_hb_pass(const LatDev& L, int mu, int parity, double beta, uint64_t seed, uint32_t sweep,
                            int n_hits, uint32_t* status, cudaStream_t s, int block, const int* frozen = nullptr);
 
-// Pass (mu = 3, parity) of the last sweep of a measurement: the same updates as
-// launch_hb_pass, and one FP64 partial per block of 128 threads written to parts[0 ..
-// hb_meas_blocks(L)): the sum over the block's sites x of Re tr of the spatial plaquettes
-// P_ij(x), i < j < 3, plus for parity 1 Re tr(U_3(x) A_3(x)) with the updated link.  After
-// both parities, the partials of the two passes sum to the sum of Re tr P over all 6V
+// The passes mu = 3 of the last sweep of a measurement: the updates of launch_hb_pass for both
+// parities, and hb_meas_parts(L) FP64 partials that sum to the sum of Re tr P over all 6V
 // plaquettes of the final links.
-int hb_meas_blocks(const LatDev& L);
-cudaError_t launch_hb_pass_meas(const LatDev& L, int parity, double beta, uint64_t seed, uint32_t sweep,
-                                int n_hits, uint32_t* status, double* parts, cudaStream_t s);
+int hb_meas_parts(const LatDev& L);
+cudaError_t launch_hb_meas(const LatDev& L, double beta, uint64_t seed, uint32_t sweep, int n_hits, uint32_t* status,
+                           double* parts, cudaStream_t s, int block, uint64_t* launches);
 
 // ---- observables (k_obs.cu) --------------------------------------------------------
 // Reductions write per-block partial sums into scratch (nparts doubles per quantity,
@@ -70,7 +67,7 @@ struct StatusCopy {
   uint32_t* host = nullptr;
 };
 cudaError_t launch_plaquette(const LatDev& L, double* scratch, double* out, const StatusCopy& st, cudaStream_t s);
-// Plaquette sum with nblocks reduction blocks (scratch holds nblocks doubles); out[0] = sum.
+// Plaquette sum with at most nblocks reduction blocks (scratch holds nblocks doubles); out[0] = sum.
 cudaError_t launch_plaquette_partials(const LatDev& L, int nblocks, double* scratch, double* out, cudaStream_t s);
 int reduce_threads();
 // out[0] = sum of parts[0 .. n) in a fixed order; tmp holds 256 doubles.

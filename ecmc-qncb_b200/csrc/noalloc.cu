@@ -61,9 +61,7 @@ extern "C" int qcb_plaquette_noalloc(const void* links, const int dims[4], int p
 
   // One partial per reduction block; the grid never exceeds the library's reduction grid.
   const uint64_t want = (vol + (uint64_t)reduce_threads() - 1) / (uint64_t)reduce_threads();
-  const int nblocks = (int)(want < (uint64_t)reduce_blocks() ? want : (uint64_t)reduce_blocks());
-  if (nblocks > QCB_NOALLOC_MAX_PARTIALS)
-    return set_error(QCB_ERR_INVALID, "reduction needs more partial sums than the static scratch holds");
+  const int nblocks = (int)(want < (uint64_t)QCB_NOALLOC_MAX_PARTIALS ? want : (uint64_t)QCB_NOALLOC_MAX_PARTIALS);
 
   double* scratch = nullptr;
   cudaError_t e = cudaGetSymbolAddress((void**)&scratch, g_noalloc_scratch);
