@@ -2,11 +2,14 @@
 //
 // A pass over a small lattice has fewer links than the chip has lanes and takes as long as one
 // link: thousands of dependent FP64 instructions.  Here lanes 0, 1, 2 of a group form a row each
-// of the staple sum, and the Kennedy-Pendleton attempts of a draw go to the lanes side by side
-// (the first accepted one counts, as in the loop of kp_draw_inline; the draws are a function of
-// their counters).  Every element and every draw is computed by the operations of hb_link.cuh in
-// their order, so the links are the same bit for bit.  Pass on 8^4, 18-real: 14.2 -> 11.3 us, on 12^4
-// 17.9 -> 13.4 us.  In FP32, and with 12-real links (whose third rows take all lanes' rows), four
+// of the staple sum, and lane sg takes the draw of subgroup sg: what two attempts and the
+// direction need of their random words alone (logarithms, sines) is computed before the links
+// arrive, the three subgroups side by side.  Every element and every draw is computed by the
+// operations of hb_link.cuh in their order, so the links are the same bit for bit.  Pass on 8^4,
+// 18-real: one lane 11.6 us, four lanes 9.0 (with the attempts of one draw side by side, behind the
+// staple, 10.1); on 12^4 12.3 and 11.9.  (One lane with its words ahead, in shared memory, is
+// slower: 32^4 192 us against 185, FP32 8^4 7.0 against 5.7: the loads wait for the words there.)
+// In FP32, and with 12-real links (whose third rows take all lanes' rows), four
 // lanes were slower on 10^4 already, and on 8^4 in FP32 (5.7 against 8.5 us).
 #pragma once
 #include "hb_link.cuh"

@@ -34,7 +34,6 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_FLOW_MINB32
                   const uint32_t* __restrict__ prefix, int nlat, int swap, int step) {
   typedef arith_t<S> R;
   typedef Links<S, NR> F;
-  pdl_launch_dependents();
   pdl_wait();
   const int l = MULTI ? lattice_of(prefix, nlat, blockIdx.x) : 0;
   const FlowLat& L = MULTI ? lats[l] : one;

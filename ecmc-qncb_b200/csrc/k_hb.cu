@@ -54,9 +54,6 @@ template <typename S, int NR, int MU, bool FROZEN>
 __global__ void __launch_bounds__(128, HbMinBlocks<S>::value) k_hb_pass(Geom g, Links<S, NR> f, int par, S beta, uint32_t k0,
                                                  uint32_t k1, uint32_t sweep, int n_hits, uint32_t* status,
                                                  FrozenMask fm) {
-  // programmatic dependent launch: the next pass may be scheduled during this one's last
-  // wave; this pass reads nothing before the previous kernel has completed
-  pdl_launch_dependents();
   pdl_wait();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.Vh) return;
@@ -71,7 +68,6 @@ template <bool FROZEN>
 __global__ void __launch_bounds__(128) k_hb_quad(Geom g, Links<double, 18> f, int mu, int par, double beta, uint32_t k0,
                                                  uint32_t k1, uint32_t sweep, int n_hits, uint32_t* status,
                                                  FrozenMask fm) {
-  pdl_launch_dependents();
   pdl_wait();
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (i >= g.Vh) return;
@@ -85,14 +81,14 @@ __global__ void __launch_bounds__(128) k_hb_quad(Geom g, Links<double, 18> f, in
 }
 
 // Four lanes per link while all of a pass's links are then resident at once (148 SMs of three
-// blocks of 32 links): 12^4 (10368 links) takes 12.1 us against 17.8, 14^4 (19208) 19.5 against 18.6.
+// blocks of 32 links): 12x12x12x16 (13824 links) takes 12.1 us against 12.4,
+// 12x12x14x16 (16128) 18.8 against 12.6; 8^4 9.0 against 11.6.
 static bool quad_pass(const LatDev& L) {
   return L.prec == QCB_PREC_FP64 && L.nr == 18 && L.g.Vh <= 148u * 3u * 32u;
 }
 
 // Launch with programmatic stream serialization: the pass's blocks become resident while the
-// previous kernel drains and wait in pdl_wait().  Measured per pass: 32^4 FP32-12 74.7 -> 72.9
-// us, 64^4 1211 -> 1144 us, 32^4 FP64-18 200.7 -> 197.4 us.
+// previous kernel drains and wait in pdl_wait() (pass on 16^4 FP32-12, us: 9.6 without, 7.1).
 template <typename S, int NR, int MU>
 static cudaError_t hb_pass_launch(dim3 grid, int block, cudaStream_t s, const Geom& g, const Links<S, NR>& f, int par,
                                   S beta, uint32_t k0, uint32_t k1, uint32_t sweep, int n_hits, uint32_t* status,
@@ -137,7 +133,6 @@ __global__ void __launch_bounds__(128, HbMinBlocks<S>::value) k_hb_pass_meas(Geo
                                                                             int rows, double* __restrict__ parts) {
   typedef arith_t<S> R;
   __shared__ double sh[4];
-  pdl_launch_dependents();
   pdl_wait();
   double v = 0.0;
   if ((int)blockIdx.x < nb) {
@@ -165,7 +160,6 @@ __global__ void __launch_bounds__(128) k_hb_quad_meas(Geom g, Links<double, 18> 
                                                       uint32_t k1, uint32_t sweep, int n_hits, uint32_t* status,
                                                       double* __restrict__ parts) {
   __shared__ double sh[4];
-  pdl_launch_dependents();
   pdl_wait();
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   double v = 0.0;

@@ -131,7 +131,6 @@ template <typename S, int NR, bool TRACE, bool MULTI>
 __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_LOOPS_MINB32 : QCB_LOOPS_MINB64)
     k_loops(const __grid_constant__ FlowLat one, const FlowLat* __restrict__ lats, const uint32_t* __restrict__ prefix,
             int nlat, int swap, int step) {
-  pdl_launch_dependents();
   pdl_wait();
   const int l = MULTI ? lattice_of(prefix, nlat, blockIdx.x) : 0;
   const FlowLat& L = MULTI ? lats[l] : one;
@@ -200,7 +199,6 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_QE_MINB32 :
                const uint32_t* __restrict__ prefix, int nlat, int swap, double* __restrict__ parts, uint32_t first,
                uint32_t nparts) {
   __shared__ double sh[FLOW_THREADS / 32];
-  pdl_launch_dependents();
   pdl_wait();
   const int l = MULTI ? lattice_of(prefix, nlat, blockIdx.x) : 0;
   const FlowLat& L = MULTI ? lats[l] : one;

@@ -39,7 +39,6 @@ __global__ void __launch_bounds__(TOTAL_THREADS) k_total(const double* __restric
                                                          const uint32_t* __restrict__ status,
                                                          uint32_t* __restrict__ host_status) {
   __shared__ double ls[TOTAL_THREADS / 32], lc[TOTAL_THREADS / 32];
-  pdl_launch_dependents();
   pdl_wait();
   const double* p = parts + (size_t)blockIdx.x * n;
   double s = 0.0, c = 0.0;
@@ -74,7 +73,6 @@ template <typename S, int NR>
 __global__ void __launch_bounds__(RED_THREADS, RedMinBlocks<S>::value) k_plaquette(Geom g, Links<S, NR> f,
                                                                                    double* __restrict__ parts) {
   __shared__ double sh[RED_THREADS / 32];
-  pdl_launch_dependents();
   pdl_wait();
   double acc = 0.0;
   const int par = block_parity();
