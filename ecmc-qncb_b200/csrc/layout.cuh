@@ -285,7 +285,7 @@ struct AlgStore<float> {
   static constexpr int NC = 2;
 };
 
-template <typename S, int LM = LD_RO>
+template <typename S>
 struct AlgField {
   typedef typename AlgStore<S>::V V;
   static constexpr int NC = AlgStore<S>::NC;
@@ -299,8 +299,9 @@ struct AlgField {
     alg8<R> z;
     const S* q;
     V v[NC];
+    const V* at = p + idx(mu, par, 0, i);
 #pragma unroll
-    for (int c = 0; c < NC; ++c) v[c] = (LM == LD_CG) ? __ldcg(&p[idx(mu, par, c, i)]) : p[idx(mu, par, c, i)];
+    for (int c = 0; c < NC; ++c) v[c] = at[c * (size_t)stride];
     q = reinterpret_cast<const S*>(v);
 #pragma unroll
     for (int k = 0; k < 8; ++k) z.a[k] = R(q[k]);
@@ -312,8 +313,9 @@ struct AlgField {
     S* q = reinterpret_cast<S*>(v);
 #pragma unroll
     for (int k = 0; k < 8; ++k) q[k] = S(z.a[k]);
+    V* at = p + idx(mu, par, 0, i);
 #pragma unroll
-    for (int c = 0; c < NC; ++c) p[idx(mu, par, c, i)] = v[c];
+    for (int c = 0; c < NC; ++c) at[c * (size_t)stride] = v[c];
   }
 };
 
