@@ -523,6 +523,11 @@ int qcb_server_create(qcb_ctx* ctx, const qcb_server_config* cfg, qcb_server** o
       cudaMallocHost(&s->h_out, 3 * (size_t)s->cap * sizeof(double)) != cudaSuccess ||
       cudaMemset(s->d_status, 0, 4 * sizeof(uint32_t)) != cudaSuccess)
     return bail("cannot allocate server buffers");
+  // Loop buffer of the flow jobs that fit into the arena (a job's loops take less than half of its
+  // links and accumulator).  Grown in the first ticks instead, its cudaFree and cudaMalloc held a
+  // tick for up to 0.6 s while the driver cleared memory freed before.  Less is no error: the jobs
+  // then take turns.
+  if (loops_reserve(&s->loops, std::max<size_t>(budget / 2, 1), 1) != cudaSuccess) cudaGetLastError();
   s->t0 = std::chrono::steady_clock::now();
   s->thr = std::thread(scheduler, s);
   ctx_ref(ctx);

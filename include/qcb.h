@@ -323,7 +323,9 @@ typedef struct qcb_job_result {
 } qcb_job_result;
 typedef struct qcb_server_config {
   int precision, storage; /* of every job's lattice */
-  size_t hbm_budget;      /* bytes of device work space (0: 80% of the free memory) */
+  size_t hbm_budget;      /* bytes of device work space (0: 80% of the free memory); the plaquette
+                             loops of the flow jobs take half as much beside it, at most 1 GiB
+                             (or two time slices' of a larger lattice), less if not free */
   int max_jobs;           /* concurrent jobs (0: 256) */
   int quantum_sweeps;     /* sweeps per sweeps-job per tick (0: 2) */
   int quantum_steps;      /* RK3 steps per flow-job per tick (0: 4) */
