@@ -130,7 +130,13 @@ int loop_rounds(qcb_lattice* L, const LatDev& d, void* b, double eps, std::vecto
   qcb_ctx* c = L->ctx;
   const Geom& g = d.g;
   const size_t least = loops_bytes(g, d.prec, 2);
-  if (loops_reserve(&c->loops, loops_bytes(g, d.prec, g.L[3]), least) != cudaSuccess)
+  size_t want = loops_bytes(g, d.prec, g.L[3]), free = 0, total = 0;
+  // The full buffer at once where it is a sixteenth of the free memory or less: growing it for a
+  // larger lattice frees and allocates again, which took up to 0.6 s behind memory that the driver
+  // was still clearing.
+  if (want > c->loops.bytes && cudaMemGetInfo(&free, &total) == cudaSuccess && free / 16 >= LOOPS_MAX_BYTES)
+    want = std::max(want, LOOPS_MAX_BYTES);
+  if (loops_reserve(&c->loops, want, least) != cudaSuccess)
     return fail(QCB_ERR_NOMEM, "cannot allocate the plaquette-loop work space");
   const LoopDev k = loops_view(c->loops, 0, g, d.prec, loops_slices(g, d.prec, c->loops.bytes));
   *rounds = flow_rounds(d, k);

@@ -476,19 +476,19 @@ __device__ __forceinline__ void exp_coef64(const double (&xa)[8], double (&q)[6]
   for (int k = 0; k < 6; ++k) q[k] = c[k];
 }
 
-// q0, q1, q2 of exp(X) in R.
+// q0 (in FP32 q0 - 1), q1, q2 of exp(X) in R.
 template <typename R>
 __device__ __forceinline__ void exp_coef(const alg8<R>& x, cx<R>& q0, cx<R>& q1, cx<R>& q2) {
   double xa[8], q[6];
 #pragma unroll
   for (int k = 0; k < 8; ++k) xa[k] = (double)x.a[k];
   exp_coef64(xa, q);
-  q0 = mk<R>(R(q[0]), R(q[1]));
+  q0 = mk<R>(R(is_fp32<R>::value ? q[0] - 1.0 : q[0]), R(q[1]));
   q1 = mk<R>(R(q[2]), R(q[3]));
   q2 = mk<R>(R(q[4]), R(q[5]));
 }
 
-// Returns exp(X).
+// Returns exp(X); in FP32 exp(X) - 1, whose entries are of the order of X and keep their last bits.
 template <typename R>
 __device__ __forceinline__ m3<R> exp_su3(const alg8<R>& x) {
   cx<R> q0, q1, q2;
