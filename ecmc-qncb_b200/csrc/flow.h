@@ -20,10 +20,13 @@
 namespace qcb {
 
 // The loop buffer as the kernels see it: slices time slices of 6 planes x 2 parities, chunk
-// arrays of `stride` elements (the algebra layout of AlgField), then the traces.
+// arrays of `stride` elements (the algebra layout of AlgField), then the traces, then (18-real
+// links) a byte for each of the 4 x 2 links of a checkerboard index that is set where the link is not
+// unitary.
 struct LoopDev {
   void* p;
   void* tr;
+  uint8_t* off;
   uint32_t stride;
   int slices;
 };

@@ -13,7 +13,7 @@ static size_t loops_stride(const Geom& g, int slices) {
   return ((size_t)slices * (size_t)(g.str[3] / 2) + 63) / 64 * 64;
 }
 size_t loops_bytes(const Geom& g, int prec, int slices) {
-  return (size_t)(6 * 2 * 9) * loops_stride(g, slices) * (prec == QCB_PREC_FP64 ? 8 : 4);
+  return loops_stride(g, slices) * ((size_t)(6 * 2 * 9) * (prec == QCB_PREC_FP64 ? 8 : 4) + 4 * 2);
 }
 int loops_slices(const Geom& g, int prec, size_t bytes) {
   if (loops_bytes(g, prec, g.L[3]) <= bytes) return g.L[3];
@@ -46,6 +46,7 @@ LoopDev loops_view(const LoopBuf& buf, size_t off, const Geom& g, int prec, int 
   LoopDev k;
   k.p = (char*)buf.p + off;
   k.tr = (char*)buf.p + off + 6 * 2 * 8 * st * es;
+  k.off = (uint8_t*)buf.p + off + 6 * 2 * 9 * st * es;
   k.stride = (uint32_t)st;
   k.slices = slices;
   return k;
@@ -114,7 +115,13 @@ __device__ __forceinline__ void loops_site(const FlowLat& L, const Links<S, NR>&
     const int mu = p < 3 ? 0 : (p < 5 ? 1 : 2), nu = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
     if (mu != have) U = lead<Links<S, NR>, R>(f, mu, par, i);
     have = mu;
-    const m3<R> W = plaquette_loop<Links<S, NR>, R>(f, U, mu, nu, par, i, cb_index((uint32_t)((int32_t)x.s + sel4(o.up, mu))),
+    const m3<R> Unu = lead<Links<S, NR>, R>(f, nu, par, i);
+    if constexpr (NR == 18 && TRACE) {  // each link once: U_0, U_3, U_1, U_2
+      if (p == 0 || p == 3 || p == 5) K.store_off(mu, par, jx, off_unitary<S>(U));
+      if (p == 2) K.store_off(3, par, jx, off_unitary<S>(Unu));
+    }
+    const m3<R> W = plaquette_loop<Links<S, NR>, R>(f, U, Unu, mu, nu, par,
+                                                    cb_index((uint32_t)((int32_t)x.s + sel4(o.up, mu))),
                                                     cb_index((uint32_t)((int32_t)x.s + sel4(o.up, nu))));
     K.template store<R>(p, par, jx, proj_ta(W));
     if (TRACE) K.template store_tr<R>(p, par, jx, (W.e[0][0].im + W.e[1][1].im + W.e[2][2].im) * R(1.0 / 3.0));
@@ -164,6 +171,9 @@ cudaError_t launch_loops(const FlowSet& s, int prec, int nr, bool trace, int swa
 // Three transports a plane where four leaves were nine products: Q and E of 32^4 alone, loops
 // included, FP32 12-real 572 -> 370 us, FP64 18-real 1301 -> 720 us; with the loops already there
 // for an RK3 step, FP32 210 us more.
+// In 18-real storage the bytes of the links that are not unitary are read first, for all planes
+// together: 20x24x28x36 with SU(3) links FP64 296 us without the test, 320 with it (335 with the
+// bytes read plane by plane); links that need the products 530, FP32 200, 217 and 312.
 template <typename S, int NR>
 __device__ __forceinline__ void qe_site(const FlowLat& L, const Links<S, NR>& f, int par, uint32_t i, double* q,
                                         double* e) {
@@ -171,12 +181,30 @@ __device__ __forceinline__ void qe_site(const FlowLat& L, const Links<S, NR>& f,
   const Loops<S> K(L.k, L.g);
   const Coord x = cb_coord(L.g, par, i);
   const NbOff o = nb_offsets(L.g, x);
+  unsigned bad = 0;
+  if constexpr (NR == 18) {
+    const int t = x.c[3], tm = t == 0 ? L.g.L[3] - 1 : t - 1;
+    bool side[4];  // U_d(x-d)
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      const uint32_t k = (uint32_t)((int32_t)x.s + o.dn[d]) >> 1;
+      side[d] = K.load_off(d, par ^ 1, d == 3 ? K.at(k, tm, t - 1) : K.at(k, t, t));
+    }
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+      const int mu = p < 3 ? 0 : (p < 5 ? 1 : 2), nu = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
+      const uint32_t k = (uint32_t)((int32_t)x.s + o.dn[mu] + o.dn[nu]) >> 1;
+      const bool far = K.load_off(nu, par, nu == 3 ? K.at(k, tm, t - 1) : K.at(k, t, t));
+      if (side[mu] || side[nu] || far) bad |= 1u << p;
+    }
+  }
   ah9<R> prev;
 #pragma unroll 1
   for (int p = 0; p < 6; ++p) {
     const int h = p >> 1;
     const int mu = (p & 1) == 0 ? 0 : (h == 0 ? 2 : 1), nu = (p & 1) == 0 ? h + 1 : (h == 2 ? 2 : 3);
-    const ah9<R> F = clover_plane<Links<S, NR>, S, R>(f, K, x, o, mu, nu, par, i, L.g.L[3]);
+    const bool multiply = (bad >> plane_of(mu, nu)) & 1;
+    const ah9<R> F = clover_plane<Links<S, NR>, S, R>(f, K, x, o, mu, nu, par, i, L.g.L[3], multiply);
     *e += (double)sqnorm_ah(F);
     if (p & 1) {
       const double t = (double)re_tr_ah(prev, F);

@@ -13,6 +13,12 @@
 // with Ad(U) M = U^dag M U.  Each plaquette is multiplied out once (three products) instead of
 // seven times for the flow and sixteen for the clover, and a transport of eight reals costs
 // about as much as one product.
+//
+// The conjugated loop ends in U_nu(x-nu)^dag U_nu(x-nu) where the staple and the leaf do not, so this
+// holds for unitary links only.  12-real storage keeps two rows and takes the links as SU(3)
+// everywhere.  18-real storage holds whatever was written to it (links from a single-precision
+// file, say, unitary to 1e-7), so there the loops kernel also tests every link (off_unitary), and a
+// loop is moved along a link that fails by multiplying out the product that it stands for (leaf_*).
 #pragma once
 #include <type_traits>
 
@@ -32,11 +38,12 @@ struct Loops {
   static constexpr int NC = AlgStore<S>::NC;
   V* p;
   S* tr;
+  uint8_t* off;
   uint32_t stride, half;
   int slices;
   bool full;
   __device__ __forceinline__ Loops(const LoopDev& k, const Geom& g)
-      : p(reinterpret_cast<V*>(k.p)), tr(reinterpret_cast<S*>(k.tr)), stride(k.stride),
+      : p(reinterpret_cast<V*>(k.p)), tr(reinterpret_cast<S*>(k.tr)), off(k.off), stride(k.stride),
         half((uint32_t)g.str[3] >> 1), slices(k.slices), full(k.slices >= g.L[3]) {}
   // place of checkerboard site i of time t, read as slice tv
   __device__ __forceinline__ uint32_t at(uint32_t i, int t, int tv) const {
@@ -76,7 +83,39 @@ struct Loops {
   __device__ __forceinline__ void store_tr(int plane, int par, uint32_t j, R v) const {
     tr[(size_t)(plane * 2 + par) * stride + j] = S(v);
   }
+  __device__ __forceinline__ bool load_off(int mu, int par, uint32_t j) const {
+    return __ldg(&off[(size_t)(mu * 2 + par) * stride + j]) != 0;
+  }
+  __device__ __forceinline__ void store_off(int mu, int par, uint32_t j, bool v) const {
+    off[(size_t)(mu * 2 + par) * stride + j] = v ? 1 : 0;
+  }
 };
+
+// Whether |U U^dag - 1| is above 2^-40 (FP32: 2^-20) in the Frobenius norm, or not a number; the
+// relative error of a loop moved along U is at most about that.  Measured on 16^4, the largest of all
+// links: FP64 after 10000 sweeps 1.8e-13, after 1000 RK3 steps 4e-14; FP32 after an RK3 step (which
+// ends with re-orthonormalised links) 1.4e-7, after 10 sweeps 5e-6 and after 2000 3e-4, so that the
+// clover of FP32 18-real links is multiplied out behind sweeps.
+template <typename S, typename R>
+__device__ __forceinline__ bool off_unitary(const m3<R>& U) {
+  constexpr double BOUND = sizeof(S) == 8 ? 0x1p-80 : 0x1p-40;
+  R s = 0;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    R d = R(-1);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) d = fma(U.e[r][k].re, U.e[r][k].re, fma(U.e[r][k].im, U.e[r][k].im, d));
+    s = fma(d, d, s);
+#pragma unroll
+    for (int q = r + 1; q < 3; ++q) {
+      cx<R> o = mk<R>(R(0), R(0));
+#pragma unroll
+      for (int k = 0; k < 3; ++k) o = cfma_nc(U.e[r][k], U.e[q][k], o);
+      s = fma(R(2), fma(o.re, o.re, o.im * o.im), s);
+    }
+  }
+  return !(s <= R(BOUND));
+}
 
 // The leading link of a product: its stored rows (12-real), or all of it.
 template <typename F, typename R>
@@ -91,10 +130,9 @@ __device__ __forceinline__ m3<R> lead(const F& f, int mu, int par, uint32_t i) {
 // the three products from the stored rows of their first factors; row 2 of the second and of L
 // from the cross product (each is in SU(3)).
 template <typename F, typename R>
-__device__ __forceinline__ m3<R> plaquette_loop(const F& f, const m3<R>& Umu, int mu, int nu, int par, uint32_t i,
-                                                uint32_t ixmu, uint32_t ixnu) {
+__device__ __forceinline__ m3<R> plaquette_loop(const F& f, const m3<R>& Umu, const m3<R>& Unu, int mu, int nu,
+                                                int par, uint32_t ixmu, uint32_t ixnu) {
   const int opp = par ^ 1;
-  const m3<R> Unu = lead<F, R>(f, nu, par, i);
   if constexpr (F::NREAL == 12) {
     const m3<R> G = mul_nn_rows01(Umu, f.template load<R>(nu, opp, ixmu));
     m3<R> H = mul_nn_rows01(Unu, f.template load<R>(mu, opp, ixnu));
@@ -173,18 +211,71 @@ __device__ __forceinline__ alg8<R> transport(const m3<R>& U, const alg8<R>& K) {
   return r;
 }
 
+// a + sg b, sg = +-1
+template <typename R>
+__device__ __forceinline__ void add_alg(alg8<R>& a, const alg8<R>& b, R sg = R(1)) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) a.a[q] = fma(sg, b.a[q], a.a[q]);
+}
+
+// P_TA of the loop L_{mu nu}(y) (either order of mu and nu), begun at y+nu instead of y:
+// U_nu(y)^dag U_mu(y) U_nu(y+mu) U_mu(y+nu)^dag.  iy, iymu, iynu: y (parity py), y+mu, y+nu.
+template <typename F, typename R>
+__device__ __forceinline__ alg8<R> leaf_beside(const F& f, int mu, int nu, int py, uint32_t iy, uint32_t iymu,
+                                               uint32_t iynu) {
+  m3<R> M = mul_an(f.template load<R>(nu, py, iy), f.template load<R>(mu, py, iy));
+  M = mul_nn(M, f.template load<R>(nu, py ^ 1, iymu));
+  return proj_ta(mul_na(M, f.template load<R>(mu, py ^ 1, iynu)));
+}
+// The same begun at z+mu+nu: [U_nu(z) U_mu(z+nu)]^dag U_mu(z) U_nu(z+mu).
+template <typename F, typename R>
+__device__ __forceinline__ alg8<R> leaf_across(const F& f, int mu, int nu, int pz, uint32_t iz, uint32_t izmu,
+                                               uint32_t iznu) {
+  const m3<R> H = mul_nn(f.template load<R>(nu, pz, iz), f.template load<R>(mu, pz ^ 1, iznu));
+  const m3<R> G = mul_nn(f.template load<R>(mu, pz, iz), f.template load<R>(nu, pz ^ 1, izmu));
+  return proj_ta(mul_an(H, G));
+}
+// Out of line, so that the products cost the transports beside them no registers (the clover in FP32
+// has them in line: 380 us so, 312 in line on 20x24x28x36 with links that need them).
+template <typename F, typename R>
+__device__ __noinline__ alg8<R> leaf_beside_call(F f, int mu, int nu, int py, uint32_t iy, uint32_t iymu,
+                                                 uint32_t iynu) {
+  return leaf_beside<F, R>(f, mu, nu, py, iy, iymu, iynu);
+}
+template <typename F, typename R>
+__device__ __noinline__ alg8<R> leaf_across_call(F f, int mu, int nu, int pz, uint32_t iz, uint32_t izmu,
+                                                 uint32_t iznu) {
+  return leaf_across<F, R>(f, mu, nu, pz, iz, izmu, iznu);
+}
+
 // The loops below site x in direction nu, K_{mu nu}(x-nu) of the three mu != nu (mu ascending,
 // K_{nu mu} where nu < mu), moved to x: out[k] = Ad(U_nu(x-nu)) K.
 template <typename F, typename S, typename R>
 __device__ __forceinline__ void transported(const Geom& g, const F& f, const Loops<S>& K, const Coord& x, int nu,
                                             int par, alg8<R> (&out)[3]) {
   const int opp = par ^ 1, t = x.c[3], L = g.L[nu], d = g.str[nu];
-  const uint32_t iy = cb_index((uint32_t)((int32_t)x.s + (sel4(x.c, nu) == 0 ? (L - 1) * d : -d)));
+  const int32_t sy = (int32_t)x.s + (sel4(x.c, nu) == 0 ? (L - 1) * d : -d);
+  const uint32_t iy = cb_index((uint32_t)sy);
   const uint32_t jy = nu == 3 ? K.at(iy, t == 0 ? L - 1 : t - 1, t - 1) : K.at(iy, t, t);
   const int p0 = nu == 0 ? 0 : nu - 1, p1 = nu < 2 ? 3 * nu + (1 - nu) : nu + 1, p2 = nu < 2 ? 2 + 2 * nu : 5;
   const m3<R> U = f.template load<R>(nu, opp, iy);
   const alg8<R> k0 = K.template load<R>(p0, opp, jy), k1 = K.template load<R>(p1, opp, jy),
                 k2 = K.template load<R>(p2, opp, jy);
+  if constexpr (F::NREAL == 18) {
+    if (off_unitary<S>(U)) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int mu = k + (k >= nu);
+        const int32_t up = sel4(x.c, mu) + 1 == g.L[mu] ? (1 - g.L[mu]) * g.str[mu] : g.str[mu];
+        out[k] = leaf_beside_call<F, R>(f, mu, nu, opp, iy, cb_index((uint32_t)(sy + up)), cb_index(x.s));
+        if (mu > nu) {
+#pragma unroll
+          for (int a = 0; a < 8; ++a) out[k].a[a] = -out[k].a[a];
+        }
+      }
+      return;
+    }
+  }
   out[0] = transport(U, k0);
   out[1] = transport(U, k1);
   out[2] = transport(U, k2);
@@ -222,17 +313,12 @@ __device__ __forceinline__ R sqnorm_ah(const ah9<R>& A) {
   return fma(R(2), t, s);
 }
 
-// a + sg b, sg = +-1
-template <typename R>
-__device__ __forceinline__ void add_alg(alg8<R>& a, const alg8<R>& b, R sg = R(1)) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q) a.a[q] = fma(sg, b.a[q], a.a[q]);
-}
 // F_{mu nu}(x) = (C - C^dag) / 8 (observables_mpi.cpp:81-82), C the sum of the four leaves: a
-// quarter of the transported loops, their traces (invariant under transport) on the diagonal.
+// quarter of the transported loops, their traces (the same at every corner) on the diagonal.  multiply:
+// one of the three links that loops move along here is not unitary.
 template <typename F, typename S, typename R>
 __device__ __forceinline__ ah9<R> clover_plane(const F& f, const Loops<S>& K, const Coord& x, const NbOff& o, int mu,
-                                               int nu, int par, uint32_t i, int Lt) {
+                                               int nu, int par, uint32_t i, int Lt, bool multiply) {
   const int opp = par ^ 1, t = x.c[3], plane = plane_of(mu, nu);
   const int tm = t == 0 ? Lt - 1 : t - 1;
   const int32_t s = (int32_t)x.s, dmu = sel4(o.dn, mu), dnu = sel4(o.dn, nu);
@@ -240,10 +326,27 @@ __device__ __forceinline__ ah9<R> clover_plane(const F& f, const Loops<S>& K, co
   // only nu can be the time direction (mu < nu)
   const int tn = nu == 3 ? tm : t, vn = nu == 3 ? t - 1 : t;
   const uint32_t j0 = K.at(i, t, t), jmu = K.at(imu, t, t), jnu = K.at(inu, tn, vn), jmn = K.at(imn, tn, vn);
-  alg8<R> B = transport(f.template load<R>(nu, par, imn), K.template load<R>(plane, par, jmn));
-  add_alg(B, K.template load<R>(plane, opp, jmu));
-  alg8<R> A = transport(f.template load<R>(mu, opp, imu), B);
-  add_alg(A, transport(f.template load<R>(nu, opp, inu), K.template load<R>(plane, opp, jnu)));
+  alg8<R> A;
+  if (multiply) {
+    if constexpr (F::NREAL == 18) {
+      const int32_t umu = sel4(o.up, mu), unu = sel4(o.up, nu);
+      const uint32_t iun = cb_index((uint32_t)(s + dmu + unu)), ium = cb_index((uint32_t)(s + dnu + umu));
+      if constexpr (is_fp32<R>::value) {
+        A = leaf_across<F, R>(f, mu, nu, par, imn, inu, imu);
+        add_alg(A, leaf_beside<F, R>(f, nu, mu, opp, imu, iun, i), R(-1));
+        add_alg(A, leaf_beside<F, R>(f, mu, nu, opp, inu, ium, i));
+      } else {
+        A = leaf_across_call<F, R>(f, mu, nu, par, imn, inu, imu);
+        add_alg(A, leaf_beside_call<F, R>(f, nu, mu, opp, imu, iun, i), R(-1));
+        add_alg(A, leaf_beside_call<F, R>(f, mu, nu, opp, inu, ium, i));
+      }
+    }
+  } else {
+    alg8<R> B = transport(f.template load<R>(nu, par, imn), K.template load<R>(plane, par, jmn));
+    add_alg(B, K.template load<R>(plane, opp, jmu));
+    A = transport(f.template load<R>(mu, opp, imu), B);
+    add_alg(A, transport(f.template load<R>(nu, opp, inu), K.template load<R>(plane, opp, jnu)));
+  }
   add_alg(A, K.template load<R>(plane, par, j0));
   const R tr = (K.template load_tr<R>(plane, par, j0) + K.template load_tr<R>(plane, par, jmn)) +
                (K.template load_tr<R>(plane, opp, jmu) + K.template load_tr<R>(plane, opp, jnu));

@@ -153,7 +153,9 @@ int qcb_translate(qcb_lattice* lat, const int shift[4]);
  * sum_{x, mu<nu} Re tr P_{mu nu}(x) / 3, divided by 6V.  FP64 accumulation. */
 int qcb_plaquette(qcb_lattice* lat, double* out);
 /* topo_q_e_clover_global (observables_mpi.cpp:61-150): clover charge Q (total) and energy
- * density E = (1/V) sum_x 1/2 sum_{mu<nu} |F_{mu nu}|^2 with F = (C - C^dagger)/8.  Uses the
+ * density E = (1/V) sum_x 1/2 sum_{mu<nu} |F_{mu nu}|^2 with F = (C - C^dagger)/8.
+ * C is that of the stored links: QCB_R18 links need not be unitary (those off by more than 1e-12 in
+ * FP64, 1e-6 in FP32, take longer), QCB_R12 links are taken as SU(3).  Uses the
  * context's plaquette-loop work space, as the Wilson flow does (allocated on first use, at most
  * 1 GiB or two time slices' loops, less when that much is not free). */
 int qcb_topo_qe(qcb_lattice* lat, double* q, double* e);
@@ -181,7 +183,8 @@ int qcb_plaquette_noalloc(const void* links, const int dims[4], int precision, i
  * mpi::observables::topo_charge_flowed (observables_mpi.cpp:153-178) with
  * GradientFlow::rk3_step (src/flow/gradient_flow.cpp:15-128): on a copy of the links,
  * for s < n_steps_gf: record (t, Q, E) into tQE[3s..3s+2], then n_rk_steps RK3 steps of
- * size eps.  The lattice itself is left unchanged.  tQE holds 3*n_steps_gf doubles. */
+ * size eps.  The lattice itself is left unchanged.  tQE holds 3*n_steps_gf doubles.  Links that are
+ * not unitary are taken as in qcb_topo_qe. */
 int qcb_flow_measure(qcb_lattice* lat, double eps, int n_steps_gf, int n_rk_steps,
                      double* tQE);
 /* n RK3 steps of size eps applied to the lattice in place (no measurement). */
