@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "counter.h"
+
 namespace qcb {
 
 constexpr uint64_t WAIT_NS = 2000000000ull;  // 2 s per wait
@@ -55,13 +57,13 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-// One thread waits until *p >= target.  Returns false on abort or timeout.
+// One thread waits until the counter *p has come to target (counter_reached).  Returns false on abort or timeout.
 __device__ __forceinline__ bool wait_geq(const uint32_t* p, uint32_t target, uint32_t* status,
                                          uint64_t limit_ns = WAIT_NS) {
-  if (ld_acquire_u32(p) >= target) return true;
+  if (counter_reached(ld_acquire_u32(p), target)) return true;
   const uint64_t t0 = global_ns();
   for (uint64_t it = 0;; ++it) {
-    if (ld_acquire_u32(p) >= target) return true;
+    if (counter_reached(ld_acquire_u32(p), target)) return true;
     if (ld_acquire_u32(&status[2])) return false;
     if (global_ns() - t0 > limit_ns || it > WAIT_MAX_ITERS) {
       atomicAdd(&status[1], 1u);
