@@ -31,6 +31,7 @@ struct qcb_batch {
   std::vector<uint32_t> hb_tile, flow_tile;
   BatchLat* d_desc = nullptr;  // n, of the lattices' links
   BatchLat* h_desc = nullptr;  // pinned mirror
+  cudaEvent_t uploaded = nullptr;  // behind the latest copy from h_desc
   uint32_t* d_prefix = nullptr;  // hb (n+1) | plaquette (n+1)
   std::vector<uint32_t> h_prefix;
   uint32_t per_hb = 0, nred = 0;
@@ -101,9 +102,23 @@ void pass_groups(const std::vector<qcb_lattice*>& lats, uint64_t* groups, uint64
   }
 }
 
+// Copies the descriptors to the device, on the stream; the next change of the mirror waits for the copy
+// (open_desc), which may be queued behind earlier launches.
+int upload_desc(qcb_batch* b) {
+  BCU(cudaMemcpyAsync(b->d_desc, b->h_desc, (size_t)b->n * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream),
+      "descriptor upload");
+  BCU(cudaEventRecord(b->uploaded, b->ctx->stream), "event");
+  return QCB_OK;
+}
+int open_desc(qcb_batch* b) {
+  BCU(cudaEventSynchronize(b->uploaded), "descriptor upload");
+  return QCB_OK;
+}
+
 // Rebuild descriptors and prefix sums from the lattices and tiles; upload them.
 int upload_layout(qcb_batch* b) {
   const int n = b->n;
+  BTRY(open_desc(b));
   b->h_prefix.assign(2 * (n + 1), 0);
   uint32_t* ph = &b->h_prefix[0];
   uint32_t* pr = &b->h_prefix[n + 1];
@@ -129,8 +144,7 @@ int upload_layout(qcb_batch* b) {
   BCU(cudaMemcpyAsync(b->d_prefix, b->h_prefix.data(), b->h_prefix.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
                       b->ctx->stream),
       "prefix upload");
-  BCU(cudaMemcpyAsync(b->d_desc, b->h_desc, (size_t)n * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream),
-      "descriptor upload");
+  BTRY(upload_desc(b));
   BCU(cudaStreamSynchronize(b->ctx->stream), "sync");
   drop_flow(b);
   return QCB_OK;
@@ -138,17 +152,17 @@ int upload_layout(qcb_batch* b) {
 
 // Heatbath parameters go into the descriptors (host mirror + async upload).
 int set_hb_params(qcb_batch* b, const double* betas, const uint64_t* seeds, const uint64_t* sweep_offsets) {
-  for (int l = 0; l < b->n; ++l) {
+  for (int l = 0; l < b->n; ++l)
     if (!(betas[l] > 0.0)) return bfail(QCB_ERR_INVALID, "beta must be positive");
+  BTRY(open_desc(b));
+  for (int l = 0; l < b->n; ++l) {
     BatchLat& d = b->h_desc[l];
     d.beta = betas[l];
     d.k0 = (uint32_t)seeds[l];
     d.k1 = (uint32_t)(seeds[l] >> 32);
     d.sweep0 = (uint32_t)sweep_offsets[l];
   }
-  BCU(cudaMemcpyAsync(b->d_desc, b->h_desc, (size_t)b->n * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream),
-      "descriptor upload");
-  return QCB_OK;
+  return upload_desc(b);
 }
 
 // The lattices as items of a flow plan: on the links, or (copies) on fw0.
@@ -348,6 +362,7 @@ int qcb_batch_create(qcb_ctx* ctx, int n, qcb_lattice* const* lats, qcb_batch** 
   }
   if (cudaMalloc(&b->d_desc, (size_t)n * sizeof(BatchLat)) != cudaSuccess ||
       cudaMallocHost(&b->h_desc, (size_t)n * sizeof(BatchLat)) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming) != cudaSuccess ||
       cudaMalloc(&b->d_prefix, 2 * (size_t)(n + 1) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&b->d_done, (size_t)n * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&b->d_status, 4 * sizeof(uint32_t)) != cudaSuccess ||
@@ -382,6 +397,7 @@ void batch_free(qcb_batch* b) {
   cudaFree(b->loops.p);
   cudaFree(b->d_desc);
   cudaFreeHost(b->h_desc);
+  if (b->uploaded) cudaEventDestroy(b->uploaded);
   cudaFree(b->d_prefix);
   cudaFree(b->d_done);
   cudaFree(b->d_status);
