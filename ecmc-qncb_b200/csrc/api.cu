@@ -104,6 +104,19 @@ int qcb::ensure_flow_space(qcb_lattice* L) {
   return QCB_OK;
 }
 
+int qcb::reserve_loops(qcb_ctx* c, size_t want, size_t least) {
+  if (loops_covered(c->loops, want, least)) return QCB_OK;
+  // The full buffer at once where it is a sixteenth of the free memory or less: growing it for a
+  // larger lattice frees and allocates again, which took up to 0.6 s behind memory that the driver
+  // was still clearing.
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) == cudaSuccess && free / 16 >= LOOPS_MAX_BYTES)
+    want = std::max(want, LOOPS_MAX_BYTES);
+  if (loops_reserve(&c->loops, want, least) != cudaSuccess)
+    return fail(QCB_ERR_NOMEM, "cannot allocate the plaquette-loop work space");
+  return QCB_OK;
+}
+
 namespace {
 LatDev with_links(const LatDev& d, void* p) {
   LatDev r = d;
@@ -111,33 +124,34 @@ LatDev with_links(const LatDev& d, void* p) {
   return r;
 }
 
-// Device buffer of at least `need` doubles for the partial sums of fused measurements.
-int ensure_meas(qcb_lattice* L, size_t need) {
-  if (L->meas_n >= need) return QCB_OK;
-  cudaFree(L->meas);
-  L->meas = nullptr;
-  L->meas_n = 0;
-  if (cudaMalloc(&L->meas, need * sizeof(double)) != cudaSuccess) {
+// The context's scratch with at least `need` doubles.  Replacing it is safe behind queued work: all
+// users are on the context's stream, and cudaFree waits for them.
+int ensure_scratch(qcb_ctx* c, size_t need) {
+  if (c->scratch_n >= need) return QCB_OK;
+  cudaFree(c->d_scratch);
+  c->d_scratch = nullptr;
+  c->scratch_n = 0;
+  if (cudaMalloc(&c->d_scratch, need * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     return fail(QCB_ERR_NOMEM, "cannot allocate the measurement partial sums");
   }
-  L->meas_n = need;
+  c->scratch_n = need;
   return QCB_OK;
+}
+
+// Doubles that the measurements of a lattice need at most: the plaquette, a measured sweep, or Q and E
+// (two sums for a block of 128 sites and one more a round, of which there are at most L_t).
+size_t scratch_for(const LatDev& d) {
+  const size_t qe = 2 * ((size_t)d.g.V / 128 + 1 + (size_t)d.g.L[3]) + 512, hb = (size_t)hb_meas_parts(d) + 256;
+  return std::max(4 * (size_t)reduce_blocks(), std::max(qe, hb));
 }
 
 // The rounds of lattice d (links a, other buffer b) through the context's loop buffer.
 int loop_rounds(qcb_lattice* L, const LatDev& d, void* b, double eps, std::vector<FlowLat>* rounds) {
   qcb_ctx* c = L->ctx;
   const Geom& g = d.g;
-  const size_t least = loops_bytes(g, d.prec, 2);
-  size_t want = loops_bytes(g, d.prec, g.L[3]), free = 0, total = 0;
-  // The full buffer at once where it is a sixteenth of the free memory or less: growing it for a
-  // larger lattice frees and allocates again, which took up to 0.6 s behind memory that the driver
-  // was still clearing.
-  if (want > c->loops.bytes && cudaMemGetInfo(&free, &total) == cudaSuccess && free / 16 >= LOOPS_MAX_BYTES)
-    want = std::max(want, LOOPS_MAX_BYTES);
-  if (loops_reserve(&c->loops, want, least) != cudaSuccess)
-    return fail(QCB_ERR_NOMEM, "cannot allocate the plaquette-loop work space");
+  const int r_ = reserve_loops(c, loops_bytes(g, d.prec, g.L[3]), loops_bytes(g, d.prec, 2));
+  if (r_ != QCB_OK) return r_;
   const LoopDev k = loops_view(c->loops, 0, g, d.prec, loops_slices(g, d.prec, c->loops.bytes));
   *rounds = flow_rounds(d, k);
   for (FlowLat& r : *rounds) {
@@ -191,9 +205,9 @@ int rk3(qcb_lattice* L, const std::vector<FlowLat>& rounds, int step, double* qe
   double* parts = nullptr;
   const uint32_t n = qe_dev ? qe_parts(rounds) : 0;
   if (qe_dev) {
-    const int r_ = ensure_meas(L, 2 * (size_t)n + 512);
+    const int r_ = ensure_scratch(c, 2 * (size_t)n + 512);
     if (r_ != QCB_OK) return r_;
-    parts = L->meas;
+    parts = c->d_scratch;
   }
   int r_ = loop_pass(L, rounds, odd, 1, parts);
   if (r_ == QCB_OK) r_ = loop_pass(L, rounds, odd ^ 1, 2, nullptr);
@@ -211,10 +225,10 @@ int rk3(qcb_lattice* L, const std::vector<FlowLat>& rounds, int step, double* qe
 int qe_async(qcb_lattice* L, const std::vector<FlowLat>& rounds, int swap, double* dst, const StatusCopy& st) {
   qcb_ctx* c = L->ctx;
   const uint32_t n = qe_parts(rounds);
-  int r_ = ensure_meas(L, 2 * (size_t)n + 512);
-  if (r_ == QCB_OK) r_ = loop_pass(L, rounds, swap, 0, L->meas);
+  int r_ = ensure_scratch(c, 2 * (size_t)n + 512);
+  if (r_ == QCB_OK) r_ = loop_pass(L, rounds, swap, 0, c->d_scratch);
   if (r_ != QCB_OK) return r_;
-  CU(launch_qe_from_parts(L->meas, (int)n, L->meas + 2 * (size_t)n, dst, 1.0 / (double)L->dev.g.Vg, st, c->stream,
+  CU(launch_qe_from_parts(c->d_scratch, (int)n, c->d_scratch + 2 * (size_t)n, dst, 1.0 / (double)L->dev.g.Vg, st, c->stream,
                           &c->launches),
      "Q/E sums");
   return QCB_OK;
@@ -270,7 +284,7 @@ int qcb_ctx_create(int device, unsigned flags, qcb_ctx** out) {
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_status, 4 * sizeof(uint32_t)) != cudaSuccess ||
       cudaMallocHost(&c->h_status, 4 * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&c->d_scratch, 4 * (size_t)reduce_blocks() * sizeof(double)) != cudaSuccess ||
+      ensure_scratch(c, 4 * (size_t)reduce_blocks()) != QCB_OK ||
       cudaMalloc(&c->d_out, 64 * sizeof(double)) != cudaSuccess ||
       cudaMallocHost(&c->h_out, 64 * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
@@ -397,6 +411,7 @@ int qcb_lattice_create(qcb_ctx* c, const int dims[4], int precision, int storage
     }
   }
   c->launches++;
+  ensure_scratch(c, scratch_for(L->dev));  // the measurement that needs it tries again
   c->refs++;  // under the context lock
   *out = L;
   return QCB_OK;
@@ -440,6 +455,7 @@ int qcb_lattice_create_slab(qcb_ctx* c, const int global_dims[4], int t0, int t_
     }
   }
   c->launches++;
+  ensure_scratch(c, scratch_for(L->dev));
   c->refs++;
   *out = L;
   return QCB_OK;
@@ -456,7 +472,6 @@ int qcb_lattice_destroy(qcb_lattice* L) {
     cudaFree(L->fw[0]);
     cudaFree(L->fw[1]);
     cudaFree(L->fz);
-    cudaFree(L->meas);
     cudaGetLastError();
   }
   delete L;
@@ -784,7 +799,7 @@ int qcb_heatbath_plaquette(qcb_lattice* L, double beta, int n_sweeps, int n_hits
     c->launches += 2;
   } else {
     const int np = hb_meas_parts(L->dev);
-    TRY(ensure_meas(L, (size_t)np + 256));
+    TRY(ensure_scratch(c, (size_t)np + 256));
     for (int s = 0; s < n_sweeps; ++s) {
       const uint32_t sweep = (uint32_t)(sweep_offset + (uint64_t)s);
       const bool last = s == n_sweeps - 1;
@@ -795,10 +810,10 @@ int qcb_heatbath_plaquette(qcb_lattice* L, double beta, int n_sweeps, int n_hits
           c->launches++;
         }
       if (last)
-        CU(launch_hb_meas(L->dev, beta, seed, sweep, n_hits, c->d_status, L->meas, c->stream, c->block, &c->launches),
+        CU(launch_hb_meas(L->dev, beta, seed, sweep, n_hits, c->d_status, c->d_scratch, c->stream, c->block, &c->launches),
            "measuring heatbath passes");
     }
-    CU(launch_sum_parts(L->meas, np, L->meas + np, c->h_out, {c->d_status, c->h_status}, c->stream, &c->launches),
+    CU(launch_sum_parts(c->d_scratch, np, c->d_scratch + np, c->h_out, {c->d_status, c->h_status}, c->stream, &c->launches),
        "plaquette sum");
   }
   TRY(wait_status(c));

@@ -35,10 +35,11 @@ struct qcb_batch {
   uint32_t* d_prefix = nullptr;  // hb (n+1) | plaquette (n+1)
   std::vector<uint32_t> h_prefix;
   uint32_t per_hb = 0, nred = 0;
-  // Flow and clover (made on first use): on the links with the copy fw0 as the other buffer,
-  // and on copies (fw0 with fw1).  The plans differ in their descriptors only.
-  LoopBuf loops;
+  // Flow and clover: on the links with the copy fw0 as the other buffer, and on copies (fw0 with fw1).
+  // The plans differ in their descriptors only.  They point into the context's loop buffer of
+  // generation loops_gen, and are remade when that has been replaced.
   bool have_flow = false;
+  uint64_t loops_gen = 0;
   FlowPlan flow[2];
   FlowLat* d_flow[2] = {nullptr, nullptr};
   uint32_t* d_flow_prefix = nullptr;  // the plan's prefix, then its qe_prefix
@@ -115,7 +116,9 @@ int open_desc(qcb_batch* b) {
   return QCB_OK;
 }
 
-// Rebuild descriptors and prefix sums from the lattices and tiles; upload them.
+int ensure_flow_plan(qcb_batch* b);
+
+// Rebuild descriptors and prefix sums from the lattices and tiles, upload them, and make the flow's plans.
 int upload_layout(qcb_batch* b) {
   const int n = b->n;
   BTRY(open_desc(b));
@@ -147,6 +150,7 @@ int upload_layout(qcb_batch* b) {
   BTRY(upload_desc(b));
   BCU(cudaStreamSynchronize(b->ctx->stream), "sync");
   drop_flow(b);
+  if (ensure_flow_plan(b) != QCB_OK) drop_flow(b);  // the call that needs it tries again
   return QCB_OK;
 }
 
@@ -186,15 +190,18 @@ std::vector<FlowItem> flow_items(const std::vector<qcb_lattice*>& lats, const st
   return items;
 }
 
-// Loop buffer, plans and their device arrays, made on first use.
+// Plans and their device arrays on the context's loop buffer, made at the batch's creation and again
+// when the tiles or the buffer have changed.
 int ensure_flow_plan(qcb_batch* b) {
-  if (b->have_flow) return QCB_OK;
   size_t want = 0, least = 0;
   flow_plan_bytes(flow_items(b->lats, b->flow_tile, 0), &want, &least);
-  if (loops_reserve(&b->loops, want, least) != cudaSuccess)
-    return bfail(QCB_ERR_NOMEM, "cannot allocate the batch's plaquette-loop work space");
+  BTRY(reserve_loops(b->ctx, want, least));
+  const LoopBuf& loops = b->ctx->loops;
+  if (b->have_flow && b->loops_gen == loops.gen) return QCB_OK;
+  drop_flow(b);
+  b->loops_gen = loops.gen;
   for (int k = 0; k < 2; ++k) {
-    b->flow[k] = flow_plan(flow_items(b->lats, b->flow_tile, k), b->loops);
+    b->flow[k] = flow_plan(flow_items(b->lats, b->flow_tile, k), loops);
     BCU(cudaMalloc(&b->d_flow[k], b->flow[k].lats.size() * sizeof(FlowLat)), "flow descriptors");
   }
   std::vector<uint32_t> pre = b->flow[0].prefix;
@@ -394,7 +401,6 @@ int qcb_batch_destroy(qcb_batch* b) {
 namespace {
 void batch_free(qcb_batch* b) {
   drop_flow(b);
-  cudaFree(b->loops.p);
   cudaFree(b->d_desc);
   cudaFreeHost(b->h_desc);
   if (b->uploaded) cudaEventDestroy(b->uploaded);
@@ -694,7 +700,7 @@ extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
             items[j].b = lats[j]->fw[0];
             items[j].eps = 0.02;
           }
-          fp = flow_plan(items, b->loops);
+          fp = flow_plan(items, b->ctx->loops);
           BCU(cudaMemcpyAsync(d_flow, fp.lats.data(), fp.lats.size() * sizeof(FlowLat), cudaMemcpyHostToDevice,
                               b->ctx->stream),
               "H2D");

@@ -13,13 +13,16 @@ struct qcb_ctx {
   int block = 0;
   uint32_t* d_status = nullptr;  // [0] KP cap hits
   uint32_t* h_status = nullptr;  // pinned mirror
-  double* d_scratch = nullptr;   // reduction partials
+  // Partial sums of the reductions.  It grows with the largest lattice (ensure_scratch, at its creation),
+  // so the first measurement of a lattice does not allocate.
+  double* d_scratch = nullptr;
+  size_t scratch_n = 0;
   double* d_out = nullptr;       // small results
   double* h_out = nullptr;       // pinned mirror
   double* d_stage[2] = {nullptr, nullptr};
   size_t stage_bytes = 0;
   double* h_stage = nullptr;  // pinned, for file I/O
-  // Plaquette loops of the flow and the clover, shared by the context's lattices (its calls
+  // Plaquette loops of the flow and the clover, shared by the context's lattices and batches (its calls
   // run in stream order); allocated on first use, at most LOOPS_MAX_BYTES or two time slices.
   qcb::LoopBuf loops;
   uint64_t launches = 0;
@@ -38,9 +41,6 @@ struct qcb_lattice {
   // Wilson-flow work space, allocated on first use: two link buffers + accumulator.
   void* fw[2] = {nullptr, nullptr};
   void* fz = nullptr;
-  // Partial sums of the measuring heatbath passes, allocated on first use.
-  double* meas = nullptr;
-  size_t meas_n = 0;
   // Slab of a larger lattice (qcb_lattice_create_slab): global extents and the global time
   // of local time 1; slab_tl == 0 for a whole lattice.
   int gdims[4] = {0, 0, 0, 0};
@@ -53,6 +53,8 @@ void ctx_ref(qcb_ctx* c);
 void ctx_unref(qcb_ctx* c);
 // Allocates a lattice's Wilson-flow work space (two link buffers + accumulator) once.
 int ensure_flow_space(qcb_lattice* L);
+// Makes the context's loop buffer answer a request (loops_reserve); QCB_ERR_NOMEM below `least`.
+int reserve_loops(qcb_ctx* c, size_t want, size_t least);
 // Reads and clears the context's device status words (after synchronising its stream).
 int check_status(qcb_ctx* c);
 int wait_status(qcb_ctx* c);

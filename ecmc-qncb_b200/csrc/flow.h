@@ -45,11 +45,12 @@ struct FlowLat {
   int nsteps;     // RK3 steps the lattice takes part in
 };
 
-// Owner of a loop buffer (a context, a batch, a server).
+// A loop buffer (of a context, used by its lattices and batches, or of a server).
 struct LoopBuf {
   void* p = nullptr;
   size_t bytes = 0;
   size_t wanted = 0;  // the largest size asked for (not tried again once it did not fit)
+  uint64_t gen = 0;   // goes up when p is replaced: plans made on the old one are then remade
 };
 
 // Largest loop buffer.  1 GiB holds a whole 32^4 (FP64 453 MB) and more than three slices of
@@ -61,6 +62,9 @@ constexpr size_t LOOPS_MAX_BYTES = 1ull << 30;
 size_t loops_bytes(const Geom& g, int prec, int slices);
 // Slices of g that fit into `bytes` (at most L_t; 0 if fewer than the two a round needs).
 int loops_slices(const Geom& g, int prec, size_t bytes);
+// The size that loops_reserve aims at for a request, and whether buf answers it as it is.
+size_t loops_target(size_t want, size_t least);
+bool loops_covered(const LoopBuf& buf, size_t want, size_t least);
 // Grows buf to want bytes (at most LOOPS_MAX_BYTES), or to the most that can be allocated, but
 // no less than least.  The caller has no work in flight that uses the buffer it replaces, or
 // lets cudaFree wait for it.

@@ -23,13 +23,21 @@ int loops_slices(const Geom& g, int prec, size_t bytes) {
   while (n >= 2 && loops_bytes(g, prec, n) > bytes) --n;
   return n >= 2 ? n : 0;
 }
-cudaError_t loops_reserve(LoopBuf* buf, size_t want, size_t least) {
+size_t loops_target(size_t want, size_t least) {
   if (want > LOOPS_MAX_BYTES) want = LOOPS_MAX_BYTES;
-  if (want < least) want = least;
-  if (buf->bytes >= want || (buf->bytes >= least && buf->wanted >= want)) return cudaSuccess;
+  return want < least ? least : want;
+}
+bool loops_covered(const LoopBuf& buf, size_t want, size_t least) {
+  want = loops_target(want, least);
+  return buf.bytes >= want || (buf.bytes >= least && buf.wanted >= want);
+}
+cudaError_t loops_reserve(LoopBuf* buf, size_t want, size_t least) {
+  if (loops_covered(*buf, want, least)) return cudaSuccess;
+  want = loops_target(want, least);
   cudaFree(buf->p);
   buf->p = nullptr;
   buf->bytes = 0;
+  buf->gen++;
   buf->wanted = want;
   for (size_t n = want;; n = n / 2 > least ? n / 2 : least) {
     if (cudaMalloc(&buf->p, n) == cudaSuccess) {

@@ -196,8 +196,8 @@ int qcb_flow_steps(qcb_lattice* lat, double eps, int n);
  * sizes (same context, precision and storage).  The heatbath is one persistent cooperative
  * launch: work items (lattice, level, tile of sites) run level-major, each lattice's levels
  * in order, different lattices overlapping.  The flow and the clover run stage by stage, each
- * launch covering the lattices whose plaquette loops fit into the batch's loop buffer together
- * (at most 1 GiB, or two time slices of the largest lattice; allocated on first use).  Every
+ * launch covering the lattices whose plaquette loops fit into the loop buffer together
+ * (at most 1 GiB, or two time slices of the largest lattice; the buffer is the context's).  Every
  * result is bit-identical to running the lattice alone through qcb_heatbath / qcb_flow_steps
  * with the same seed and sweep counter.
  * The batch borrows the lattices: they must outlive it. */
