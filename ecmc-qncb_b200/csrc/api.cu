@@ -372,6 +372,15 @@ int qcb_ctx_set_block(qcb_ctx* c, int threads) {
   return QCB_OK;
 }
 
+int qcb_ctx_set_loop_bytes(qcb_ctx* c, size_t bytes) {
+  CHECK_CTX(c);
+  LOCK(c);
+  TRY(set_device(c));
+  c->loops.limit = bytes;
+  loops_drop(&c->loops, [](void* p) { cudaFree(p); });
+  return QCB_OK;
+}
+
 int qcb_ctx_stream(qcb_ctx* c, void** stream) {
   CHECK_CTX(c);
   if (!stream) return fail(QCB_ERR_INVALID, "null stream pointer");

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "loop_buf.h"
 
 namespace qcb {
 
@@ -45,29 +46,12 @@ struct FlowLat {
   int nsteps;     // RK3 steps the lattice takes part in
 };
 
-// A loop buffer (of a context, used by its lattices and batches, or of a server).
-struct LoopBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  size_t wanted = 0;  // the largest size asked for (not tried again once it did not fit)
-  uint64_t gen = 0;   // goes up when p is replaced: plans made on the old one are then remade
-};
-
-// Largest loop buffer.  1 GiB holds a whole 32^4 (FP64 453 MB) and more than three slices of
-// any lattice below 2^30 sites with L_t >= 12; 64^4 runs in rounds of 18 slices in FP32 and 8
-// in FP64, each of over a million sites, so that a round's launches fill the device.
-constexpr size_t LOOPS_MAX_BYTES = 1ull << 30;
-
 // Bytes of the loops of `slices` time slices.
 size_t loops_bytes(const Geom& g, int prec, int slices);
 // Slices of g that fit into `bytes` (at most L_t; 0 if fewer than the two a round needs).
 int loops_slices(const Geom& g, int prec, size_t bytes);
-// The size that loops_reserve aims at for a request, and whether buf answers it as it is.
-size_t loops_target(size_t want, size_t least);
-bool loops_covered(const LoopBuf& buf, size_t want, size_t least);
-// Grows buf to want bytes (at most LOOPS_MAX_BYTES), or to the most that can be allocated, but
-// no less than least.  The caller has no work in flight that uses the buffer it replaces, or
-// lets cudaFree wait for it.
+// Grows buf on the device (loops_grow); cudaErrorMemoryAllocation when it holds less than least.
+// The caller has no work in flight that uses the buffer it replaces, or lets cudaFree wait for it.
 cudaError_t loops_reserve(LoopBuf* buf, size_t want, size_t least);
 // The buffer from offset `off` as lattice g's loops (slices as loops_slices gives them).
 LoopDev loops_view(const LoopBuf& buf, size_t off, const Geom& g, int prec, int slices);

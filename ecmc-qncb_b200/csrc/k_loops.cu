@@ -3,6 +3,8 @@
 // References: clover_site, local_q_e_clover and topo_q_e_clover(_global)
 // (src/observables/observables_mpi.cpp:61-150) for Q and E; the loops also carry the force of
 // the Wilson flow (loops.cuh).
+#include <algorithm>
+
 #include "flow_launch.cuh"
 #include "reduce.cuh"
 
@@ -12,42 +14,24 @@ namespace qcb {
 static size_t loops_stride(const Geom& g, int slices) {
   return ((size_t)slices * (size_t)(g.str[3] / 2) + 63) / 64 * 64;
 }
-size_t loops_bytes(const Geom& g, int prec, int slices) {
-  return loops_stride(g, slices) * ((size_t)(6 * 2 * 9) * (prec == QCB_PREC_FP64 ? 8 : 4) + 4 * 2);
-}
+static size_t index_bytes(int prec) { return (size_t)(6 * 2 * 9) * (prec == QCB_PREC_FP64 ? 8 : 4) + 4 * 2; }
+size_t loops_bytes(const Geom& g, int prec, int slices) { return loops_stride(g, slices) * index_bytes(prec); }
 int loops_slices(const Geom& g, int prec, size_t bytes) {
   if (loops_bytes(g, prec, g.L[3]) <= bytes) return g.L[3];
-  const size_t one = loops_bytes(g, prec, 1);
-  int n = (int)(bytes / one);
-  if (n > g.L[3] - 1) n = g.L[3] - 1;
+  // the padding of the stride is that of all slices together, so the estimate leaves it out
+  const size_t most = bytes / ((size_t)(g.str[3] / 2) * index_bytes(prec));
+  int n = (int)std::min(most, (size_t)(g.L[3] - 1));
   while (n >= 2 && loops_bytes(g, prec, n) > bytes) --n;
   return n >= 2 ? n : 0;
 }
-size_t loops_target(size_t want, size_t least) {
-  if (want > LOOPS_MAX_BYTES) want = LOOPS_MAX_BYTES;
-  return want < least ? least : want;
-}
-bool loops_covered(const LoopBuf& buf, size_t want, size_t least) {
-  want = loops_target(want, least);
-  return buf.bytes >= want || (buf.bytes >= least && buf.wanted >= want);
-}
 cudaError_t loops_reserve(LoopBuf* buf, size_t want, size_t least) {
-  if (loops_covered(*buf, want, least)) return cudaSuccess;
-  want = loops_target(want, least);
-  cudaFree(buf->p);
-  buf->p = nullptr;
-  buf->bytes = 0;
-  buf->gen++;
-  buf->wanted = want;
-  for (size_t n = want;; n = n / 2 > least ? n / 2 : least) {
-    if (cudaMalloc(&buf->p, n) == cudaSuccess) {
-      buf->bytes = n;
-      return cudaSuccess;
-    }
+  auto alloc = [](size_t n) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, n) == cudaSuccess) return p;
     cudaGetLastError();
-    buf->p = nullptr;
-    if (n <= least) return cudaErrorMemoryAllocation;
-  }
+    return (void*)nullptr;
+  };
+  return loops_grow(buf, want, least, alloc, [](void* p) { cudaFree(p); }) ? cudaSuccess : cudaErrorMemoryAllocation;
 }
 LoopDev loops_view(const LoopBuf& buf, size_t off, const Geom& g, int prec, int slices) {
   const size_t es = prec == QCB_PREC_FP64 ? 8 : 4, st = loops_stride(g, slices);

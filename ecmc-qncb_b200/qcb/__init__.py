@@ -70,6 +70,10 @@ class Context:
     def set_block(self, threads: int) -> None:
         check(lib().qcb_ctx_set_block(self.h, threads))
 
+    def set_loop_bytes(self, limit: int | None = None) -> None:
+        """Most device memory of the flow's and the clover's plaquette loops (None: the default)."""
+        check(lib().qcb_ctx_set_loop_bytes(self.h, C.c_size_t(-1).value if limit is None else int(limit)))
+
     @property
     def stream(self) -> int:
         s = C.c_void_p()

@@ -115,6 +115,7 @@ SIGNATURES = {
     "qcb_ctx_sync": (C.c_int, [_vp]),
     "qcb_ctx_launch_count": (C.c_int, [_vp, C.POINTER(C.c_uint64)]),
     "qcb_ctx_set_block": (C.c_int, [_vp, C.c_int]),
+    "qcb_ctx_set_loop_bytes": (C.c_int, [_vp, C.c_size_t]),
     "qcb_ctx_stream": (C.c_int, [_vp, C.POINTER(C.c_void_p)]),
     "qcb_lattice_create": (C.c_int, [_vp, _ip, C.c_int, C.c_int, C.POINTER(C.c_void_p)]),
     "qcb_lattice_destroy": (C.c_int, [_vp]),

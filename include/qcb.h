@@ -68,6 +68,12 @@ int qcb_ctx_launch_count(qcb_ctx* ctx, uint64_t* count);
 /* Thread-block size used by subsequent launches of the per-link/per-site kernels
  * (0 = built-in default).  Results do not depend on it. */
 int qcb_ctx_set_block(qcb_ctx* ctx, int threads);
+/* Most device memory, in bytes, of the plaquette-loop work space that the Wilson flow and Q/E use: one
+ * buffer for the context's lattices and batches, and one for each server created after this call
+ * (SIZE_MAX, the default: up to 1 GiB, or two time slices of a larger lattice).  A lattice whose loops do
+ * not fit is worked through in rounds of time slices; its results do not depend on that but for the
+ * order of the sums of Q and E.  It takes at least two time slices.  The present buffer is released. */
+int qcb_ctx_set_loop_bytes(qcb_ctx* ctx, size_t bytes);
 /* The cudaStream_t the context launches on (as void*). */
 int qcb_ctx_stream(qcb_ctx* ctx, void** stream);
 
