@@ -104,17 +104,15 @@ int qcb::ensure_flow_space(qcb_lattice* L) {
   return QCB_OK;
 }
 
-int qcb::reserve_loops(qcb_ctx* c, size_t want, size_t least) {
-  if (loops_covered(c->loops, want, least)) return QCB_OK;
+void qcb::reserve_loops(qcb_ctx* c, size_t want, size_t least) {
+  if (loops_covered(c->loops, want, least)) return;
   // The full buffer at once where it is a sixteenth of the free memory or less: growing it for a
   // larger lattice frees and allocates again, which took up to 0.6 s behind memory that the driver
   // was still clearing.
   size_t free = 0, total = 0;
   if (cudaMemGetInfo(&free, &total) == cudaSuccess && free / 16 >= LOOPS_MAX_BYTES)
     want = std::max(want, LOOPS_MAX_BYTES);
-  if (loops_reserve(&c->loops, want, least) != cudaSuccess)
-    return fail(QCB_ERR_NOMEM, "cannot allocate the plaquette-loop work space");
-  return QCB_OK;
+  loops_reserve(&c->loops, want, least);
 }
 
 namespace {
@@ -147,19 +145,18 @@ size_t scratch_for(const LatDev& d) {
 }
 
 // The rounds of lattice d (links a, other buffer b) through the context's loop buffer.
-int loop_rounds(qcb_lattice* L, const LatDev& d, void* b, double eps, std::vector<FlowLat>* rounds) {
+std::vector<FlowLat> loop_rounds(qcb_lattice* L, const LatDev& d, void* b, double eps) {
   qcb_ctx* c = L->ctx;
   const Geom& g = d.g;
-  const int r_ = reserve_loops(c, loops_bytes(g, d.prec, g.L[3]), loops_bytes(g, d.prec, 2));
-  if (r_ != QCB_OK) return r_;
+  reserve_loops(c, loops_bytes(g, d.prec, g.L[3]), loops_bytes(g, d.prec, 2));
   const LoopDev k = loops_view(c->loops, 0, g, d.prec, loops_slices(g, d.prec, c->loops.bytes));
-  *rounds = flow_rounds(d, k);
-  for (FlowLat& r : *rounds) {
+  std::vector<FlowLat> rounds = flow_rounds(d, k);
+  for (FlowLat& r : rounds) {
     r.b = b;
     r.acc = L->fz;
     r.eps = eps;
   }
-  return QCB_OK;
+  return rounds;
 }
 
 // The loops of every round of the links selected by swap, then (parts != nullptr) the clover
@@ -176,6 +173,18 @@ int loop_pass(qcb_lattice* L, const std::vector<FlowLat>& rounds, int swap, int 
   const uint32_t n = parts ? qe_parts(rounds) : 0;
   uint32_t first = 0;
   for (const FlowLat& r : rounds) {
+    if (!r.k.p) {
+      if (parts) {
+        CU(launch_clover(r, prec, nr, swap, parts, first, n, c->stream), "clover Q/E");
+        first += qe_blocks(r);
+        c->launches++;
+      }
+      if (stage) {
+        CU(launch_flow_links(r, prec, nr, stage, swap, c->stream), "flow stage");
+        c->launches++;
+      }
+      continue;
+    }
     FlowSet s;
     s.one = r;
     s.blocks = loops_blocks(r);
@@ -897,8 +906,7 @@ int qcb_topo_qe(qcb_lattice* L, double* q, double* e) {
   qcb_ctx* c = L->ctx;
   LOCK(c);
   TRY(set_device(c));
-  std::vector<FlowLat> rounds;
-  TRY(loop_rounds(L, L->dev, nullptr, 0.0, &rounds));
+  const std::vector<FlowLat> rounds = loop_rounds(L, L->dev, nullptr, 0.0);
   TRY(qe_async(L, rounds, 0, c->h_out, {c->d_status, c->h_status}));
   TRY(wait_status(c));
   *q = c->h_out[0];
@@ -919,7 +927,7 @@ int qcb_flow_measure(qcb_lattice* L, double eps, int n_steps_gf, int n_rk_steps,
   // gf.copy(field): the flow runs on a copy (observables_mpi.cpp:320).
   CU(cudaMemcpyAsync(L->fw[0], L->dev.links, L->bytes, cudaMemcpyDeviceToDevice, c->stream), "D2D copy");
   std::vector<FlowLat> rounds;
-  if (n_steps_gf > 0) TRY(loop_rounds(L, with_links(L->dev, L->fw[0]), L->fw[1], eps, &rounds));
+  if (n_steps_gf > 0) rounds = loop_rounds(L, with_links(L->dev, L->fw[0]), L->fw[1], eps);
   double t = 0.0;
   int step = 0;
   const int chunk = 32;  // (t, Q, E) records staged in d_out (64 doubles) between host reads
@@ -957,7 +965,7 @@ int qcb_flow_steps(qcb_lattice* L, double eps, int n) {
   // Each RK3 step ping-pongs between the primary buffer and fw[0]; the result is copied
   // back to the primary buffer when it ends up in fw[0].
   std::vector<FlowLat> rounds;
-  if (n > 0) TRY(loop_rounds(L, L->dev, L->fw[0], eps, &rounds));
+  if (n > 0) rounds = loop_rounds(L, L->dev, L->fw[0], eps);
   for (int r = 0; r < n; ++r) TRY(rk3(L, rounds, r, nullptr));
   if (n & 1)
     CU(cudaMemcpyAsync(L->dev.links, L->fw[0], L->bytes, cudaMemcpyDeviceToDevice, c->stream), "D2D copy");
@@ -990,8 +998,7 @@ int qcb_flow_stage(qcb_lattice* L, int stage, double eps, int step) {
   TRY(ensure_flow_space(L));
   // step s ping-pongs between the links (a) and the work buffer fw[0] (b) as qcb_flow_steps:
   // stage 1 a -> b, stage 2 b -> a, stage 3 a -> b, with a and b swapped for odd s
-  std::vector<FlowLat> rounds;
-  TRY(loop_rounds(L, L->dev, L->fw[0], eps, &rounds));
+  const std::vector<FlowLat> rounds = loop_rounds(L, L->dev, L->fw[0], eps);
   return loop_pass(L, rounds, (step & 1) ^ (stage == 2 ? 1 : 0), stage, nullptr);
 }
 

@@ -195,7 +195,7 @@ std::vector<FlowItem> flow_items(const std::vector<qcb_lattice*>& lats, const st
 int ensure_flow_plan(qcb_batch* b) {
   size_t want = 0, least = 0;
   flow_plan_bytes(flow_items(b->lats, b->flow_tile, 0), &want, &least);
-  BTRY(reserve_loops(b->ctx, want, least));
+  reserve_loops(b->ctx, want, least);
   const LoopBuf& loops = b->ctx->loops;
   if (b->have_flow && b->loops_gen == loops.gen) return QCB_OK;
   drop_flow(b);

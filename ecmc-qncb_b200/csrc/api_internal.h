@@ -53,8 +53,8 @@ void ctx_ref(qcb_ctx* c);
 void ctx_unref(qcb_ctx* c);
 // Allocates a lattice's Wilson-flow work space (two link buffers + accumulator) once.
 int ensure_flow_space(qcb_lattice* L);
-// Makes the context's loop buffer answer a request (loops_reserve); QCB_ERR_NOMEM below `least`.
-int reserve_loops(qcb_ctx* c, size_t want, size_t least);
+// Makes the context's loop buffer answer a request as far as the memory goes (loops_reserve).
+void reserve_loops(qcb_ctx* c, size_t want, size_t least);
 // Reads and clears the context's device status words (after synchronising its stream).
 int check_status(qcb_ctx* c);
 int wait_status(qcb_ctx* c);

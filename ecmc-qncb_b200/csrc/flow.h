@@ -8,7 +8,10 @@
 //
 // The loops live in a buffer of a bounded number of time slices (LoopBuf).  A lattice whose
 // loops do not fit is worked through in rounds of consecutive slices; the buffer then is a
-// ring in which the slice before a round's first stays from the round before.
+// ring in which the slice before a round's first stays from the round before.  Where not even two
+// slices fit (device memory is full, or the user's limit is smaller), the round has no loops
+// (k.p == nullptr): staples and leaves are multiplied out link by link (launch_flow_links,
+// launch_clover), which takes no work space.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -56,7 +59,7 @@ cudaError_t loops_reserve(LoopBuf* buf, size_t want, size_t least);
 // The buffer from offset `off` as lattice g's loops (slices as loops_slices gives them).
 LoopDev loops_view(const LoopBuf& buf, size_t off, const Geom& g, int prec, int slices);
 
-// The rounds of lattice L with loops k (a, b, acc, eps, tile and nsteps are the caller's).
+// The rounds of lattice L with loops k, or one without loops (a, b, acc, eps, tile and nsteps are the caller's).
 std::vector<FlowLat> flow_rounds(const LatDev& L, const LoopDev& k);
 
 // Blocks of a round's three kernels.
@@ -82,6 +85,10 @@ cudaError_t launch_flow_update(const FlowSet& s, int prec, int nr, int stage, in
 // from loops computed with trace = true.
 cudaError_t launch_loops_qe(const FlowSet& s, int prec, int nr, int swap, double* parts, uint32_t first, uint32_t n,
                             cudaStream_t st);
+// The same for a round without loops, from the links alone.
+cudaError_t launch_flow_links(const FlowLat& r, int prec, int nr, int stage, int swap, cudaStream_t st);
+cudaError_t launch_clover(const FlowLat& r, int prec, int nr, int swap, double* parts, uint32_t first, uint32_t n,
+                          cudaStream_t st);
 
 // ---- many lattices ------------------------------------------------------------------------
 // One lattice of a plan: links (L.links = a), the other buffer b and the accumulator (flow
@@ -97,7 +104,7 @@ struct FlowItem {
 
 // Lattices worked through together: groups whose loops fit into the buffer at once, one after
 // another, each group's kernels covering all its lattices; a lattice whose loops do not fit is
-// a group of its own with several rounds.
+// a group of its own with several rounds, or one without loops.
 struct FlowPlan {
   struct Round {
     int first, n;            // lats[first .. first + n)

@@ -64,7 +64,7 @@ FlowPlan flow_plan(const std::vector<FlowItem>& items, const LoopBuf& buf) {
     }
     const int slices = loops_slices(it.L.g, it.L.prec, buf.bytes - used);
     const std::vector<FlowLat> rounds = flow_rounds(it.L, loops_view(buf, used, it.L.g, it.L.prec, slices));
-    if (rounds.size() == 1) {
+    if (rounds.size() == 1 && rounds[0].k.p) {
       add(it, rounds[0]);
       used += all;
       open = true;
@@ -106,6 +106,14 @@ cudaError_t run_flow_plan(const FlowPlan& p, const FlowLat* d_lats, const uint32
       for (int stage = 1; stage <= 3; ++stage) {
         const int swap = (odd ^ (step & 1)) ^ (stage == 2 ? 1 : 0);
         for (const FlowPlan::Round& rd : g) {
+          const FlowLat& only = p.lats[rd.first];
+          if (!only.k.p) {
+            if (step >= only.nsteps) continue;
+            const cudaError_t e = launch_flow_links(only, prec, nr, stage, swap, st);
+            if (e != cudaSuccess) return e;
+            ++*launches;
+            continue;
+          }
           cudaError_t e = launch_loops(set_of(rd, d_lats, d_prefix, 0, rd.loops), prec, nr, false, swap, step, st);
           if (e == cudaSuccess)
             e = launch_flow_update(set_of(rd, d_lats, d_prefix, 1, rd.update), prec, nr, stage, swap, step, st);
@@ -121,6 +129,12 @@ cudaError_t run_qe_plan(const FlowPlan& p, const FlowLat* d_lats, const uint32_t
   const uint32_t n = p.qe_prefix.back();
   for (const auto& g : p.groups)
     for (const FlowPlan::Round& rd : g) {
+      if (!p.lats[rd.first].k.p) {
+        const cudaError_t e = launch_clover(p.lats[rd.first], prec, nr, odd, parts, rd.qe_first, n, st);
+        if (e != cudaSuccess) return e;
+        ++*launches;
+        continue;
+      }
       cudaError_t e = launch_loops(set_of(rd, d_lats, d_prefix, 0, rd.loops), prec, nr, true, odd, 0, st);
       if (e == cudaSuccess)
         e = launch_loops_qe(set_of(rd, d_lats, d_prefix, 2, rd.qe), prec, nr, odd, parts, rd.qe_first, n, st);

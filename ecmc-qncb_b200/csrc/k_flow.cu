@@ -109,6 +109,56 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_FLOW_MINB32
   }
 }
 
+// The stage without loops: one thread per link, its staples multiplied out.
+template <typename S, int NR>
+__global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? 4 : 2)
+    k_flow_links(const __grid_constant__ FlowLat L, int swap, int stage) {
+  typedef arith_t<S> R;
+  typedef Links<S, NR> F;
+  pdl_wait();
+  const uint32_t half = (uint32_t)(L.g.str[3] >> 1), n = (uint32_t)(L.t1 - L.t0) * half,
+                 k = (blockIdx.x >> 1) * FLOW_THREADS + threadIdx.x;
+  if (k >= n) return;
+  const int par = (int)(blockIdx.x & 1), mu = (int)blockIdx.y;
+  const uint32_t i = (uint32_t)L.t0 * half + k;
+  const F src = flow_links<S, NR>(L, swap), dst = flow_links<S, NR>(L, swap ^ 1);
+  AlgField<S> acc;
+  acc.p = reinterpret_cast<typename AlgField<S>::V*>(L.acc);
+  acc.stride = L.g.stride;
+  const m3<R> A = staple_sum_rt<F, R>(L.g, src, cb_coord(L.g, par, i), mu, par, i);
+  const m3<R> U = src.template load<R>(mu, par, i);
+  alg8<R> Z = proj_ta(mul_nn(U, A)), Z0;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) Z.a[a] = -Z.a[a];
+  if (stage != 1) Z0 = acc.template load<R>(mu, par, i);
+  const R eps = R(S(L.eps));
+  alg8<R> X;
+  if (stage == 1)
+    X = flow_x<1, AlgField<S>, R>(acc, Z, Z0, eps, mu, par, i);
+  else if (stage == 2)
+    X = flow_x<2, AlgField<S>, R>(acc, Z, Z0, eps, mu, par, i);
+  else
+    X = flow_x<3, AlgField<S>, R>(acc, Z, Z0, eps, mu, par, i);
+  m3<R> Un = flow_product<F, R>(exp_su3(X), U);
+  flow_reunit<R>(Un, stage);
+  dst.template store<R>(mu, par, i, Un);
+}
+
+template <typename S, int NR>
+static cudaError_t flow_links_impl(const FlowLat& r, int stage, int swap, cudaStream_t st) {
+  const uint32_t n = (uint32_t)(r.t1 - r.t0) * (uint32_t)(r.g.str[3] >> 1);
+  return pdl_launch(k_flow_links<S, NR>, dim3(2 * ((n + FLOW_THREADS - 1) / FLOW_THREADS), 4), FLOW_THREADS, st, r, swap,
+                    stage);
+}
+
+cudaError_t launch_flow_links(const FlowLat& r, int prec, int nr, int stage, int swap, cudaStream_t st) {
+  if (stage < 1 || stage > 3) return cudaErrorInvalidValue;
+  LatDev probe;
+  probe.prec = prec;
+  probe.nr = nr;
+  QCB_DISPATCH_STORE(probe, flow_links_impl, r, stage, swap, st);
+}
+
 template <typename S, int NR>
 static cudaError_t update_impl(const FlowSet& s, int stage, int swap, int step, cudaStream_t st) {
   if (s.blocks == 0) return cudaSuccess;

@@ -35,7 +35,8 @@ cudaError_t loops_reserve(LoopBuf* buf, size_t want, size_t least) {
 }
 LoopDev loops_view(const LoopBuf& buf, size_t off, const Geom& g, int prec, int slices) {
   const size_t es = prec == QCB_PREC_FP64 ? 8 : 4, st = loops_stride(g, slices);
-  LoopDev k;
+  LoopDev k = {};
+  if (slices == 0) return k;
   k.p = (char*)buf.p + off;
   k.tr = (char*)buf.p + off + 6 * 2 * 8 * st * es;
   k.off = (uint8_t*)buf.p + off + 6 * 2 * 9 * st * es;
@@ -57,7 +58,12 @@ std::vector<FlowLat> flow_rounds(const LatDev& L, const LoopDev& k) {
   r.tile = 32;
   r.nsteps = 1 << 30;
   const bool full = k.slices >= g.L[3];
-  if (!full && k.slices < 2) return out;  // no room: nothing can run (loops_reserve rules it out)
+  if (!k.p) {
+    r.t0 = g.tlo;
+    r.t1 = g.thi + 1;
+    r.kt0 = r.kn = 0;
+    return {r};
+  }
   for (int t = g.tlo; t <= g.thi;) {
     const int room = full ? g.L[3] : k.slices - 1;  // one slot holds the slice before the round
     r.t0 = t;
@@ -234,6 +240,82 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_QE_MINB32 :
     parts[first + blockIdx.x] = bq;
     parts[nparts + first + blockIdx.x] = be;
   }
+}
+
+// F_{mu nu} = (C - C^dag) / 8 of the plaquette leaf M: its share.
+template <typename R>
+__device__ __forceinline__ void add_leaf(ah9<R>& F, const m3<R>& M, R sg) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) F.d[k] = fma(R(0.25) * sg, M.e[k][k].im, F.d[k]);
+  const int a[3] = {0, 0, 1}, b[3] = {1, 2, 2};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    F.o[k].re = fma(R(0.125) * sg, M.e[a[k]][b[k]].re - M.e[b[k]][a[k]].re, F.o[k].re);
+    F.o[k].im = fma(R(0.125) * sg, M.e[a[k]][b[k]].im + M.e[b[k]][a[k]].im, F.o[k].im);
+  }
+}
+
+// Q and E without loops: the four leaves of every plane multiplied out (twelve products).
+template <typename S, int NR>
+__global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? 4 : 2)
+    k_clover(const __grid_constant__ FlowLat L, int swap, double* __restrict__ parts, uint32_t first, uint32_t nparts) {
+  typedef arith_t<S> R;
+  typedef Links<S, NR> F;
+  __shared__ double sh[FLOW_THREADS / 32];
+  pdl_wait();
+  const F f = flow_links<S, NR>(L, swap);
+  const uint32_t half = (uint32_t)(L.g.str[3] >> 1), n = (uint32_t)(L.t1 - L.t0) * half, k = block_site(blockIdx.x);
+  const int par = block_parity(), opp = par ^ 1;
+  double q = 0.0, e = 0.0;
+  if (k < n) {
+    const uint32_t i = (uint32_t)L.t0 * half + k;
+    const Coord x = cb_coord(L.g, par, i);
+    const NbOff o = nb_offsets(L.g, x);
+    const int32_t s = (int32_t)x.s;
+    ah9<R> prev;
+#pragma unroll 1
+    for (int p = 0; p < 6; ++p) {
+      const int h = p >> 1;
+      const int mu = (p & 1) == 0 ? 0 : (h == 0 ? 2 : 1), nu = (p & 1) == 0 ? h + 1 : (h == 2 ? 2 : 3);
+      const int32_t umu = sel4(o.up, mu), unu = sel4(o.up, nu), dmu = sel4(o.dn, mu), dnu = sel4(o.dn, nu);
+      const uint32_t imu = cb_index((uint32_t)(s + dmu)), inu = cb_index((uint32_t)(s + dnu)),
+                     imn = cb_index((uint32_t)(s + dmu + dnu)), iun = cb_index((uint32_t)(s + dmu + unu)),
+                     ium = cb_index((uint32_t)(s + dnu + umu));
+      ah9<R> A = {};
+      const m3<R> G = mul_nn(f.template load<R>(mu, par, i), f.template load<R>(nu, opp, cb_index((uint32_t)(s + umu))));
+      const m3<R> H = mul_nn(f.template load<R>(nu, par, i), f.template load<R>(mu, opp, cb_index((uint32_t)(s + unu))));
+      add_leaf(A, mul_na(G, H), R(1));
+      add_leaf(A, loop_beside<F, R>(f, nu, mu, opp, imu, iun, i), R(-1));
+      add_leaf(A, loop_across<F, R>(f, mu, nu, par, imn, inu, imu), R(1));
+      add_leaf(A, loop_beside<F, R>(f, mu, nu, opp, inu, ium, i), R(1));
+      e += (double)sqnorm_ah(A);
+      if (p & 1) {
+        const double t = (double)re_tr_ah(prev, A);
+        q += h == 1 ? -t : t;
+      } else {
+        prev = A;
+      }
+    }
+  }
+  const double bq = block_sum<FLOW_THREADS>(q, sh);
+  const double be = block_sum<FLOW_THREADS>(e, sh);
+  if (threadIdx.x == 0) {
+    parts[first + blockIdx.x] = bq;
+    parts[nparts + first + blockIdx.x] = be;
+  }
+}
+
+template <typename S, int NR>
+static cudaError_t clover_impl(const FlowLat& r, int swap, double* parts, uint32_t first, uint32_t n, cudaStream_t st) {
+  return pdl_launch(k_clover<S, NR>, dim3(qe_blocks(r)), FLOW_THREADS, st, r, swap, parts, first, n);
+}
+
+cudaError_t launch_clover(const FlowLat& r, int prec, int nr, int swap, double* parts, uint32_t first, uint32_t n,
+                          cudaStream_t st) {
+  LatDev probe;
+  probe.prec = prec;
+  probe.nr = nr;
+  QCB_DISPATCH_STORE(probe, clover_impl, r, swap, parts, first, n, st);
 }
 
 template <typename S, int NR>

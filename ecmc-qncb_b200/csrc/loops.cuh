@@ -218,22 +218,33 @@ __device__ __forceinline__ void add_alg(alg8<R>& a, const alg8<R>& b, R sg = R(1
   for (int q = 0; q < 8; ++q) a.a[q] = fma(sg, b.a[q], a.a[q]);
 }
 
-// P_TA of the loop L_{mu nu}(y) (either order of mu and nu), begun at y+nu instead of y:
+// The loop L_{mu nu}(y) (either order of mu and nu), begun at y+nu instead of y:
 // U_nu(y)^dag U_mu(y) U_nu(y+mu) U_mu(y+nu)^dag.  iy, iymu, iynu: y (parity py), y+mu, y+nu.
 template <typename F, typename R>
-__device__ __forceinline__ alg8<R> leaf_beside(const F& f, int mu, int nu, int py, uint32_t iy, uint32_t iymu,
-                                               uint32_t iynu) {
+__device__ __forceinline__ m3<R> loop_beside(const F& f, int mu, int nu, int py, uint32_t iy, uint32_t iymu,
+                                             uint32_t iynu) {
   m3<R> M = mul_an(f.template load<R>(nu, py, iy), f.template load<R>(mu, py, iy));
   M = mul_nn(M, f.template load<R>(nu, py ^ 1, iymu));
-  return proj_ta(mul_na(M, f.template load<R>(mu, py ^ 1, iynu)));
+  return mul_na(M, f.template load<R>(mu, py ^ 1, iynu));
 }
 // The same begun at z+mu+nu: [U_nu(z) U_mu(z+nu)]^dag U_mu(z) U_nu(z+mu).
 template <typename F, typename R>
-__device__ __forceinline__ alg8<R> leaf_across(const F& f, int mu, int nu, int pz, uint32_t iz, uint32_t izmu,
-                                               uint32_t iznu) {
+__device__ __forceinline__ m3<R> loop_across(const F& f, int mu, int nu, int pz, uint32_t iz, uint32_t izmu,
+                                             uint32_t iznu) {
   const m3<R> H = mul_nn(f.template load<R>(nu, pz, iz), f.template load<R>(mu, pz ^ 1, iznu));
   const m3<R> G = mul_nn(f.template load<R>(mu, pz, iz), f.template load<R>(nu, pz ^ 1, izmu));
-  return proj_ta(mul_an(H, G));
+  return mul_an(H, G);
+}
+// P_TA of the two.
+template <typename F, typename R>
+__device__ __forceinline__ alg8<R> leaf_beside(const F& f, int mu, int nu, int py, uint32_t iy, uint32_t iymu,
+                                               uint32_t iynu) {
+  return proj_ta(loop_beside<F, R>(f, mu, nu, py, iy, iymu, iynu));
+}
+template <typename F, typename R>
+__device__ __forceinline__ alg8<R> leaf_across(const F& f, int mu, int nu, int pz, uint32_t iz, uint32_t izmu,
+                                               uint32_t iznu) {
+  return proj_ta(loop_across<F, R>(f, mu, nu, pz, iz, izmu, iznu));
 }
 // Out of line, so that the products cost the transports beside them no registers (the clover in FP32
 // has them in line: 380 us so, 312 in line on 20x24x28x36 with links that need them).

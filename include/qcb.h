@@ -72,7 +72,9 @@ int qcb_ctx_set_block(qcb_ctx* ctx, int threads);
  * buffer for the context's lattices and batches, and one for each server created after this call
  * (SIZE_MAX, the default: up to 1 GiB, or two time slices of a larger lattice).  A lattice whose loops do
  * not fit is worked through in rounds of time slices; its results do not depend on that but for the
- * order of the sums of Q and E.  It takes at least two time slices.  The present buffer is released. */
+ * order of the sums of Q and E.  Where not even two time slices fit, under this limit or because device
+ * memory is short, staples and clover leaves are multiplied out without work space (slower, and rounded
+ * differently).  The present buffer is released. */
 int qcb_ctx_set_loop_bytes(qcb_ctx* ctx, size_t bytes);
 /* The cudaStream_t the context launches on (as void*). */
 int qcb_ctx_stream(qcb_ctx* ctx, void** stream);
