@@ -109,7 +109,8 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_FLOW_MINB32
   }
 }
 
-// The stage without loops: one thread per link, its staples multiplied out.
+// The stage without loops: one thread per link, its staples multiplied out.  RK3 step of 20x24x28x36:
+// FP64 18-real 1350 us (880 with loops), FP32 12-real 555 (440).
 template <typename S, int NR>
 __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? 4 : 2)
     k_flow_links(const __grid_constant__ FlowLat L, int swap, int stage) {

@@ -130,9 +130,10 @@ __device__ __forceinline__ m3<R> lead(const F& f, int mu, int par, uint32_t i) {
 // the three products from the stored rows of their first factors; row 2 of the second and of L
 // from the cross product (each is in SU(3)).
 template <typename F, typename R>
-__device__ __forceinline__ m3<R> plaquette_loop(const F& f, const m3<R>& Umu, const m3<R>& Unu, int mu, int nu,
-                                                int par, uint32_t ixmu, uint32_t ixnu) {
+__device__ __forceinline__ m3<R> plaquette_loop(const F& f, const m3<R>& Umu, int mu, int nu, int par, uint32_t i,
+                                                uint32_t ixmu, uint32_t ixnu) {
   const int opp = par ^ 1;
+  const m3<R> Unu = lead<F, R>(f, nu, par, i);
   if constexpr (F::NREAL == 12) {
     const m3<R> G = mul_nn_rows01(Umu, f.template load<R>(nu, opp, ixmu));
     m3<R> H = mul_nn_rows01(Unu, f.template load<R>(mu, opp, ixnu));
