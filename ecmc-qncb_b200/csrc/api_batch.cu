@@ -612,6 +612,112 @@ void write_cache(const char* path, const std::map<std::string, int>& m) {
 
 }  // namespace
 
+namespace {
+
+// Times the whole batch on scratch copies of its lattices (heatbath on fw1, flow on fw1 and fw0), four
+// sweeps (one alone favours smaller items than a long run) or an RK3 step, with given work items: the
+// best of three runs, or the first that is not below `limit`.
+struct Tuner {
+  qcb_batch* b;
+  BatchLat* d_dsc = nullptr;
+  FlowLat* d_flow = nullptr;
+  uint32_t* d_pre = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  uint64_t groups = 0, largest = 0;
+
+  explicit Tuner(qcb_batch* batch) : b(batch) { pass_groups(b->lats, &groups, &largest); }
+  Tuner(const Tuner&) = delete;
+  ~Tuner() {
+    cudaFree(d_dsc);
+    cudaFree(d_flow);
+    cudaFree(d_pre);
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+  }
+  int open() {
+    BTRY(ensure_flow_plan(b));
+    const size_t rounds = b->flow[0].lats.size();
+    BCU(cudaMalloc(&d_dsc, b->n * sizeof(BatchLat)), "tune alloc");
+    BCU(cudaMalloc(&d_flow, rounds * sizeof(FlowLat)), "tune alloc");
+    BCU(cudaMalloc(&d_pre, 6 * rounds * sizeof(uint32_t)), "tune alloc");  // at least n + 1 for the heatbath
+    BCU(cudaEventCreate(&e0), "event");
+    BCU(cudaEventCreate(&e1), "event");
+    for (qcb_lattice* L : b->lats)
+      BCU(cudaMemcpyAsync(L->fw[1], L->dev.links, L->bytes, cudaMemcpyDeviceToDevice, b->ctx->stream), "copy");
+    return QCB_OK;
+  }
+  uint32_t hb_item(uint32_t most) const { return batch_tile(most, groups, largest, b->prec); }
+
+  template <typename F>
+  int best_of(const F& launch, float limit, float* ms) {
+    *ms = 1e30f;
+    for (int rep = 0; rep < 3; ++rep) {
+      BCU(cudaMemsetAsync(b->d_done, 0, b->n * sizeof(uint32_t), b->ctx->stream), "memset");
+      BCU(cudaEventRecord(e0, b->ctx->stream), "event");
+      BTRY(launch());
+      BCU(cudaEventRecord(e1, b->ctx->stream), "event");
+      BCU(cudaEventSynchronize(e1), "event sync");
+      float t = 0;
+      BCU(cudaEventElapsedTime(&t, e0, e1), "elapsed");
+      *ms = std::min(*ms, t);
+      if (t >= limit) break;
+    }
+    return QCB_OK;
+  }
+  int heatbath(const std::vector<uint32_t>& tile, float limit, float* ms) {
+    std::vector<BatchLat> dsc(b->n);
+    std::vector<uint32_t> pre(b->n + 1, 0);
+    for (int l = 0; l < b->n; ++l) {
+      BatchLat& d = dsc[l];
+      memset(&d, 0, sizeof d);
+      d.g = b->lats[l]->dev.g;
+      d.links = b->lats[l]->fw[1];
+      d.beta = 6.0;
+      d.k0 = 12345u;
+      d.tile = hb_item(tile[l]);
+      d.ntiles = ceil_div(d.g.Vh, d.tile);
+      pre[l + 1] = pre[l] + d.ntiles;
+    }
+    BCU(cudaMemcpyAsync(d_dsc, dsc.data(), b->n * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream), "H2D");
+    BCU(cudaMemcpyAsync(d_pre, pre.data(), pre.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, b->ctx->stream), "H2D");
+    BatchRun r;
+    r.lats = d_dsc;
+    r.prefix = d_pre;
+    r.nlat = b->n;
+    r.per_level = pre[b->n];
+    r.done = b->d_done;
+    r.status = b->d_status;
+    r.n_hits = 1;
+    r.nlevels = 32;
+    return best_of([&]() -> int {
+      BCU(launch_batch(r, b->prec, b->nr, 128, 0, b->ctx->stream), "tune launch");
+      b->ctx->launches++;
+      return QCB_OK;
+    }, limit, ms);
+  }
+  int flow(const std::vector<uint32_t>& tile, float limit, float* ms) {
+    std::vector<FlowItem> items = flow_items(b->lats, tile, 0);
+    for (int l = 0; l < b->n; ++l) {
+      items[l].L.links = b->lats[l]->fw[1];
+      items[l].b = b->lats[l]->fw[0];
+      items[l].eps = 0.02;
+    }
+    const FlowPlan fp = flow_plan(items, b->ctx->loops);
+    BCU(cudaMemcpyAsync(d_flow, fp.lats.data(), fp.lats.size() * sizeof(FlowLat), cudaMemcpyHostToDevice,
+                        b->ctx->stream),
+        "H2D");
+    BCU(cudaMemcpyAsync(d_pre, fp.prefix.data(), fp.prefix.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                        b->ctx->stream),
+        "H2D");
+    return best_of([&]() -> int {
+      BCU(run_flow_plan(fp, d_flow, d_pre, b->prec, b->nr, 0, 1, b->ctx->stream, &b->ctx->launches), "tune launch");
+      return QCB_OK;
+    }, limit, ms);
+  }
+};
+
+}  // namespace
+
 extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
   if (!b) return bfail(QCB_ERR_INVALID, "null batch");
   std::lock_guard<std::mutex> lk(b->ctx->mu);
@@ -629,126 +735,59 @@ extern "C" int qcb_batch_autotune(qcb_batch* b, const char* cache_path) {
             std::to_string(g.L[3])]
         .push_back(l);
   }
-  const int cands[] = {128, 256, 512, 1024, 2048};
-  std::vector<uint32_t> hb(b->hb_tile), fl(b->flow_tile);
-  cudaEvent_t e0, e1;
-  BCU(cudaEventCreate(&e0), "event");
-  BCU(cudaEventCreate(&e1), "event");
+  // What is not bounded by a choice stays at the default bound, under which the launch's own rule
+  // (batch_tile, flow_plan) decides.
+  std::vector<uint32_t> tile[2] = {std::vector<uint32_t>(b->n, DEFAULT_TILE), std::vector<uint32_t>(b->n, DEFAULT_TILE)};
+  std::vector<std::string> open;
   for (auto& kv : by_size) {
-    const std::string khb = pfx + "hb|" + kv.first, kfl = pfx + "flow|" + kv.first;
-    if (cache.count(khb) && cache.count(kfl)) {
+    if (cache.count(pfx + "hb|" + kv.first) && cache.count(pfx + "flow|" + kv.first)) {
       for (int l : kv.second) {
-        hb[l] = (uint32_t)cache[khb];
-        fl[l] = (uint32_t)cache[kfl];
+        tile[0][l] = (uint32_t)cache[pfx + "hb|" + kv.first];
+        tile[1][l] = (uint32_t)cache[pfx + "flow|" + kv.first];
       }
-      continue;
-    }
-    // A sub-batch of this size's lattices, timed on scratch copies: the heatbath runs on
-    // fw1 (copied from the links) and the flow on fw1/fw0, so the lattices are untouched.
-    BTRY(ensure_flow_plan(b));
-    const int m = (int)kv.second.size();
-    std::vector<qcb_lattice*> lats(m);
-    for (int j = 0; j < m; ++j) {
-      qcb_lattice* L = lats[j] = b->lats[kv.second[j]];
-      BCU(cudaMemcpyAsync(L->fw[1], L->dev.links, L->bytes, cudaMemcpyDeviceToDevice, b->ctx->stream), "copy");
-    }
-    uint64_t groups = 0, largest = 0;
-    pass_groups(lats, &groups, &largest);
-    std::vector<BatchLat> dsc(m);
-    std::vector<uint32_t> pre(m + 1, 0);
-    BatchLat* d_dsc = nullptr;
-    FlowLat* d_flow = nullptr;
-    uint32_t* d_pre = nullptr;
-    const size_t rounds = b->flow[0].lats.size() + (size_t)m;
-    BCU(cudaMalloc(&d_dsc, m * sizeof(BatchLat)), "tune alloc");
-    BCU(cudaMalloc(&d_flow, rounds * sizeof(FlowLat)), "tune alloc");
-    BCU(cudaMalloc(&d_pre, 6 * rounds * sizeof(uint32_t)), "tune alloc");
-    float best_hb = 1e30f, best_fl = 1e30f;
-    int arg_hb = DEFAULT_TILE, arg_fl = DEFAULT_TILE;
-    for (int kind = 0; kind < 2; ++kind)
-      for (int cand : cands) {
-        if (cand > 2 * (int)lats[0]->dev.g.Vh && cand != cands[0]) continue;  // larger than the lattice
-        BatchRun r;
-        FlowPlan fp;
-        if (kind == 0) {
-          for (int j = 0; j < m; ++j) {
-            BatchLat& d = dsc[j];
-            memset(&d, 0, sizeof d);
-            d.g = lats[j]->dev.g;
-            d.links = lats[j]->fw[1];
-            d.beta = 6.0;
-            d.k0 = 12345u;
-            d.tile = batch_tile((uint32_t)cand, groups, largest, b->prec);
-            d.ntiles = ceil_div(d.g.Vh, d.tile);
-            pre[j + 1] = pre[j] + d.ntiles;
-          }
-          r.lats = d_dsc;
-          r.prefix = d_pre;
-          r.nlat = m;
-          r.per_level = pre[m];
-          r.done = b->d_done;
-          r.status = b->d_status;
-          r.n_hits = 1;
-          r.nlevels = 16;  // 2 sweeps
-          BCU(cudaMemcpyAsync(d_dsc, dsc.data(), m * sizeof(BatchLat), cudaMemcpyHostToDevice, b->ctx->stream), "H2D");
-          BCU(cudaMemcpyAsync(d_pre, pre.data(), (m + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, b->ctx->stream),
-              "H2D");
-        } else {
-          std::vector<FlowItem> items = flow_items(lats, std::vector<uint32_t>(m, (uint32_t)cand), 0);
-          for (int j = 0; j < m; ++j) {
-            items[j].L.links = lats[j]->fw[1];
-            items[j].b = lats[j]->fw[0];
-            items[j].eps = 0.02;
-          }
-          fp = flow_plan(items, b->ctx->loops);
-          BCU(cudaMemcpyAsync(d_flow, fp.lats.data(), fp.lats.size() * sizeof(FlowLat), cudaMemcpyHostToDevice,
-                              b->ctx->stream),
-              "H2D");
-          BCU(cudaMemcpyAsync(d_pre, fp.prefix.data(), fp.prefix.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                              b->ctx->stream),
-              "H2D");
-        }
-        float best = 1e30f;
-        for (int rep = 0; rep < 3; ++rep) {
-          BCU(cudaMemsetAsync(b->d_done, 0, m * sizeof(uint32_t), b->ctx->stream), "memset");
-          BCU(cudaEventRecord(e0, b->ctx->stream), "event");
-          if (kind == 0) {
-            BCU(launch_batch(r, b->prec, b->nr, 128, 0, b->ctx->stream), "tune launch");
-            b->ctx->launches++;
-          } else {  // 2 RK3 steps
-            BCU(run_flow_plan(fp, d_flow, d_pre, b->prec, b->nr, 0, 2, b->ctx->stream, &b->ctx->launches),
-                "tune launch");
-          }
-          BCU(cudaEventRecord(e1, b->ctx->stream), "event");
-          BCU(cudaEventSynchronize(e1), "event sync");
-          float ms = 0;
-          BCU(cudaEventElapsedTime(&ms, e0, e1), "elapsed");
-          if (rep > 0) best = std::min(best, ms);
-        }
-        if (kind == 0 && best < best_hb) {
-          best_hb = best;
-          arg_hb = cand;
-        }
-        if (kind == 1 && best < best_fl) {
-          best_fl = best;
-          arg_fl = cand;
-        }
-      }
-    cudaFree(d_dsc);
-    cudaFree(d_flow);
-    cudaFree(d_pre);
-    cache[khb] = arg_hb;
-    cache[kfl] = arg_fl;
-    for (int l : kv.second) {
-      hb[l] = (uint32_t)arg_hb;
-      fl[l] = (uint32_t)arg_fl;
+    } else {
+      open.push_back(kv.first);
     }
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  if (!open.empty()) {
+    Tuner t(b);
+    BTRY(t.open());
+    for (int kind = 0; kind < 2; ++kind) {
+      // the bounds under which the launch differs from the one under the default bound, one for each item
+      // size, from half of the rule's on (FP32 heatbath, 54 lattices: 32 links take 10.4 ms, 160 8.4)
+      const uint32_t rule = kind == 0 ? t.hb_item(DEFAULT_TILE) : flow_tile_most(flow_items(b->lats, tile[1], 0));
+      std::vector<uint32_t> cands;
+      uint32_t last = 0;
+      for (uint32_t c = 32; c < rule; c += 32) {
+        const uint32_t item = kind == 0 ? t.hb_item(c) : c;
+        if (item != last && item != rule && 2 * item >= rule) cands.push_back(c);
+        last = item;
+      }
+      auto time = [&](float limit, float* ms) {
+        return kind == 0 ? t.heatbath(tile[0], limit, ms) : t.flow(tile[1], limit, ms);
+      };
+      float base = 0;
+      if (!cands.empty()) BTRY(time(1e30f, &base));
+      for (const std::string& size : open) {
+        uint32_t pick = DEFAULT_TILE;
+        for (uint32_t c : cands) {
+          for (int l : by_size[size]) tile[kind][l] = c;
+          const float below = 0.98f * base;  // by more than repeated runs differ
+          float ms = 0;
+          BTRY(time(below, &ms));
+          if (ms < below) {
+            base = ms;
+            pick = c;
+          }
+        }
+        for (int l : by_size[size]) tile[kind][l] = pick;
+        cache[pfx + (kind == 0 ? "hb|" : "flow|") + size] = (int)pick;
+      }
+    }
+  }
   BTRY(batch_status(b));
   write_cache(cache_path, cache);
-  b->hb_tile = hb;
-  b->flow_tile = fl;
+  b->hb_tile = tile[0];
+  b->flow_tile = tile[1];
   return upload_layout(b);
 }

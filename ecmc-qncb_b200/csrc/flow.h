@@ -119,6 +119,8 @@ struct FlowPlan {
 };
 // Buffer sizes for these lattices: all loops at once, and the least one round of each needs.
 void flow_plan_bytes(const std::vector<FlowItem>& items, size_t* want, size_t* least);
+// Most sites per work item of a plan; an item's own tile only makes it smaller.
+uint32_t flow_tile_most(const std::vector<FlowItem>& items);
 FlowPlan flow_plan(const std::vector<FlowItem>& items, const LoopBuf& buf);
 // n RK3 steps of every lattice from its links a (odd = 0) or b (odd = 1), and the clover sums
 // of the links; d_lats and d_prefix are the plan's arrays on the device.  *launches counts.

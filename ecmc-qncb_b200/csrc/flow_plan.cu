@@ -14,14 +14,17 @@ void flow_plan_bytes(const std::vector<FlowItem>& items, size_t* want, size_t* l
   }
 }
 
-FlowPlan flow_plan(const std::vector<FlowItem>& items, const LoopBuf& buf) {
-  // Sites per work item: the items' own value, but at most 128 (a block's threads), and 32 while the
-  // whole plan then has fewer than 4096 update blocks.  Four RK3 steps, FP32 12-real: 4^4 with 6^4
-  // 89 us with 32, 159 with 128, 258 with 256; eight of 8^4 207, 315, 474; four of 12^4 380, 396,
-  // 614; 54 of 8^4 to 16^4 9.14 ms, 8.93, 9.03.
+// At most 128 (a block's threads), and 32 while the whole plan then has fewer than 4096 update blocks.
+// Four RK3 steps, FP32 12-real: 4^4 with 6^4 89 us with 32, 159 with 128, 258 with 256; eight of 8^4 207,
+// 315, 474; four of 12^4 380, 396, 614; 54 of 8^4 to 16^4 9.14 ms, 8.93, 9.03.
+uint32_t flow_tile_most(const std::vector<FlowItem>& items) {
   uint64_t blocks = 0;
   for (const FlowItem& it : items) blocks += 2 * ((uint64_t)(it.L.g.Vh + 31) / 32);
-  const uint32_t most = blocks < 4096 ? 32u : 128u;
+  return blocks < 4096 ? 32u : 128u;
+}
+
+FlowPlan flow_plan(const std::vector<FlowItem>& items, const LoopBuf& buf) {
+  const uint32_t most = flow_tile_most(items);
   FlowPlan p;
   p.qe_prefix.push_back(0);
   auto add = [&](const FlowItem& it, FlowLat r) {

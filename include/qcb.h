@@ -239,10 +239,13 @@ typedef struct qcb_batch_plan {
 } qcb_batch_plan;
 int qcb_batch_run(qcb_batch* b, const qcb_batch_plan* plan, const double* betas, const uint64_t* seeds,
                   const uint64_t* sweep_offsets, double* results, int* used_graph);
-/* Project-written autotuner: for each distinct lattice size of the batch, times the
- * heatbath and the flow of that size's lattices on scratch copies for candidate tiles and
- * keeps the fastest; results are cached in the JSON file cache_path (created if absent,
- * NULL = no cache) under keys "<device name>|<precision>-<storage>|<hb|flow>|LxLyLzLt". */
+/* Project-written autotuner of the tiles: for each distinct lattice size of the batch, times the
+ * heatbath and the flow of the whole batch on scratch copies under the bounds that make the work items
+ * of that size smaller, down to a half, and keeps one that is faster by more than 2%, else the default bound (256,
+ * which leaves the items' size to the launch).  Where the launch has one size only (FP64 heatbath, the
+ * flow of small batches) nothing is timed.  Results are cached in the JSON file cache_path (created if
+ * absent, NULL = no cache) under keys "<device name>|<precision>-<storage>|<hb|flow>|LxLyLzLt"; cached sizes
+ * are not timed again. */
 int qcb_batch_autotune(qcb_batch* b, const char* cache_path);
 
 /* ---- slabs: one lattice split along t over several devices or processes ------------------
