@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(128, HbMinBlocks<S>::value) k_hb_pass_meas(Geo
     const uint32_t b = blockIdx.x - (uint32_t)nb, i = block_site(b / rows);
     const int par = block_parity();
     if (i < g.Vh)
-      v = site_plaquettes<Links<S, NR>, R>(g, f, cb_coord(g, par, i), par, i, (int)(b % rows), rows, 3);
+      v = site_plaquettes<Links<S, NR>, R, true>(g, f, cb_coord(g, par, i), par, i, (int)(b % rows), rows, 3);
   }
   const double b = block_sum<128>(v, sh);
   if (threadIdx.x == 0) parts[blockIdx.x] = b;
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(128) k_hb_quad_meas(Geom g, Links<double, 18> 
     const Coord x = cb_coord(g, par, i);
     double retr = 0;
     fails = hb_update_quad<Links<double, 18>, true>(q, g, f, x, 3, par, i, beta, k0, k1, sweep, n_hits, &retr);
-    const double p = plaquette_plane<Links<double, 18>, double>(g, f, x, par, i, q.lane == 2 ? 1 : 0, q.lane == 0 ? 1 : 2);
+    const double p = plaquette_plane<Links<double, 18>, double, true>(g, f, x, par, i, q.lane == 2 ? 1 : 0, q.lane == 0 ? 1 : 2);
     const double sum = q.get(p, 0) + q.get(p, 1) + q.get(p, 2);
     if (q.lane == 0) {
       v = sum;

@@ -158,7 +158,8 @@ int qcb_translate(qcb_lattice* lat, const int shift[4]);
 
 /* ---- observables -------------------------------------------------------------------
  * mpi::observables::mean_plaquette_global (src/observables/observables_mpi.cpp:8-43):
- * sum_{x, mu<nu} Re tr P_{mu nu}(x) / 3, divided by 6V.  FP64 accumulation. */
+ * sum_{x, mu<nu} Re tr P_{mu nu}(x) / 3, divided by 6V.  FP64 accumulation.  Of the stored links, unitary
+ * or not (QCB_R12: rows 0 and 1, and their conjugate cross product). */
 int qcb_plaquette(qcb_lattice* lat, double* out);
 /* topo_q_e_clover_global (observables_mpi.cpp:61-150): clover charge Q (total) and energy
  * density E = (1/V) sum_x 1/2 sum_{mu<nu} |F_{mu nu}|^2 with F = (C - C^dagger)/8.

@@ -98,3 +98,22 @@ def test_batch_and_single_are_the_same_off_su3(ctx):
     for f, g in zip(single, batched):
         assert np.array_equal(f.get_links(), g.get_links())
     batch.close()
+
+
+@pytest.mark.parametrize("dims", DIMS)
+@pytest.mark.parametrize("prec,nr,tol", [("fp64", 12, 1e-13), ("fp64", 18, 1e-13), ("fp32", 12, 1e-6), ("fp32", 18, 1e-6)])
+def test_plaquette_is_that_of_the_stored_links(ctx, dims, prec, nr, tol):
+    """12-real storage keeps rows 0 and 1 as they were written; the link is these and their conjugate cross
+    product.  A plaquette of FP32 links is two products and a trace, below 20 roundings of 6e-8, and the
+    mean of hundreds of them is closer."""
+    u = off_by(orc.hot_philox(dims, 12), 1e-2, 5)
+    f = qcb.GaugeField(ctx, dims, prec, nr)
+    f.set_links(u)
+    stored = f.get_links()
+    assert np.abs(stored[..., :2, :] - u[..., :2, :]).max() < 1e-7
+    ref = orc.plaquette(stored, dims)
+    assert abs(qcb.observables.mean_plaquette_global(f) - ref) < tol
+    batch = qcb.Batch(ctx, [f])
+    assert abs(batch.plaquette()[0] - ref) < tol
+    batch.close()
+    f.close()
