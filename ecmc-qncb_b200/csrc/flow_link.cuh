@@ -28,10 +28,11 @@ __device__ __forceinline__ void flow_reunit(m3<R>& U, int stage) {
   }
 }
 
-// U' = exp(X) U from E = exp_su3(X).  FP32: U + (exp(X) - 1) U, whose products are small, so that one
-// rounding at the links' size remains (Q after nine RK3 steps on 24^4 against the FP64 flow, rms of six
-// lattices: 2.0e-7, with the products of exp(X) itself 3.4e-7; RK3 step 880 -> 884 us).  12-real storage keeps rows 0 and 1 only (the FP64
-// re-orthonormalisation of stage 3 also reads only those), so row 2 of the product is not formed.
+// U' = exp(X) U from E = flow_exp(X).  FP32: U + (exp(X) - 1) U, whose products are small, so that one
+// rounding at the links' size remains (Q after nine RK3 steps on 24^4 against the FP64 flow, rms of
+// six lattices: 2.0e-7, with the products of exp(X) itself 3.4e-7; RK3 step 880 -> 884 us).  12-real
+// storage keeps rows 0 and 1 only (the FP64 re-orthonormalisation of stage 3 also reads only those), so
+// row 2 of the product is not formed.
 template <typename F, typename R>
 __device__ __forceinline__ m3<R> flow_product(const m3<R>& E, const m3<R>& U) {
   constexpr int ROWS = F::NREAL == 12 ? 2 : 3;

@@ -4,9 +4,8 @@
 // The reference runs one lattice per process (src/bin/gauge_hb_ncb.cpp:18-201).  Here a
 // batch of lattices of different sizes and couplings shares one cooperative launch: the
 // work of every lattice is cut into levels (checkerboard heatbath passes) and each level into
-// tiles of sites.  Work items are ordered level-major across
-// lattices, item j = (level, lattice, tile), and warp w of W processes items w, w+W, w+2W, ...
-// in order.  Before an item of level k of lattice l starts, all tiles of level k-1 of the
+// tiles of sites.  Work items are ordered level-major across lattices, item j = (level, lattice,
+// tile), and warp w of W processes items w, w+W, w+2W, ... in order.  Before an item of level k of lattice l starts, all tiles of level k-1 of the
 // same lattice must be finished: a per-lattice counter done[l] counts finished tiles, and
 // the warp waits (acquire) until done[l] >= k * ntiles[l].  Levels of different lattices
 // overlap freely, so small lattices do not serialise the GPU.
@@ -15,9 +14,8 @@
 // increasing order, and the cooperative launch makes all of them co-resident; so the
 // smallest unfinished item always has its dependencies done.  Every wait is bounded by
 // wall-clock time (WAIT_NS); a warp that gives up raises an abort flag that makes every
-// other warp return, and the host reports the error.  Links are read
-// with L2-coherent loads (LD_CG), because warps read links that other warps wrote in the
-// same launch.
+// other warp return, and the host reports the error.  Links are read with L2-coherent loads
+// (LD_CG), because warps read links that other warps wrote in the same launch.
 //
 // Bound: at large batches the FP32 pipes, as a single lattice's pass; at small ones the latency of
 // a level (one link's chain, then the counter's round trip).  An item is a warp's, not a block's:
@@ -228,9 +226,8 @@ cudaError_t launch_wait_probe(const uint32_t* flag, uint32_t* status, uint64_t l
 
 // ---- batched observables --------------------------------------------------------------------
 // Plaquette: one reduction item per (lattice, tile of RED_SITES sites, half of each parity), partial
-// sums parts[item].  Plaquette and
-// clover partials are then added by one block per lattice in a fixed order with Neumaier
-// compensation.
+// sums parts[item].  Plaquette and clover partials are then added by one block per lattice in a fixed
+// order with Neumaier compensation.
 constexpr int RED_SITES = 128;
 int batch_red_sites() { return RED_SITES; }
 

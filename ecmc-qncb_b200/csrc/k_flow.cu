@@ -9,21 +9,20 @@
 // previous stage; the force accumulator holds 8 reals per link.
 //
 // Measured per RK3 step on 32^4, against kernels that multiplied out the staples of every link
-// (twelve products each; in FP32 ten, with one product shared by a plane's two links): FP64
-// 18-real 2.65 -> 1.93 ms, FP32 12-real 1.08 -> 0.92 ms.  Of a stage, the loops take a third and the
-// update two thirds (FP32 215 us, 0.71-0.85 GB of DRAM traffic, 56% issue; FP64 420-480 us, 56% of
-// the DRAM rate).  A smaller loop buffer, whose rounds of slices would stay in L2, costs more in
-// half-filled last waves than it saves: 110, 70 and 24 MB made the FP32 step 1.05, 1.09 and 1.24 ms where 1 GiB made it 0.97.
+// (twelve products each; in FP32 ten, with one product shared by a plane's two links), in turn on one
+// box: FP64 18-real 2.71 -> 2.00 ms, FP32 12-real 1.05 -> 0.91 ms.  Of an FP32 stage, the loops take
+// 110 us and the update 187 to 214 (0.71-0.85 GB of DRAM traffic, 68% issue).  A smaller loop buffer, whose
+// rounds of slices would stay in L2, costs more in half-filled last waves than it saves: 110, 70 and
+// 24 MB made the FP32 step 1.05, 1.09 and 1.24 ms where 1 GiB made it 0.97.
 #include "flow_launch.cuh"
 #include "flow_link.cuh"
 
 namespace qcb {
 
-// Four warps work on 32 sites of one parity.  Warp nu first moves the three loops K_{mu nu}(x-nu)
-// up along U_nu(x-nu), which it loads and completes once
-// into shared memory; then warp mu sums its link's force from them and applies the stage.
-// (18-real: the test whether U_nu(x-nu) is unitary is hidden, RK3 step of 20x24x28x36 FP64 880 us
-// with and without; with every link off, 1400 us.)
+// Four warps work on 32 sites of one parity.  Warp nu first moves the three loops K_{mu nu}(x-nu) up
+// along U_nu(x-nu), which it loads and completes once, into shared memory; then warp mu sums its link's
+// force from them and applies the stage.  (18-real: the test whether U_nu(x-nu) is unitary is hidden, RK3
+// step of 20x24x28x36 FP64 880 us with and without; with every link off, 1400 us.)
 #ifndef QCB_FLOW_MINB32
 #define QCB_FLOW_MINB32 5
 #endif
@@ -102,7 +101,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? QCB_FLOW_MINB32
         add_alg(Z, B, nu > w ? R(1) : R(-1));
       }
       const alg8<R> X = flow_x<STAGE, AlgField<S>, R>(acc, Z, Z0, eps, w, par, i);
-      m3<R> Un = flow_product<F, R>(exp_su3(X), U);
+      m3<R> Un = flow_product<F, R>(flow_exp(X), U);
       flow_reunit<R>(Un, STAGE);
       dst.template store<R>(w, par, i, Un);
     }
@@ -140,7 +139,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, sizeof(S) == 4 ? 4 : 2)
     X = flow_x<2, AlgField<S>, R>(acc, Z, Z0, eps, mu, par, i);
   else
     X = flow_x<3, AlgField<S>, R>(acc, Z, Z0, eps, mu, par, i);
-  m3<R> Un = flow_product<F, R>(exp_su3(X), U);
+  m3<R> Un = flow_product<F, R>(flow_exp(X), U);
   flow_reunit<R>(Un, stage);
   dst.template store<R>(mu, par, i, Un);
 }

@@ -90,7 +90,7 @@ uint32_t update_blocks(const FlowLat& r) { return 2 * tiles_of(r.g, r.t1 - r.t0,
 
 // ---- the loops --------------------------------------------------------------------------
 // One thread per site and grid row: row y of n takes planes y, y + n, ...; the planes run
-// through one body that is not unrolled.  Measured on 32^4 FP32 12-real: 125 us, 0.37 GB of DRAM
+// through one body that is not unrolled.  Measured on 32^4 FP32 12-real: 110 us, 0.37 GB of DRAM
 // traffic (the links read and the loops written once), bound by the FP32 pipes and by the latency
 // of its sixteen links; FP64 18-real 250 us.  Six rows instead of one make a small lattice's few
 // blocks six times as many; from 2048 blocks the chip is full without that, and one row reads
@@ -165,8 +165,8 @@ cudaError_t launch_loops(const FlowSet& s, int prec, int nr, bool trace, int swa
 // |F_mu nu|^2 (the 1/(4 pi^2) and 1/2 are applied to the totals).  The six planes run through
 // one body, in the pairs (01, 23), (02, 13), (03, 12); each pair's share is added in FP64.
 // Three transports a plane where four leaves were nine products: Q and E of 32^4 alone, loops
-// included, FP32 12-real 572 -> 370 us, FP64 18-real 1301 -> 720 us; with the loops already there
-// for an RK3 step, FP32 210 us more.
+// included, FP32 12-real 442 -> 315 us, FP64 18-real 1073 -> 680 us; with the loops already there
+// for an RK3 step, FP32 187 us more.
 // In 18-real storage the bytes of the links that are not unitary are read first, for all planes
 // together: 20x24x28x36 with SU(3) links FP64 296 us without the test, 320 with it (335 with the
 // bytes read plane by plane); links that need the products 530, FP32 200, 217 and 312.

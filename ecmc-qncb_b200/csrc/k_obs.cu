@@ -2,9 +2,10 @@
 //
 // Reference: mean_plaquette_local / _global (src/observables/observables_mpi.cpp:8-43): serial
 // sum of Re tr(U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag)/3 over x and mu < nu, / (6V).
-// Here: one thread per site (a slab skips its halo slices), per-site value in the lattice's arithmetic type, converted to FP64; FP64 tree reduction inside each block; the block partials are
-// summed in a fixed order with Neumaier compensation by k_total.  The grid
-// is a fixed multiple of the SM count (grid-stride loop), so the scratch is bounded.
+// Here: one thread per site (a slab skips its halo slices), the site's value in the lattice's
+// arithmetic type, converted to FP64, and an FP64 tree in each block; k_total adds the block sums in a fixed
+// order with Neumaier compensation.  The grid has a block for 64 checkerboard indices up to a bound
+// (the library's RED_BLOCKS, or the caller's scratch), beyond which blocks stride.
 #include <algorithm>
 
 #include "dispatch.cuh"
@@ -18,8 +19,8 @@ constexpr int RED_THREADS = 128;
 // One block per 64 checkerboard indices up to 60 per SM (32^4: 8192), from there a grid-stride loop.
 constexpr int RED_BLOCKS = 148 * 60;
 
-// Minimum resident blocks per SM of the reduction (32^4: FP32 5 114 us, 4 121; FP64 3 224 us, 2 267,
-// 4 235).
+// Minimum resident blocks per SM of the reduction (32^4, 18-real: FP64 3 224 us, 2 267, 4 235; FP32
+// 12-real with the third rows of products rebuilt: 5 114 us, 4 121).
 template <typename S>
 struct RedMinBlocks {
   static constexpr int value = sizeof(S) == 4 ? 5 : 3;

@@ -15,11 +15,6 @@ struct LatDev {
   void* links;
 };
 
-// Device description of one su(3) algebra field (flow accumulator), same precision.
-struct AlgDev {
-  void* p;
-};
-
 size_t link_bytes(const Geom& g, int prec, int nr);
 size_t alg_bytes(const Geom& g, int prec);
 Geom make_geom(const int dims[4]);

@@ -59,7 +59,7 @@ extern "C" int qcb_plaquette_noalloc(const void* links, const int dims[4], int p
   L.nr = storage;
   L.links = const_cast<void*>(links);
 
-  // One partial per reduction block; the grid never exceeds the library's reduction grid.
+  // One partial per reduction block; blocks of a larger lattice stride over its sites.
   const uint64_t want = (vol + (uint64_t)reduce_threads() - 1) / (uint64_t)reduce_threads();
   const int nblocks = (int)(want < (uint64_t)QCB_NOALLOC_MAX_PARTIALS ? want : (uint64_t)QCB_NOALLOC_MAX_PARTIALS);
 

@@ -526,7 +526,10 @@ int qcb_server_create(qcb_ctx* ctx, const qcb_server_config* cfg, qcb_server** o
   // links and accumulator).  Grown in the first ticks instead, its cudaFree and cudaMalloc held a
   // tick for up to 0.6 s while the driver cleared memory freed before.  Less is no error: the jobs
   // then take turns.
-  s->loops.limit = ctx->loops.limit;
+  {
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    s->loops.limit = ctx->loops.limit;
+  }
   loops_reserve(&s->loops, std::max<size_t>(budget / 2, 1), 1);
   s->t0 = std::chrono::steady_clock::now();
   s->thr = std::thread(scheduler, s);

@@ -213,20 +213,6 @@ __device__ __forceinline__ void acc_an(m3<R>& acc, const m3<R>& a, const m3<R>& 
       acc.e[i][j] = s;
     }
 }
-// acc += a^dagger * b^dagger
-template <typename R>
-__device__ __forceinline__ void acc_aa(m3<R>& acc, const m3<R>& a, const m3<R>& b) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      cx<R> s = acc.e[i][j];
-      s = cfma_cc(a.e[0][i], b.e[j][0], s);
-      s = cfma_cc(a.e[1][i], b.e[j][1], s);
-      s = cfma_cc(a.e[2][i], b.e[j][2], s);
-      acc.e[i][j] = s;
-    }
-}
 // Rows 0 and 1 of a * b^dagger (only rows 0 and 1 of a are read; row 2 of c is unset).
 template <typename R>
 __device__ __forceinline__ m3<R> mul_na_rows01(const m3<R>& a, const m3<R>& b) {
@@ -265,13 +251,6 @@ __device__ __forceinline__ void add_m3(m3<R>& acc, const m3<R>& w) {
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) acc.e[i][j] = acc.e[i][j] + w.e[i][j];
-}
-template <typename R>
-__device__ __forceinline__ void add_m3_adj(m3<R>& acc, const m3<R>& w) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) acc.e[i][j] = acc.e[i][j] + conj(w.e[j][i]);
 }
 // Re tr(a * b)
 template <typename R>
@@ -488,9 +467,10 @@ __device__ __forceinline__ void exp_coef(const alg8<R>& x, cx<R>& q0, cx<R>& q1,
   q2 = mk<R>(R(q[4]), R(q[5]));
 }
 
-// Returns exp(X); in FP32 exp(X) - 1, whose entries are of the order of X and keep their last bits.
+// The factor of the flow's product (flow_link.cuh): exp(X), in FP32 exp(X) - 1, whose entries are of the
+// order of X and keep their last bits.
 template <typename R>
-__device__ __forceinline__ m3<R> exp_su3(const alg8<R>& x) {
+__device__ __forceinline__ m3<R> flow_exp(const alg8<R>& x) {
   cx<R> q0, q1, q2;
   exp_coef(x, q0, q1, q2);
   m3<R> X = alg_to_m3(x);

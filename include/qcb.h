@@ -180,10 +180,10 @@ int qcb_topo_qe(qcb_lattice* lat, double* q, double* e);
  * QCB_NOALLOC_MAX_PARTIALS doubles (16 KiB per GPU, held until the process exits).  Every
  * call looks up that array's device address for the current device; the first call on a
  * device also loads the library's device code there (make it before any stream capture).
- * Calls share the array, so calls that overlap on the GPU race; requests that would need
- * more partial sums than the array holds are rejected with QCB_ERR_INVALID, and so are
- * links not aligned to the storage's chunk size (16 bytes; 8 for FP32 18-real) and an out
- * pointer not aligned to 8 bytes. */
+ * Calls share the array, so calls that overlap on the GPU race; a lattice of more than 128 sites for each
+ * of its partial sums is summed in strides.  Links not aligned to the storage's chunk size (16
+ * bytes; 8 for FP32 18-real) and an out pointer not aligned to 8 bytes are rejected with
+ * QCB_ERR_INVALID. */
 #define QCB_NOALLOC_MAX_PARTIALS 2048
 int qcb_plaquette_noalloc(const void* links, const int dims[4], int precision, int storage, size_t stride,
                           double* out, void* stream);
