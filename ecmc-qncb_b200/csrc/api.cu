@@ -122,17 +122,18 @@ LatDev with_links(const LatDev& d, void* p) {
   return r;
 }
 
-// The context's scratch with at least `need` doubles.  Replacing it is safe behind queued work: all
-// users are on the context's stream, and cudaFree waits for them.
+// The context's scratch with at least `need` doubles; the present one stays when there is no memory for
+// a larger one.  Replacing it is safe behind queued work: all users are on the context's stream, and
+// cudaFree waits for them.
 int ensure_scratch(qcb_ctx* c, size_t need) {
   if (c->scratch_n >= need) return QCB_OK;
-  cudaFree(c->d_scratch);
-  c->d_scratch = nullptr;
-  c->scratch_n = 0;
-  if (cudaMalloc(&c->d_scratch, need * sizeof(double)) != cudaSuccess) {
+  double* p = nullptr;
+  if (cudaMalloc(&p, need * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     return fail(QCB_ERR_NOMEM, "cannot allocate the measurement partial sums");
   }
+  cudaFree(c->d_scratch);
+  c->d_scratch = p;
   c->scratch_n = need;
   return QCB_OK;
 }

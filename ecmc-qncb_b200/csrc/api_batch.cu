@@ -47,7 +47,7 @@ struct qcb_batch {
   uint32_t* d_done = nullptr;
   uint32_t* d_status = nullptr;  // [0] KP cap hits, [1] wait timeouts, [2] abort
   uint32_t* h_status = nullptr;
-  double* d_scratch = nullptr;  // 2 * nred
+  double* d_scratch = nullptr;  // nred
   double* d_out = nullptr;
   double* h_out = nullptr;
   size_t out_cap = 0;
@@ -141,9 +141,8 @@ int upload_layout(qcb_batch* b) {
   }
   b->per_hb = ph[n];
   b->nred = pr[n];
-  cudaFree(b->d_scratch);
-  b->d_scratch = nullptr;
-  BCU(cudaMalloc(&b->d_scratch, (size_t)b->nred * sizeof(double)), "batch scratch");
+  if (!b->d_scratch)  // its size is that of the lattices, whatever the tiles
+    BCU(cudaMalloc(&b->d_scratch, (size_t)b->nred * sizeof(double)), "batch scratch");
   BCU(cudaMemcpyAsync(b->d_prefix, b->h_prefix.data(), b->h_prefix.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
                       b->ctx->stream),
       "prefix upload");
