@@ -6,6 +6,7 @@ import pytest
 import oracle as orc
 import qcb
 from qcb import _lib
+from qcb import slabs as qs
 
 pytestmark = pytest.mark.gpu
 
@@ -117,3 +118,28 @@ def test_plaquette_is_that_of_the_stored_links(ctx, dims, prec, nr, tol):
     assert abs(batch.plaquette()[0] - ref) < tol
     batch.close()
     f.close()
+
+
+@pytest.mark.parametrize("prec,size", [("fp64", 1e-4), ("fp32", 1e-3)])
+def test_rounds_and_slabs_are_the_same_off_su3(ctx, prec, size):
+    """Bad links next to the edges of rounds of time slices and of slabs, where the loops' neighbours come
+    from the round before or from a halo: the links are those of the whole lattice, bit for bit."""
+    dims = (4, 6, 4, 12)
+    u = off_by(orc.hot_philox(dims, 14), size, 6, 0.1)
+    c = qcb.Context(0)
+    whole, rounds = qcb.GaugeField(ctx, dims, prec, 18), qcb.GaugeField(c, dims, prec, 18)
+    c.set_loop_bytes(3 * 64 * (108 * (8 if prec == "fp64" else 4) + 8))  # 48 indices a slice: three or four
+    sl = qs.SlabLattice(ctx, dims, 3, prec, 18)
+    for f in (whole, rounds, sl):
+        f.set_links(u)
+    q, e = qcb.observables.topo_q_e_clover_global(whole)
+    for a, b in (qcb.observables.topo_q_e_clover_global(rounds), sl.topo_qe()):
+        assert abs(a - q) <= 1e-12 * max(1.0, abs(q)) and abs(b - e) <= 1e-12 * e
+    _lib.check(_lib.lib().qcb_flow_steps(whole.h, 0.02, 2))
+    _lib.check(_lib.lib().qcb_flow_steps(rounds.h, 0.02, 2))
+    sl.flow_steps(0.02, 2)
+    assert np.array_equal(rounds.get_links(), whole.get_links())
+    assert np.array_equal(sl.get_links(), whole.get_links())
+    sl.close()
+    c.close()
+    whole.close()
