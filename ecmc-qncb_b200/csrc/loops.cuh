@@ -91,14 +91,16 @@ struct Loops {
   }
 };
 
-// Whether |U U^dag - 1| is above 2^-40 (FP32: 2^-20) in the Frobenius norm, or not a number; the
+// Whether |U U^dag - 1| is above 2^-40 (FP32: 2^-21) in the Frobenius norm, or not a number; the
 // relative error of a loop moved along U is at most about that.  Measured on 16^4, the largest of all
 // links: FP64 after 10000 sweeps 1.8e-13, after 1000 RK3 steps 4e-14; FP32 after an RK3 step (which
-// ends with re-orthonormalised links) 1.4e-7, after 10 sweeps 5e-6 and after 2000 3e-4, so that the
-// clover of FP32 18-real links is multiplied out behind sweeps.
+// ends with re-orthonormalised links) or when SU(3) links are rounded 1.4e-7, after 10 sweeps 5e-6 and
+// after 2000 3e-4, all in one direction, so that the clover of FP32 18-real links is multiplied out
+// behind sweeps.  (At 2^-22 the bound meets the rounding between the stages of an RK3 step: 20x24x28x36
+// FP32 18-real 582 us a step, 540 at 2^-21.)
 template <typename S, typename R>
 __device__ __forceinline__ bool off_unitary(const m3<R>& U) {
-  constexpr double BOUND = sizeof(S) == 8 ? 0x1p-80 : 0x1p-40;
+  constexpr double BOUND = sizeof(S) == 8 ? 0x1p-80 : 0x1p-42;
   R s = 0;
 #pragma unroll
   for (int r = 0; r < 3; ++r) {

@@ -164,7 +164,7 @@ int qcb_plaquette(qcb_lattice* lat, double* out);
 /* topo_q_e_clover_global (observables_mpi.cpp:61-150): clover charge Q (total) and energy
  * density E = (1/V) sum_x 1/2 sum_{mu<nu} |F_{mu nu}|^2 with F = (C - C^dagger)/8.
  * C is that of the stored links: QCB_R18 links need not be unitary (those off by more than 1e-12 in
- * FP64, 1e-6 in FP32, take longer), QCB_R12 links are taken as SU(3).  Uses the
+ * FP64, 5e-7 in FP32, take longer), QCB_R12 links are taken as SU(3).  Uses the
  * context's plaquette-loop work space, as the Wilson flow does (allocated on first use, at most
  * 1 GiB or two time slices' loops, less when that much is not free). */
 int qcb_topo_qe(qcb_lattice* lat, double* q, double* e);

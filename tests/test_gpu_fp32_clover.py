@@ -29,3 +29,21 @@ def test_energy_density_is_unbiased(ctx, nr):
     assert abs(np.mean(rel)) < 6e-10, (np.mean(rel), np.std(rel))
     for g in (h, d, f):
         g.close()
+
+
+def test_energy_density_of_links_slightly_off_unitarity(ctx):
+    """FP32 18-real links with |U| a few roundings above 1, as a handful of sweeps leaves them: E is that of the
+    stored links (FP64 on the same links), within the rounding noise of 25000 planes (3e-7 / 160 each
+    field, ten times that), where loops moved along them as if they were unitary are off by 8e-7."""
+    dims = (8, 8, 8, 8)
+    h, d = qcb.GaugeField(ctx, dims), qcb.GaugeField(ctx, dims)
+    f = qcb.GaugeField(ctx, dims, "fp32", 18)
+    h.hot_start(3)
+    _lib.check(_lib.lib().qcb_heatbath(h.h, 6.0, 20, 1, 7, 0))
+    f.set_links(h.get_links() * (1 + 2e-7))
+    d.copy_from(f)
+    _, e = qcb.observables.topo_q_e_clover_global(f)
+    _, ref = qcb.observables.topo_q_e_clover_global(d)
+    assert abs(e - ref) < 2e-8 * ref, (e - ref) / ref
+    for g in (h, d, f):
+        g.close()

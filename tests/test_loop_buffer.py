@@ -65,3 +65,11 @@ def test_growth(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", str(CSRC), str(src), "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_limit_needs_a_context():
+    import qcb
+
+    lib = qcb._lib.lib()
+    assert lib.qcb_ctx_set_loop_bytes(None, 0) == 1
+    assert b"null" in lib.qcb_last_error()
