@@ -117,11 +117,10 @@ __device__ __forceinline__ void loops_site(const FlowLat& L, const Links<S, NR>&
       if (p == 0 || p == 3 || p == 5) K.store_off(mu, par, jx, off_unitary<S>(U));
       if (p == 2) K.store_off(3, par, jx, off_unitary<S>(f.template load<R>(3, par, i)));
     }
-    R tr;
-    const alg8<R> z = plaquette_alg<Links<S, NR>, R>(f, U, mu, nu, par, i, cb_index((uint32_t)((int32_t)x.s + sel4(o.up, mu))),
-                                                     cb_index((uint32_t)((int32_t)x.s + sel4(o.up, nu))), &tr);
-    K.template store<R>(p, par, jx, z);
-    if (TRACE) K.template store_tr<R>(p, par, jx, tr);
+    const m3<R> W = plaquette_loop<Links<S, NR>, R>(f, U, mu, nu, par, i, cb_index((uint32_t)((int32_t)x.s + sel4(o.up, mu))),
+                                                    cb_index((uint32_t)((int32_t)x.s + sel4(o.up, nu))));
+    K.template store<R>(p, par, jx, proj_ta(W));
+    if (TRACE) K.template store_tr<R>(p, par, jx, W.e[0][0].im + W.e[1][1].im + W.e[2][2].im);
   }
 }
 

@@ -128,53 +128,25 @@ __device__ __forceinline__ m3<R> lead(const F& f, int mu, int par, uint32_t i) {
     return f.template load<R>(mu, par, i);
 }
 
-// P_TA of L_{mu nu}(x) = G H^dag, G = U_mu(x) U_nu(x+mu), H = U_nu(x) U_mu(x+nu), and the imaginary part
-// of its trace.  H H^dag is Hermitian, so the anti-Hermitian part of L is that of M = (G - H) H^dag,
-// whose entries are as small as the result's: its products round at that size instead of at 1.  That
-// matters because a loop's rounding goes into the clover of four sites at once.  Q in FP32 12-real, rms
-// error of 200 fields of 12^4 at beta 6, and after 20 RK3 steps: 1.94e-7 and 1.25e-7 with L multiplied out,
-// 1.82e-7 and 1.07e-7 so (1.42e-7 and 0.90e-7 with every leaf multiplied out by itself, in 1.4 times the
-// time); flowed on 24^4 to t = 0.2, 9.9e-7, 9.0e-7 (1.27e-6 with staples multiplied out).
-// 12-real storage: rows 0 and 1 of G, of H and of M from the stored rows of their first factors, row 2 of
-// H from the cross product; L is in SU(3), so its row 2 is that of 1 + M by the cross product,
-// conj((-M02, -M12, 1 + M00 + M11) + M0 x M1).
+// L_{mu nu} = (U_mu(x) U_nu(x+mu)) (U_nu(x) U_mu(x+nu))^dag.  12-real storage: rows 0 and 1 of
+// the three products from the stored rows of their first factors; row 2 of the second and of L
+// from the cross product (each is in SU(3)).
 template <typename F, typename R>
-__device__ __forceinline__ alg8<R> plaquette_alg(const F& f, const m3<R>& Umu, int mu, int nu, int par, uint32_t i,
-                                                 uint32_t ixmu, uint32_t ixnu, R* tr) {
+__device__ __forceinline__ m3<R> plaquette_loop(const F& f, const m3<R>& Umu, int mu, int nu, int par, uint32_t i,
+                                                uint32_t ixmu, uint32_t ixnu) {
   const int opp = par ^ 1;
   const m3<R> Unu = lead<F, R>(f, nu, par, i);
   if constexpr (F::NREAL == 12) {
-    m3<R> G = mul_nn_rows01(Umu, f.template load<R>(nu, opp, ixmu));
+    const m3<R> G = mul_nn_rows01(Umu, f.template load<R>(nu, opp, ixmu));
     m3<R> H = mul_nn_rows01(Unu, f.template load<R>(mu, opp, ixnu));
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) G.e[r][c] = G.e[r][c] - H.e[r][c];
     reconstruct_row2(H);
-    m3<R> M = mul_na_rows01(G, H);
-    reconstruct_row2(M);  // conj(M0 x M1)
-    *tr = M.e[2][2].im;   // the imaginary parts of M00, M11 and of their conjugates cancel
-    alg8<R> z;
-    const R tr3 = *tr * R(1.0 / 3.0);
-    z.a[0] = M.e[0][0].im - tr3;
-    z.a[1] = M.e[1][1].im - tr3;
-    z.a[2] = R(0.5) * (M.e[0][1].re - M.e[1][0].re);
-    z.a[3] = R(0.5) * (M.e[0][1].im + M.e[1][0].im);
-    z.a[4] = fma(R(-0.5), M.e[2][0].re, M.e[0][2].re);
-    z.a[5] = fma(R(0.5), M.e[2][0].im, M.e[0][2].im);
-    z.a[6] = fma(R(-0.5), M.e[2][1].re, M.e[1][2].re);
-    z.a[7] = fma(R(0.5), M.e[2][1].im, M.e[1][2].im);
-    return z;
+    m3<R> L = mul_na_rows01(G, H);
+    reconstruct_row2(L);
+    return L;
   } else {
-    m3<R> G = mul_nn(Umu, f.template load<R>(nu, opp, ixmu));
+    const m3<R> G = mul_nn(Umu, f.template load<R>(nu, opp, ixmu));
     const m3<R> H = mul_nn(Unu, f.template load<R>(mu, opp, ixnu));
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) G.e[r][c] = G.e[r][c] - H.e[r][c];
-    const m3<R> M = mul_na(G, H);
-    *tr = M.e[0][0].im + M.e[1][1].im + M.e[2][2].im;
-    return proj_ta(M);
+    return mul_na(G, H);
   }
 }
 
@@ -358,7 +330,7 @@ __device__ __forceinline__ R sqnorm_ah(const ah9<R>& A) {
 // F_{mu nu}(x) = (C - C^dag) / 8 (observables_mpi.cpp:81-82), C the sum of the four leaves: a
 // quarter of the transported loops, their traces (the same at every corner) on the diagonal.  The third
 // place takes what the other two leave of the whole trace: three times FP32's 1/3 is not 1, and E came
-// out 1.1e-9 too large with a third of the trace in each.  multiply: one of the three links that loops
+// out 1.1e-9 too large with a third of the trace in each (5e-10 so).  multiply: one of the three links that loops
 // move along here is not unitary.
 template <typename F, typename S, typename R>
 __device__ __forceinline__ ah9<R> clover_plane(const F& f, const Loops<S>& K, const Coord& x, const NbOff& o, int mu,
@@ -395,10 +367,10 @@ __device__ __forceinline__ ah9<R> clover_plane(const F& f, const Loops<S>& K, co
   const R tr = (K.template load_tr<R>(plane, par, j0) + K.template load_tr<R>(plane, par, jmn)) +
                (K.template load_tr<R>(plane, opp, jmu) + K.template load_tr<R>(plane, opp, jnu));
   ah9<R> out;
-  const R tr3 = tr * R(1.0 / 3.0);
-  out.d[0] = R(0.25) * (A.a[0] + tr3);
-  out.d[1] = R(0.25) * (A.a[1] + tr3);
-  out.d[2] = R(0.25) * ((tr - (tr3 + tr3)) - (A.a[0] + A.a[1]));
+  const R d0 = fma(R(1.0 / 3.0), tr, A.a[0]), d1 = fma(R(1.0 / 3.0), tr, A.a[1]);
+  out.d[0] = R(0.25) * d0;
+  out.d[1] = R(0.25) * d1;
+  out.d[2] = R(0.25) * (tr - (d0 + d1));
 #pragma unroll
   for (int k = 0; k < 3; ++k) out.o[k] = mk<R>(R(0.25) * A.a[2 + 2 * k], R(0.25) * A.a[3 + 2 * k]);
   return out;

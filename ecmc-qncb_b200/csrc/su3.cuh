@@ -385,10 +385,9 @@ template <typename R>
 __device__ __forceinline__ alg8<R> proj_ta(const m3<R>& m) {
   alg8<R> z;
   R d0 = m.e[0][0].im, d1 = m.e[1][1].im, d2 = m.e[2][2].im;
-  // (no fma here: with it the two elements and the trace give E of the clover 2e-10 too large in FP32)
-  const R tr3 = (d0 + d1 + d2) * R(1.0 / 3.0);
-  z.a[0] = d0 - tr3;
-  z.a[1] = d1 - tr3;
+  const R tr = d0 + d1 + d2;
+  z.a[0] = fma(R(-1.0 / 3.0), tr, d0);
+  z.a[1] = fma(R(-1.0 / 3.0), tr, d1);
   z.a[2] = R(0.5) * (m.e[0][1].re - m.e[1][0].re);
   z.a[3] = R(0.5) * (m.e[0][1].im + m.e[1][0].im);
   z.a[4] = R(0.5) * (m.e[0][2].re - m.e[2][0].re);
